@@ -20,9 +20,9 @@ import torch.nn.functional as F
 from torch.utils.checkpoint import checkpoint
 
 from . import ops
-from .backward import RationalAttentionPackedFunction
+from .backward import rational_attention_packed
 from .forward import compute_alibi_slopes
-from .fused_ops import (EPS, RationalSwiGLUPacked, add_mean_error_norm, head_shifted_cross_entropy, mean_error_norm,
+from .fused_ops import (EPS, add_mean_error_norm, head_shifted_cross_entropy, mean_error_norm, rational_swiglu,
                         shifted_cross_entropy)
 
 
@@ -51,7 +51,7 @@ class RationalSwiGLU(nn.Module):
         gv = self.w_gate_val(x)
         if not gv.is_cuda:
             raise RuntimeError("RationalSwiGLU: CUDA tensor required — this build has no CPU fallback")
-        return self.dropout(self.w_out(RationalSwiGLUPacked.apply(gv)))
+        return self.dropout(self.w_out(rational_swiglu(*gv.chunk(2, dim=-1))))
 
 
 class KVCache:
@@ -116,7 +116,7 @@ class AlgebraicAttention(nn.Module):
             return self.dropout(self.out(out))
         if mask is not None and cache is not None:
             raise ValueError("the key/value cache takes no padding mask")
-        out = RationalAttentionPackedFunction.apply(qkv, self.alibi_slopes, self.scale, EPS, mask)     # [B,T,C]
+        out = rational_attention_packed(qkv, self.alibi_slopes, self.scale, EPS, mask)     # [B,T,C]
         if cache is not None:
             k_cache, v_cache, state = cache
             if T > state.capacity:

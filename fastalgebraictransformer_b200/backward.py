@@ -92,8 +92,18 @@ def rational_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, alibi_
                        causal: bool = True, eps: float = EPS, key_mask: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Memory-efficient rational attention with a custom backward (reference backward.py:386-396).  ``key_mask`` (an
     extension): padding mask [B, T], 0 = the key is padding and weighs nothing for any query."""
-    if not q.is_cuda:
-        raise RuntimeError("rational_attention: CUDA tensors required — this build has no CPU fallback")
-    if key_mask is None:
-        return RationalAttentionFunction.apply(q, k, v, alibi_slopes, scale, causal, eps)
-    return RationalAttentionFunction.apply(q, k, v, alibi_slopes, scale, causal, eps, _lib.PATH_AUTO, False, key_mask)
+    if torch.compiler.is_compiling():
+        return RationalAttentionFunction.apply(q, k, v, alibi_slopes, scale, causal, eps, _lib.PATH_AUTO, False, key_mask)
+    if key_mask is None or isinstance(key_mask, torch.Tensor):
+        return ops.host.rational_attention(q, k, v, alibi_slopes, scale, causal, eps, key_mask, -1)
+    return ops.host.rational_attention(q, k, v, alibi_slopes, scale, causal, eps, key_mask.bits, key_mask.n_tokens)
+
+
+def rational_attention_packed(qkv: torch.Tensor, alibi_slopes: torch.Tensor, scale: float, eps: float = EPS, key_mask=None) -> torch.Tensor:
+    """Causal rational attention of a packed projection [B, T, 3, H, D] -> [B, T, H*D]: RationalAttentionPackedFunction with
+    its node in C++ (reference algebraic_model.py:89-107)."""
+    if torch.compiler.is_compiling():
+        return RationalAttentionPackedFunction.apply(qkv, alibi_slopes, scale, eps, key_mask)
+    if key_mask is None or isinstance(key_mask, torch.Tensor):
+        return ops.host.rational_attention_packed(qkv, alibi_slopes, scale, eps, key_mask, -1)
+    return ops.host.rational_attention_packed(qkv, alibi_slopes, scale, eps, key_mask.bits, key_mask.n_tokens)

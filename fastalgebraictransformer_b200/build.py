@@ -19,7 +19,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(PKG, "libfat_b200.so")
-OPS_SRC = os.path.join(CSRC, "torch_ops.cpp")
+OPS_SRCS = [os.path.join(CSRC, n) for n in ("torch_ops.cpp", "torch_autograd.cpp")]
 OPS_LIB = os.path.join(PKG, "libfat_torch_ops.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -75,7 +75,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link of libfat_b200.so failed")
-    build_ops(force or bool(jobs), verbose)
+    build_ops(force, verbose)
     build_wait_test(force, verbose)
     return LIB
 
@@ -113,25 +113,38 @@ def build_wait_test(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_ops(force: bool = False, verbose: bool = False) -> str:
-    """Compile csrc/torch_ops.cpp (the C++ registration of the torch.library operators) against the installed torch
-    and link it to libfat_b200.so.  Host code only: g++, no nvcc."""
+    """Compile the C++ registration of the torch.library operators (csrc/torch_ops.cpp) and their autograd nodes and Python
+    entry points (csrc/torch_autograd.cpp) against the installed torch and link them to libfat_b200.so; the result is also
+    an extension module.  Host code only: g++, no nvcc."""
     header = os.path.join(PKG, "..", "include", "fat_b200.h")
-    if not (force or _stale(OPS_LIB, [OPS_SRC, header, LIB])):
+    if not (force or _stale(OPS_LIB, [*OPS_SRCS, header, LIB])):
         return OPS_LIB
+    import sysconfig
+
     import torch
     from torch.utils import cpp_extension as ce
     cuda_home = os.environ.get("CUDA_HOME") or os.path.dirname(os.path.dirname(_nvcc()))
     cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
-    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", OPS_SRC, "-o", OPS_LIB,
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I" + os.path.join(cuda_home, "include")]
-    cmd += ["-I" + p for p in ce.include_paths()]
-    cmd += ["-L" + p for p in ce.library_paths()]
-    cmd += ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-L" + PKG, "-lfat_b200", "-Wl,-rpath,$ORIGIN"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or r.returncode:
-        sys.stderr.write(r.stdout + r.stderr)
-    if r.returncode:
-        raise RuntimeError("build of libfat_torch_ops.so failed")
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             "-I" + os.path.join(cuda_home, "include"), "-I" + sysconfig.get_paths()["include"]]
+    flags += ["-I" + p for p in ce.include_paths()]
+    objs = [os.path.join(OBJ, os.path.basename(src)[:-4] + ".o") for src in OPS_SRCS]
+    cmds = [[cxx, *flags, "-c", src, "-o", obj] for src, obj in zip(OPS_SRCS, objs) if force or _stale(obj, [src, header])]
+    link = [cxx, "-shared", *objs, "-o", OPS_LIB] + ["-L" + p for p in ce.library_paths()]
+    link += ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-L" + PKG, "-lfat_b200", "-Wl,-rpath,$ORIGIN"]
+
+    def run(cmd):
+        return subprocess.run(cmd, capture_output=True, text=True)
+
+    with cf.ThreadPoolExecutor(max_workers=2) as ex:
+        results = list(ex.map(run, cmds))
+    if all(r.returncode == 0 for r in results):
+        results.append(run(link))
+    for r in results:
+        if verbose or r.returncode:
+            sys.stderr.write(r.stdout + r.stderr)
+        if r.returncode:
+            raise RuntimeError("build of libfat_torch_ops.so failed")
     return OPS_LIB
 
 

@@ -344,8 +344,7 @@ bool tiles_vectorisable(const AttnParams& p, bool bwd) {
 
 template <typename Kern>
 int launch(Kern kern, const AttnParams& p, bool vec, int tiles, size_t smem, cudaStream_t st, const char* what) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) { set_error("%s: cannot reserve %zu bytes of shared memory: %s", what, smem, cudaGetErrorString(e)); return FAT_ERR_LAUNCH; }
+  if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, what)) return rc;
   dim3 grid(tiles, p.H, p.B);
   kern<<<grid, NT, smem, st>>>(p, vec);
   return check_launch(what);

@@ -1178,10 +1178,7 @@ bool make_qk_maps(const AttnParams& p, CUtensorMap* mq, CUtensorMap* mk, bool k_
 
 template <typename Kern, typename Maps>
 int launch_main(Kern kern, const Maps& maps, const AttnParams& p, size_t smem, int threads, cudaStream_t st, const char* what) {
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
-    set_error("%s: cannot reserve %zu bytes of shared memory", what, smem);
-    return FAT_ERR_LAUNCH;
-  }
+  if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, what)) return rc;
   const dim3 grid(banded_grid((p.T + BLK - 1) / BLK, p.B * p.H, kBwdBands));
   kern<<<grid, threads, smem, st>>>(maps, p);
   return check_launch(what);
@@ -1211,11 +1208,11 @@ template <typename T, int D>
 int launch_bwd_fused(const AttnParams& p, cudaStream_t st) {
   float* dq_acc = ws_dq_acc(p);
   auto kern = p.key_mask ? attn_bwd_fused_tc_kernel<T, D, true> : attn_bwd_fused_tc_kernel<T, D, false>;
-  cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess ||
-      fa.numRegs * kFusedThreads < 256 * kFusedRegsEw + 128 * kFusedRegsDrain + 128 * kFusedRegsAux) {
+  int regs = 0;
+  if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), sizeof(FusedSmem<D>), "attn_bwd_fused_tc", &regs)) return rc;
+  if (regs * kFusedThreads < 256 * kFusedRegsEw + 128 * kFusedRegsDrain + 128 * kFusedRegsAux) {
     // the warpgroups could never collect their register shares: refuse instead of letting setmaxnreg.inc wait
-    set_error("attn_bwd_fused: built with %d registers per thread, the register hand-over needs %d", fa.numRegs, kFusedRegsLaunch);
+    set_error("attn_bwd_fused: built with %d registers per thread, the register hand-over needs %d", regs, kFusedRegsLaunch);
     return FAT_ERR_LAUNCH;
   }
   FusedMaps m;

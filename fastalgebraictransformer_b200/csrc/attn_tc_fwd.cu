@@ -414,8 +414,7 @@ int launch_fwd(const AttnParams& p, cudaStream_t st) {
   }
   auto kern = attn_fwd_tc_kernel<T, D>;
   const size_t smem = sizeof(FwdSmem<D>) + 1024;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) { set_error("attn_fwd_tc: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e)); return FAT_ERR_LAUNCH; }
+  if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, "attn_fwd_tc")) return rc;
   const dim3 grid(banded_grid((p.T + 2 * BLK - 1) / (2 * BLK), p.B * p.H, kFwdBands));
   kern<<<grid, kFwdThreads, smem, st>>>(maps, p);
   return check_launch("attn_fwd_tc");

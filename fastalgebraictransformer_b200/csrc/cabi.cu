@@ -3,6 +3,9 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "attn_common.cuh"
 
@@ -38,6 +41,32 @@ int num_sms() {
     cached[dev].store(n, std::memory_order_relaxed);
   }
   return n;
+}
+
+int ready_kernel(const void* kernel, size_t smem_bytes, const char* what, int* regs) {
+  struct Known { size_t smem; int regs; };
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, Known> known;        // (a few dozen kernels at most)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find({kernel, dev});
+    if (it == known.end()) {
+      cudaFuncAttributes fa;
+      if ((e = cudaFuncGetAttributes(&fa, kernel)) == cudaSuccess) it = known.insert({{kernel, dev}, {0, fa.numRegs}}).first;
+    }
+    if (e == cudaSuccess && smem_bytes > it->second.smem) {
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
+      if (e == cudaSuccess) it->second.smem = smem_bytes;
+    }
+    if (e == cudaSuccess) {
+      if (regs) *regs = it->second.regs;
+      return FAT_OK;
+    }
+  }
+  set_error("%s: cannot reserve %zu bytes of shared memory: %s", what, smem_bytes, cudaGetErrorString(e));
+  return FAT_ERR_LAUNCH;
 }
 
 // The tensor-core attention kernels cover 16-bit tensors, head sizes 64 and 128 (causal or not), and pointers /

@@ -19,6 +19,11 @@ int num_sms();
 void set_error(const char* fmt, ...);          // defined in cabi.cu (thread-local buffer)
 int  check_launch(const char* what);           // cudaGetLastError -> FAT_ERR_LAUNCH
 
+// Readies a kernel for launches with `smem_bytes` of dynamic shared memory on the current device and reports its registers
+// per thread (regs may be null).  The driver is asked once per kernel and device (about 1 us per question otherwise, on
+// every launch).  FAT_OK, or FAT_ERR_LAUNCH with the error text set.
+int ready_kernel(const void* kernel, size_t smem_bytes, const char* what, int* regs = nullptr);
+
 // ---------------------------------------------------------------- element traits
 template <typename T> struct Elem;
 template <> struct Elem<float> {

@@ -826,7 +826,7 @@ int norm_bwd_t(const void* d_out, const void* x, const void* w, const float* mea
   C* partial = reinterpret_cast<C*>(ws);
   if (p.fast) {
     auto go = [&](auto kern, size_t smem) {
-      if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      if (smem > 48 * 1024) ready_kernel(reinterpret_cast<const void*>(kern), smem, "norm_bwd");   // (a failure shows in the launch)
       kern<<<p.grid, threads, smem, st>>>((const T*)d_out, (const T*)x, (const T*)w, mean, (T*)d_x, partial,
                                          n_rows, int(n_cols), dos, xs, dxs, eps, p.G, (const T*)d_add, das);
     };
@@ -834,7 +834,7 @@ int norm_bwd_t(const void* d_out, const void* x, const void* w, const float* mea
     if constexpr (sizeof(T) == 2) {
       if (p.vpt <= 2) {                                     // 16-bit rows of up to two packs per thread: the packed-arithmetic kernel
         auto go16 = [&](auto kern, size_t smem) {
-          if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+          if (smem > 48 * 1024) ready_kernel(reinterpret_cast<const void*>(kern), smem, "norm_bwd");   // (a failure shows in the launch)
           kern<<<p.grid, threads, smem, st>>>((const T*)d_out, (const T*)x, (const T*)w, mean, (T*)d_x, partial,
                                              n_rows, int(n_cols), dos, xs, dxs, eps, p.G, (const T*)d_add, das);
         };

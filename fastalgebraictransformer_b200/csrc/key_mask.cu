@@ -12,8 +12,9 @@
 namespace fat {
 namespace {
 
+template <typename E>
 __global__ void __launch_bounds__(256)
-pack_key_mask_kernel(const uint8_t* __restrict__ mask, uint32_t* __restrict__ bits, int B, int T, int words,
+pack_key_mask_kernel(const E* __restrict__ mask, uint32_t* __restrict__ bits, int B, int T, int words,
                      int64_t batch_stride, int64_t token_stride) {
   const int lane = threadIdx.x & 31;
   const int64_t n_words = int64_t(B) * words;
@@ -34,13 +35,29 @@ extern "C" int fat_key_mask_words(int T) { return T > 0 ? 4 * ((T + 127) / 128) 
 
 extern "C" int fat_pack_key_mask(const uint8_t* mask, uint32_t* bits, int B, int T, int64_t mask_batch_stride,
                                  int64_t mask_token_stride, void* stream) {
+  return fat_pack_key_mask_elems(mask, 1, bits, B, T, mask_batch_stride, mask_token_stride, stream);
+}
+
+extern "C" int fat_pack_key_mask_elems(const void* mask, int element_bytes, uint32_t* bits, int B, int T, int64_t mask_batch_stride,
+                                       int64_t mask_token_stride, void* stream) {
   if (B < 0 || T < 0) { set_error("pack_key_mask: bad shape [%d, %d]", B, T); return FAT_ERR_SHAPE; }
   if (B == 0 || T == 0) return FAT_OK;
   if (!mask || !bits) { set_error("pack_key_mask: null pointer"); return FAT_ERR_NULL; }
   const int words = fat_key_mask_words(T);
   const int64_t warps = int64_t(B) * words;
   const int64_t blocks = (warps + 7) / 8;
-  pack_key_mask_kernel<<<unsigned(blocks < 8 * int64_t(num_sms()) ? blocks : 8 * int64_t(num_sms())), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      mask, bits, B, T, words, mask_batch_stride, mask_token_stride);
-  return check_launch("pack_key_mask");
+  const unsigned grid = unsigned(blocks < 8 * int64_t(num_sms()) ? blocks : 8 * int64_t(num_sms()));
+  auto go = [&](auto zero) {
+    using E = decltype(zero);
+    pack_key_mask_kernel<E><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const E*>(mask), bits, B, T, words,
+                                                                                mask_batch_stride, mask_token_stride);
+    return check_launch("pack_key_mask");
+  };
+  switch (element_bytes) {
+    case 1: return go(uint8_t{});
+    case 2: return go(uint16_t{});
+    case 4: return go(uint32_t{});
+    case 8: return go(uint64_t{});
+    default: set_error("pack_key_mask: elements of %d bytes", element_bytes); return FAT_ERR_DTYPE;
+  }
 }

@@ -8,6 +8,7 @@
 // Built by `python -m fastalgebraictransformer_b200.build` into libfat_torch_ops.so next to libfat_b200.so.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
@@ -34,6 +35,13 @@ int dtype_tag(const Tensor& t) {
     default: TORCH_CHECK_TYPE(false, "unsupported dtype ", t.scalar_type());
   }
 }
+
+// Uninitialised CUDA tensor next to `like` (its device; dtype as given): the allocator directly, without the dispatcher,
+// which costs as much as the allocation itself.
+Tensor empty_like_options(at::IntArrayRef sizes, const Tensor& like, at::ScalarType dtype) {
+  return Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
+}
+Tensor empty_of(at::IntArrayRef sizes, const Tensor& like) { return empty_like_options(sizes, like, like.scalar_type()); }
 
 void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
@@ -85,7 +93,7 @@ Tensor device_status(int64_t device) { return status_word(int(device)); }
 Tensor swiglu_fwd(const Tensor& gate, const Tensor& value) {
   cuda_check({&gate, &value});
   TORCH_CHECK(gate.sizes() == value.sizes() && gate.scalar_type() == value.scalar_type(), "gate and value must match");
-  Tensor out = at::empty(gate.sizes(), gate.options());
+  Tensor out = empty_of(gate.sizes(), gate);
   if (gate.numel() == 0) return out;
   const Tensor g = rows(gate), v = rows(value), o = out.view({-1, gate.size(-1)});
   c10::cuda::CUDAGuard guard(gate.device());
@@ -94,20 +102,36 @@ Tensor swiglu_fwd(const Tensor& gate, const Tensor& value) {
   return out;
 }
 
-std::tuple<Tensor, Tensor> swiglu_bwd(const Tensor& d_out, const Tensor& gate, const Tensor& value) {
+void swiglu_bwd_into(const Tensor& d_out, const Tensor& gate, const Tensor& value, const Tensor& d_gate, const Tensor& d_value) {
   cuda_check({&d_out, &gate, &value});
-  const int64_t n = gate.size(-1);
-  // both gradients live in one [rows, 2n] buffer: when gate/value were the two halves of a packed projection,
-  // autograd's concatenation of the halves becomes a no-op copy target of the same layout
-  auto shape = gate.sizes().vec();
-  shape.back() = 2 * n;
-  Tensor packed = at::empty(shape, gate.options());
-  Tensor d_gate = packed.narrow(-1, 0, n), d_value = packed.narrow(-1, n, n);
-  if (gate.numel() == 0) return {d_gate, d_value};
+  if (gate.numel() == 0) return;
   const Tensor go = rows(d_out), g = rows(gate), v = rows(value), dg = rows(d_gate), dv = rows(d_value);
   c10::cuda::CUDAGuard guard(gate.device());
-  check(fat_swiglu_bwd(go.data_ptr(), g.data_ptr(), v.data_ptr(), dg.data_ptr(), dv.data_ptr(), g.size(0), n, go.stride(0),
+  check(fat_swiglu_bwd(go.data_ptr(), g.data_ptr(), v.data_ptr(), dg.data_ptr(), dv.data_ptr(), g.size(0), gate.size(-1), go.stride(0),
                        g.stride(0), v.stride(0), dg.stride(0), dv.stride(0), dtype_tag(gate), stream_of(gate)));
+}
+
+// Both gradients in one [.., 2n] tensor, gate half first: the gradient of a packed projection without a concatenation.
+Tensor swiglu_bwd_packed(const Tensor& d_out, const Tensor& gate, const Tensor& value) {
+  const int64_t n = gate.size(-1);
+  auto shape = gate.sizes().vec();
+  shape.back() = 2 * n;
+  Tensor packed = empty_of(shape, gate);
+  swiglu_bwd_into(d_out, gate, value, packed.narrow(-1, 0, n), packed.narrow(-1, n, n));
+  return packed;
+}
+
+std::tuple<Tensor, Tensor> swiglu_bwd(const Tensor& d_out, const Tensor& gate, const Tensor& value) {
+  const int64_t n = gate.size(-1);
+  const Tensor packed = swiglu_bwd_packed(d_out, gate, value);
+  return {packed.narrow(-1, 0, n), packed.narrow(-1, n, n)};
+}
+
+// Two dense gradients, for a gate and a value that are tensors of their own: a leaf keeps a dense gradient as it is, where
+// the halves of a packed buffer would be copied into dense ones (595 of 930 us at [16384, 8192] bfloat16).
+std::tuple<Tensor, Tensor> swiglu_bwd_dense(const Tensor& d_out, const Tensor& gate, const Tensor& value) {
+  Tensor d_gate = empty_of(gate.sizes(), gate), d_value = empty_of(value.sizes(), value);
+  swiglu_bwd_into(d_out, gate, value, d_gate, d_value);
   return {d_gate, d_value};
 }
 
@@ -117,9 +141,9 @@ std::tuple<Tensor, Tensor> norm_fwd(const Tensor& x, const Tensor& weight, doubl
   const int64_t n = x.size(-1);
   TORCH_CHECK(weight.dim() == 1 && weight.size(0) == n, "weight must be [n_cols]");
   const Tensor w = weight.to(x.scalar_type()).contiguous();
-  Tensor y = at::empty(x.sizes(), x.options());
+  Tensor y = empty_of(x.sizes(), x);
   const Tensor xr = rows(x);
-  Tensor mean = at::empty({xr.size(0)}, x.options().dtype(at::kFloat));
+  Tensor mean = empty_like_options({xr.size(0)}, x, at::kFloat);
   if (x.numel()) {
     const Tensor yr = y.view({-1, n});
     c10::cuda::CUDAGuard guard(x.device());
@@ -133,12 +157,12 @@ std::tuple<Tensor, Tensor> norm_bwd(const Tensor& d_out, const Tensor& x, const 
   cuda_check({&d_out, &x, &weight, &mean});
   const int64_t n = x.size(-1);
   const Tensor w = weight.to(x.scalar_type()).contiguous();
-  Tensor d_x = at::empty(x.sizes(), x.options()), d_w = at::empty({n}, x.options());
+  Tensor d_x = empty_of(x.sizes(), x), d_w = empty_of({n}, x);
   const Tensor go = rows(d_out), xr = rows(x), dxr = d_x.view({-1, n});
   const int tag = dtype_tag(x);
   c10::cuda::CUDAGuard guard(x.device());
   const size_t ws_bytes = fat_norm_bwd_workspace_bytes(xr.size(0), n, tag);
-  Tensor ws = at::empty({int64_t(ws_bytes)}, x.options().dtype(at::kByte));
+  Tensor ws = empty_like_options({int64_t(ws_bytes)}, x, at::kByte);
   check(fat_norm_bwd(go.data_ptr(), xr.data_ptr(), w.data_ptr(), mean.data_ptr<float>(), dxr.data_ptr(), d_w.data_ptr(),
                      ws.data_ptr(), ws_bytes, xr.size(0), n, go.numel() ? go.stride(0) : n, xr.numel() ? xr.stride(0) : n, n,
                      eps, tag, stream_of(x)));
@@ -152,9 +176,9 @@ std::tuple<Tensor, Tensor, Tensor> add_norm_fwd(const Tensor& x, const Tensor& r
   const int64_t n = x.size(-1);
   TORCH_CHECK(weight.dim() == 1 && weight.size(0) == n, "weight must be [n_cols]");
   const Tensor w = weight.to(x.scalar_type()).contiguous();
-  Tensor h = at::empty(x.sizes(), x.options()), y = at::empty(x.sizes(), x.options());
+  Tensor h = empty_of(x.sizes(), x), y = empty_of(x.sizes(), x);
   const Tensor xr = rows(x), rr = rows(residual);
-  Tensor mean = at::empty({xr.size(0)}, x.options().dtype(at::kFloat));
+  Tensor mean = empty_like_options({xr.size(0)}, x, at::kFloat);
   if (x.numel()) {
     const Tensor hr = h.view({-1, n}), yr = y.view({-1, n});
     c10::cuda::CUDAGuard guard(x.device());
@@ -170,7 +194,7 @@ std::tuple<Tensor, Tensor> add_norm_bwd(const Tensor& d_y, const c10::optional<T
   cuda_check({&d_y, &h, &weight, &mean});
   const int64_t n = h.size(-1);
   const Tensor w = weight.to(h.scalar_type()).contiguous();
-  Tensor d_sum = at::empty(h.sizes(), h.options()), d_w = at::empty({n}, h.options());
+  Tensor d_sum = empty_of(h.sizes(), h), d_w = empty_of({n}, h);
   const Tensor go = rows(d_y), hr = rows(h), dsr = d_sum.view({-1, n});
   Tensor dh;
   if (d_h.has_value() && d_h->defined()) dh = rows(d_h->to(h.scalar_type()));
@@ -178,7 +202,7 @@ std::tuple<Tensor, Tensor> add_norm_bwd(const Tensor& d_y, const c10::optional<T
   const int tag = dtype_tag(h);
   c10::cuda::CUDAGuard guard(h.device());
   const size_t ws_bytes = fat_norm_bwd_workspace_bytes(hr.size(0), n, tag);
-  Tensor ws = at::empty({int64_t(ws_bytes)}, h.options().dtype(at::kByte));
+  Tensor ws = empty_like_options({int64_t(ws_bytes)}, h, at::kByte);
   check(fat_add_norm_bwd(go.data_ptr(), has_dh ? dh.data_ptr() : nullptr, hr.data_ptr(), w.data_ptr(), mean.data_ptr<float>(),
                          dsr.data_ptr(), d_w.data_ptr(), ws.data_ptr(), ws_bytes, hr.size(0), n, go.numel() ? go.stride(0) : n,
                          has_dh ? dh.stride(0) : n, hr.numel() ? hr.stride(0) : n, n, eps, tag, stream_of(h)));
@@ -199,8 +223,8 @@ std::tuple<Tensor, Tensor> shifted_ce_fwd(const Tensor& logits_in, const Tensor&
   const Tensor logits = logits_in.stride(2) == 1 ? logits_in : logits_in.contiguous();
   const int64_t B = logits.size(0), T = logits.size(1), V = logits.size(2);
   const Tensor n_valid = count_valid(labels, ignore_index, V);
-  Tensor row_loss = at::empty({B * T}, logits.options().dtype(at::kFloat));
-  Tensor d_logits = at::empty({B, T, V}, logits.options());
+  Tensor row_loss = empty_like_options({B * T}, logits, at::kFloat);
+  Tensor d_logits = empty_of({B, T, V}, logits);
   if (logits.numel()) {
     c10::cuda::CUDAGuard guard(logits.device());
     check(fat_shifted_ce_fwd(logits.data_ptr(), labels.data_ptr<int64_t>(), n_valid.data_ptr<float>(), row_loss.data_ptr<float>(),
@@ -263,7 +287,7 @@ void scale_unless_one(Tensor x, const Tensor& scale) {
 Tensor softmax_fwd(const Tensor& x, double eps) {
   cuda_check({&x});
   const int64_t n = x.size(-1);
-  Tensor p = at::empty(x.sizes(), x.options());
+  Tensor p = empty_of(x.sizes(), x);
   if (x.numel()) {
     const Tensor xr = rows(x), pr = p.view({-1, n});
     c10::cuda::CUDAGuard guard(x.device());
@@ -275,7 +299,7 @@ Tensor softmax_fwd(const Tensor& x, double eps) {
 Tensor softmax_bwd(const Tensor& d_out, const Tensor& x, double eps) {
   cuda_check({&d_out, &x});
   const int64_t n = x.size(-1);
-  Tensor d_x = at::empty(x.sizes(), x.options());
+  Tensor d_x = empty_of(x.sizes(), x);
   if (x.numel()) {
     const Tensor go = rows(d_out), xr = rows(x), dxr = d_x.view({-1, n});
     c10::cuda::CUDAGuard guard(x.device());
@@ -293,8 +317,8 @@ bool is_token_major(const Tensor& t) { return t.dim() == 4 && t.size(1) > 1 && t
 
 Tensor alloc_bhtd(const Tensor& like, bool token_major) {
   const int64_t B = like.size(0), H = like.size(1), T = like.size(2), D = like.size(3);
-  if (token_major) return at::empty({B, T, H, D}, like.options()).permute({0, 2, 1, 3});
-  return at::empty({B, H, T, D}, like.options());
+  if (token_major) return empty_of({B, T, H, D}, like).permute({0, 2, 1, 3});
+  return empty_of({B, H, T, D}, like);
 }
 
 // The packed padding mask of a launch (see fat_pack_key_mask), or null when there is none.
@@ -311,13 +335,14 @@ const uint32_t* mask_bits(const c10::optional<Tensor>& key_mask, const Tensor& q
 Tensor pack_key_mask(const Tensor& mask) {
   cuda_check({&mask});
   TORCH_CHECK(mask.dim() == 2, "attention mask must be [B, T]");
-  const Tensor m = mask.scalar_type() == at::kBool ? mask : mask.ne(0);
+  // an integer is non-zero when any of its bits is set, so bool and integer masks are packed as they are
+  const Tensor m = at::isIntegralType(mask.scalar_type(), /*includeBool=*/true) ? mask : mask.ne(0);
   const int64_t B = m.size(0), T = m.size(1);
-  Tensor bits = at::empty({B, int64_t(fat_key_mask_words(int(T)))}, m.options().dtype(at::kInt));
+  Tensor bits = empty_like_options({B, int64_t(fat_key_mask_words(int(T)))}, m, at::kInt);
   if (bits.numel()) {
     c10::cuda::CUDAGuard guard(m.device());
-    check(fat_pack_key_mask(reinterpret_cast<const uint8_t*>(m.data_ptr<bool>()), reinterpret_cast<uint32_t*>(bits.data_ptr<int>()), int(B), int(T),
-                            m.stride(0), m.stride(1), stream_of(m)));
+    check(fat_pack_key_mask_elems(m.data_ptr(), int(m.element_size()), reinterpret_cast<uint32_t*>(bits.data_ptr<int>()), int(B), int(T),
+                                  m.stride(0), m.stride(1), stream_of(m)));
   }
   return bits;
 }
@@ -335,8 +360,8 @@ std::tuple<Tensor, Tensor, Tensor> attn_fwd(const Tensor& q_in, const Tensor& k_
   Tensor out = alloc_bhtd(q, token_major_out);
   // 16-bit outputs also keep their rounding residual, so the backward can form Delta = dO.O accurately (`residual` false: the
   // caller knows no backward will follow and saves the second store pass, 5 % of the forward, and the tensor)
-  Tensor out_lo = (q.element_size() == 2 && residual) ? alloc_bhtd(q, token_major_out) : at::empty({0}, q.options());
-  Tensor L = at::empty({B, H, T}, q.options().dtype(at::kFloat));
+  Tensor out_lo = (q.element_size() == 2 && residual) ? alloc_bhtd(q, token_major_out) : empty_of({0}, q);
+  Tensor L = empty_like_options({B, H, T}, q, at::kFloat);
   if (q.numel()) {
     c10::cuda::CUDAGuard guard(q.device());
     const auto qs = strides3(q), ks = strides3(k), vs = strides3(v), os = strides3(out);
@@ -348,10 +373,12 @@ std::tuple<Tensor, Tensor, Tensor> attn_fwd(const Tensor& q_in, const Tensor& k_
   return {out, L, out_lo};
 }
 
-std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& out_in,
-                                            const Tensor& out_lo_in, const Tensor& L, const Tensor& d_out_in, const Tensor& slopes,
-                                            double scale, bool causal, double eps, int64_t path, const c10::optional<Tensor>& key_mask) {
+// Fills d_q, d_k, d_v ([B,H,T,D], unit stride along D).
+void attn_bwd_into(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& out_in, const Tensor& out_lo_in,
+                   const Tensor& L, const Tensor& d_out_in, const Tensor& slopes, double scale, bool causal, double eps, int64_t path,
+                   const c10::optional<Tensor>& key_mask, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v) {
   cuda_check({&q_in, &k_in, &v_in, &out_in, &L, &d_out_in, &slopes});
+  if (q_in.numel() == 0) return;
   const Tensor q = unit_d(q_in), k = unit_d(k_in), v = unit_d(v_in), d_out = unit_d(d_out_in);
   Tensor out = unit_d(out_in), out_lo = out_lo_in;
   const int64_t B = q.size(0), H = q.size(1), T = q.size(2), D = q.size(3);
@@ -365,31 +392,52 @@ std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& q_in, const Tensor& k_
   }
   const Tensor sl = slopes.to(at::kFloat).contiguous();
   const Tensor Lc = L.contiguous();
-  Tensor d_q, d_k, d_v;
+  const int tag = dtype_tag(q);
+  c10::cuda::CUDAGuard guard(q.device());
+  const size_t ws_bytes = fat_attn_bwd_workspace_bytes(int(B), int(H), int(T), int(D), tag, int(path));
+  Tensor ws = empty_like_options({int64_t(ws_bytes)}, q, at::kByte);
+  const auto qs = strides3(q), ks = strides3(k), vs = strides3(v), os = strides3(out), dos = strides3(d_out), dqs = strides3(d_q),
+             dks = strides3(d_k), dvs = strides3(d_v);
+  check(fat_attn_bwd_masked(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lo_ptr, Lc.data_ptr<float>(), d_out.data_ptr(),
+                     sl.data_ptr<float>(), mask_bits(key_mask, q), d_q.data_ptr(), d_k.data_ptr(), d_v.data_ptr(), ws.data_ptr(), ws_bytes, int(B), int(H), int(T),
+                     int(D), qs.data(), ks.data(), vs.data(), os.data(), dos.data(), dqs.data(), dks.data(), dvs.data(), scale, eps,
+                     int(causal), tag, int(path), status_word(q.get_device()).data_ptr<int>(), stream_of(q)));
+}
+
+std::array<Tensor, 3> heads_of(const Tensor& qkv) {          // [B,T,3,H,D] -> q, k, v as [B,H,T,D] views
+  return {qkv.select(2, 0).permute({0, 2, 1, 3}), qkv.select(2, 1).permute({0, 2, 1, 3}), qkv.select(2, 2).permute({0, 2, 1, 3})};
+}
+
+std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out,
+                                            const Tensor& out_lo, const Tensor& L, const Tensor& d_out, const Tensor& slopes,
+                                            double scale, bool causal, double eps, int64_t path, const c10::optional<Tensor>& key_mask) {
+  const int64_t B = q.size(0), H = q.size(1), T = q.size(2), D = q.size(3);
+  std::array<Tensor, 3> d;
   if (is_token_major(q)) {
-    // gradients of the three slices of a packed projection go into one [B,T,3,H,D] buffer
-    Tensor packed = at::empty({B, T, 3, H, D}, q.options());
-    d_q = packed.select(2, 0).permute({0, 2, 1, 3});
-    d_k = packed.select(2, 1).permute({0, 2, 1, 3});
-    d_v = packed.select(2, 2).permute({0, 2, 1, 3});
+    d = heads_of(empty_of({B, T, 3, H, D}, q));    // gradients of the three slices of a packed projection go into one buffer
   } else {
-    d_q = at::empty({B, H, T, D}, q.options());
-    d_k = at::empty({B, H, T, D}, q.options());
-    d_v = at::empty({B, H, T, D}, q.options());
+    for (Tensor& t : d) t = empty_of({B, H, T, D}, q);
   }
-  if (q.numel()) {
-    const int tag = dtype_tag(q);
-    c10::cuda::CUDAGuard guard(q.device());
-    const size_t ws_bytes = fat_attn_bwd_workspace_bytes(int(B), int(H), int(T), int(D), tag, int(path));
-    Tensor ws = at::empty({int64_t(ws_bytes)}, q.options().dtype(at::kByte));
-    const auto qs = strides3(q), ks = strides3(k), vs = strides3(v), os = strides3(out), dos = strides3(d_out), dqs = strides3(d_q),
-               dks = strides3(d_k), dvs = strides3(d_v);
-    check(fat_attn_bwd_masked(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lo_ptr, Lc.data_ptr<float>(), d_out.data_ptr(),
-                       sl.data_ptr<float>(), mask_bits(key_mask, q), d_q.data_ptr(), d_k.data_ptr(), d_v.data_ptr(), ws.data_ptr(), ws_bytes, int(B), int(H), int(T),
-                       int(D), qs.data(), ks.data(), vs.data(), os.data(), dos.data(), dqs.data(), dks.data(), dvs.data(), scale, eps,
-                       int(causal), tag, int(path), status_word(q.get_device()).data_ptr<int>(), stream_of(q)));
-  }
-  return {d_q, d_k, d_v};
+  attn_bwd_into(q, k, v, out, out_lo, L, d_out, slopes, scale, causal, eps, path, key_mask, d[0], d[1], d[2]);
+  return {d[0], d[1], d[2]};
+}
+
+// Causal attention straight from a packed projection [B,T,3,H,D]: (out [B,H,T,D] in [B,T,H,D] memory order, L, out_lo), and
+// the gradient of the projection as one [B,T,3,H,D] tensor.
+std::tuple<Tensor, Tensor, Tensor> attn_fwd_packed(const Tensor& qkv, const Tensor& slopes, double scale, double eps,
+                                                   const c10::optional<Tensor>& key_mask, bool residual) {
+  TORCH_CHECK(qkv.dim() == 5 && qkv.size(2) == 3, "a packed projection must be [B,T,3,H,D]");
+  const auto h = heads_of(qkv);
+  return attn_fwd(h[0], h[1], h[2], slopes, scale, true, eps, 0, true, key_mask, residual);
+}
+
+Tensor attn_bwd_packed(const Tensor& qkv, const Tensor& out, const Tensor& out_lo, const Tensor& L, const Tensor& d_out,
+                       const Tensor& slopes, double scale, double eps, const c10::optional<Tensor>& key_mask) {
+  const auto h = heads_of(qkv);
+  Tensor packed = empty_of(qkv.sizes(), qkv);
+  const auto d = heads_of(packed);
+  attn_bwd_into(h[0], h[1], h[2], out, out_lo, L, d_out, slopes, scale, true, eps, 0, key_mask, d[0], d[1], d[2]);
+  return packed;
 }
 
 // One decode step over a key/value cache: appends (k_new, v_new) at row n_cached[b] of the caches and returns the
@@ -410,7 +458,7 @@ Tensor attn_decode(const Tensor& q_in, const Tensor& k_new_in, const Tensor& v_n
   const int64_t B = q.size(0), H = q.size(1), D = q.size(2);
   const Tensor sl = slopes.to(at::kFloat).contiguous();
   TORCH_CHECK(sl.numel() == H, "alibi_slopes must hold one slope per head");
-  Tensor out = at::empty({B, H, D}, q.options());
+  Tensor out = empty_of({B, H, D}, q);
   if (q.numel()) {
     c10::cuda::CUDAGuard guard(q.device());
     const std::array<int64_t, 2> qs{q.stride(0), q.stride(1)}, kns{k_new.stride(0), k_new.stride(1)}, vns{v_new.stride(0), v_new.stride(1)},
@@ -428,6 +476,8 @@ Tensor attn_decode(const Tensor& q_in, const Tensor& k_new_in, const Tensor& v_n
 TORCH_LIBRARY(algebraic, m) {
   m.def("swiglu_fwd(Tensor gate, Tensor value) -> Tensor");
   m.def("swiglu_bwd(Tensor d_out, Tensor gate, Tensor value) -> (Tensor, Tensor)");
+  m.def("swiglu_bwd_packed(Tensor d_out, Tensor gate, Tensor value) -> Tensor");
+  m.def("swiglu_bwd_dense(Tensor d_out, Tensor gate, Tensor value) -> (Tensor, Tensor)");
   m.def("norm_fwd(Tensor x, Tensor weight, float eps) -> (Tensor, Tensor)");
   m.def("norm_bwd(Tensor d_out, Tensor x, Tensor weight, Tensor mean, float eps) -> (Tensor, Tensor)");
   m.def("shifted_ce_fwd(Tensor logits, Tensor labels, int ignore_index) -> (Tensor, Tensor)");
@@ -441,6 +491,9 @@ TORCH_LIBRARY(algebraic, m) {
         "bool token_major_out, Tensor? key_mask=None, bool residual=True) -> (Tensor, Tensor, Tensor)");
   m.def("attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor out_lo, Tensor L, Tensor d_out, Tensor slopes, "
         "float scale, bool causal, float eps, int path, Tensor? key_mask=None) -> (Tensor, Tensor, Tensor)");
+  m.def("attn_fwd_packed(Tensor qkv, Tensor slopes, float scale, float eps, Tensor? key_mask, bool residual) -> (Tensor, Tensor, Tensor)");
+  m.def("attn_bwd_packed(Tensor qkv, Tensor out, Tensor out_lo, Tensor L, Tensor d_out, Tensor slopes, float scale, float eps, "
+        "Tensor? key_mask) -> Tensor");
   m.def("pack_key_mask(Tensor mask) -> Tensor");
   m.def("attn_decode(Tensor q, Tensor k_new, Tensor v_new, Tensor(a!) k_cache, Tensor(b!) v_cache, Tensor n_cached, Tensor slopes, "
         "float scale, float eps) -> Tensor");
@@ -450,6 +503,8 @@ TORCH_LIBRARY(algebraic, m) {
 TORCH_LIBRARY_IMPL(algebraic, CUDA, m) {
   m.impl("swiglu_fwd", &swiglu_fwd);
   m.impl("swiglu_bwd", &swiglu_bwd);
+  m.impl("swiglu_bwd_packed", &swiglu_bwd_packed);
+  m.impl("swiglu_bwd_dense", &swiglu_bwd_dense);
   m.impl("norm_fwd", &norm_fwd);
   m.impl("norm_bwd", &norm_bwd);
   m.impl("shifted_ce_fwd", &shifted_ce_fwd);
@@ -461,6 +516,8 @@ TORCH_LIBRARY_IMPL(algebraic, CUDA, m) {
   m.impl("softmax_bwd", &softmax_bwd);
   m.impl("attn_fwd", &attn_fwd);
   m.impl("attn_bwd", &attn_bwd);
+  m.impl("attn_fwd_packed", &attn_fwd_packed);
+  m.impl("attn_bwd_packed", &attn_bwd_packed);
   m.impl("attn_decode", &attn_decode);
   m.impl("pack_key_mask", &pack_key_mask);
 }

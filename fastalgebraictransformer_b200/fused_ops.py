@@ -3,18 +3,22 @@
 Host-side mirror of the reference's ``fused_ops.py`` (autograd Functions 435-599 and the
 convenience functions 606-636): same names, argument meaning and assertion behaviour.  The
 work is done by the sm_100a kernels behind ``torch.ops.algebraic.*``; CPU tensors are
-rejected (this package carries no fallback implementation).
+rejected (this package carries no fallback implementation).  The convenience functions go
+straight to operators whose autograd nodes are C++ (``csrc/torch_autograd.cpp``); the Function
+classes are the same formulas for code that uses them by name or traces them.
 """
 from __future__ import annotations
 
 import torch
 
-from . import ops  # noqa: F401  (registers torch.ops.algebraic)
+from . import ops  # registers torch.ops.algebraic
+from .ops import host as _host
 
 EPS = 1e-6      # added to sums / means, never inside sigma (reference fused_ops.py:20)
 NEG_INF = -1e4  # kept for API parity (reference fused_ops.py:21); the kernels skip masked keys instead
 
 _alg = torch.ops.algebraic
+_compiling = torch.compiler.is_compiling      # a tracer follows the Function classes, not the extension module
 
 
 class RationalSoftmax(torch.autograd.Function):
@@ -47,7 +51,7 @@ class RationalSwiGLU(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_output: torch.Tensor):
         gate, value = ctx.saved_tensors
-        return _alg.swiglu_bwd(grad_output, gate, value)
+        return _alg.swiglu_bwd_dense(grad_output, gate, value)
 
 
 class RationalSwiGLUPacked(torch.autograd.Function):
@@ -184,23 +188,27 @@ def _require_cuda(t: torch.Tensor, what: str) -> None:
 
 def rational_softmax(x: torch.Tensor, eps: float = EPS) -> torch.Tensor:
     """Apply rational softmax to the last dimension (reference fused_ops.py:606-615)."""
-    _require_cuda(x, "rational_softmax")
-    return RationalSoftmax.apply(x, eps)
+    if _compiling():
+        return RationalSoftmax.apply(x, eps)
+    return _host.rational_softmax(x, eps)
 
 
 def rational_swiglu(gate: torch.Tensor, value: torch.Tensor) -> torch.Tensor:
     """Apply the rational SwiGLU activation (reference fused_ops.py:618-626)."""
-    _require_cuda(gate, "rational_swiglu")
-    return RationalSwiGLU.apply(gate, value)
+    if _compiling():
+        return RationalSwiGLU.apply(gate, value)
+    return _host.rational_swiglu(gate, value)
 
 
 def add_mean_error_norm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float = EPS):
     """(x + residual, mean_error_norm(x + residual, weight)) in one pass over the tensors."""
-    _require_cuda(x, "add_mean_error_norm")
-    return AddMeanErrorNorm.apply(x, residual, weight, eps)
+    if _compiling():
+        return AddMeanErrorNorm.apply(x, residual, weight, eps)
+    return _host.add_mean_error_norm(x, residual, weight, eps)
 
 
 def mean_error_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = EPS) -> torch.Tensor:
     """Apply mean-error normalisation (reference fused_ops.py:629-636)."""
-    _require_cuda(x, "mean_error_norm")
-    return MeanErrorNorm.apply(x, weight, eps)
+    if _compiling():
+        return MeanErrorNorm.apply(x, weight, eps)
+    return _host.mean_error_norm(x, weight, eps)

@@ -2,13 +2,17 @@
 
 The operators are defined and implemented in C++ (``csrc/torch_ops.cpp`` -> ``libfat_torch_ops.so``): each one
 allocates its outputs with ATen, passes raw pointers / strides / the current CUDA stream to the C ABI of
-``libfat_b200.so`` and turns a non-zero return code into ``RuntimeError``.  This module loads that library and
-registers, from Python, the shape functions for meta tensors and the autograd formulas, so the operators compose with
-``torch.utils.checkpoint`` (non-reentrant), DDP hooks and ``torch.autograd.grad``.  There is no Python or CPU
-implementation behind them: if the library is missing, importing this module raises.
+``libfat_b200.so`` and turns a non-zero return code into ``RuntimeError``.  The differentiable ones among them
+(``rational_softmax``, ``rational_attention``, ...) have their autograd formulas in C++ (``csrc/torch_autograd.cpp``) and
+are called through ``host``, the same library as an extension module.  This module loads that library and registers,
+from Python, the shape functions for meta tensors and the autograd formulas of the remaining operators, so that all of
+them compose with ``torch.utils.checkpoint`` (non-reentrant), DDP hooks and ``torch.autograd.grad``.  There is no Python
+or CPU implementation behind them: if the library is missing, importing this module raises.
 """
 from __future__ import annotations
 
+import importlib.machinery
+import importlib.util
 import os
 from typing import Optional, Tuple
 
@@ -21,26 +25,26 @@ _NS = "algebraic"
 OPS_LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libfat_torch_ops.so")
 
 
-def _load() -> None:
-    if hasattr(torch.ops.algebraic, "attn_fwd"):
-        return
+def _load():
     for path in (_lib.LIB_PATH, OPS_LIB_PATH):
         if not os.path.exists(path):
             raise RuntimeError(f"{path} is missing: build it with `python -m fastalgebraictransformer_b200.build` "
                                "(nvcc for sm_100a, g++ for the operator registration).  This package has no fallback implementation.")
     _lib.lib()                                  # libfat_b200.so first: the operator library links against it
-    torch.ops.load_library(OPS_LIB_PATH)
+    loader = importlib.machinery.ExtensionFileLoader("libfat_torch_ops", OPS_LIB_PATH)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("libfat_torch_ops", OPS_LIB_PATH, loader=loader))
+    loader.exec_module(module)
+    return module
 
 
-_load()
+host = _load()
 _alg = torch.ops.algebraic
 
 
 def swiglu_bwd_packed(d_out: Tensor, gate: Tensor, value: Tensor) -> Tensor:
     """Both SwiGLU gradients as one [..., 2n] tensor (gate half first): what the gradient of the packed
     projection output needs, without a concatenation."""
-    d_gate, _ = _alg.swiglu_bwd(d_out, gate, value)
-    return d_gate._base if d_gate._base is not None else torch.cat(_alg.swiglu_bwd(d_out, gate, value), -1)
+    return _alg.swiglu_bwd_packed(d_out, gate, value)
 
 
 def head_shifted_ce(y: Tensor, weight: Tensor, labels: Tensor, ignore_index: int,
@@ -98,14 +102,11 @@ def attn_decode(q: Tensor, k_new: Tensor, v_new: Tensor, k_cache: Tensor, v_cach
 def attn_bwd_packed(qkv: Tensor, out: Tensor, out_lo: Tensor, L: Tensor, d_out: Tensor, slopes: Tensor,
                     scale: float, causal: bool, eps: float, path: int, key_mask: Optional[Tensor] = None) -> Tensor:
     """Gradient of a packed [B,T,3,H,D] projection: d_q, d_k, d_v written side by side into one buffer."""
+    if causal and path == 0:
+        return _alg.attn_bwd_packed(qkv, out, out_lo, L, d_out, slopes, float(scale), float(eps), key_mask)
     q, k, v = qkv.permute(2, 0, 3, 1, 4).unbind(0)
-    d_q, d_k, d_v = _alg.attn_bwd(q, k, v, out, out_lo, L, d_out, slopes, float(scale), bool(causal), float(eps), int(path), key_mask)
-    base = d_q._base
-    while base is not None and base._base is not None:
-        base = base._base
-    if base is None or base.shape != qkv.shape:           # q was not token-major after all (H == 1 or T == 1)
-        base = torch.stack((d_q, d_k, d_v), 0).permute(1, 3, 0, 2, 4).contiguous()
-    return base
+    grads = _alg.attn_bwd(q, k, v, out, out_lo, L, d_out, slopes, float(scale), bool(causal), float(eps), int(path), key_mask)
+    return torch.stack(grads, 0).permute(1, 3, 0, 2, 4).contiguous()
 
 
 # ----------------------------------------------------------------------------- shape functions (meta)
@@ -119,6 +120,60 @@ def _(d_out, gate, value):
     n = gate.shape[-1]
     packed = gate.new_empty(gate.shape[:-1] + (2 * n,))
     return packed[..., :n], packed[..., n:]
+
+
+@torch.library.register_fake(f"{_NS}::swiglu_bwd_packed")
+def _(d_out, gate, value):
+    return gate.new_empty(gate.shape[:-1] + (2 * gate.shape[-1],))
+
+
+@torch.library.register_fake(f"{_NS}::swiglu_bwd_dense")
+def _(d_out, gate, value):
+    return tuple(torch.empty_like(t, memory_format=torch.contiguous_format) for t in (gate, value))
+
+
+@torch.library.register_fake(f"{_NS}::rational_swiglu")
+def _(gate, value):
+    return torch.empty_like(gate, memory_format=torch.contiguous_format)
+
+
+@torch.library.register_fake(f"{_NS}::rational_softmax")
+def _(x, eps):
+    return torch.empty_like(x, memory_format=torch.contiguous_format)
+
+
+@torch.library.register_fake(f"{_NS}::mean_error_norm")
+def _(x, weight, eps):
+    return torch.empty_like(x, memory_format=torch.contiguous_format)
+
+
+@torch.library.register_fake(f"{_NS}::add_mean_error_norm")
+def _(x, residual, weight, eps):
+    return tuple(torch.empty_like(x, memory_format=torch.contiguous_format) for _ in range(2))
+
+
+@torch.library.register_fake(f"{_NS}::rational_attention")
+def _(q, k, v, slopes, scale, causal, eps, key_mask, mask_tokens):
+    return q.new_empty(q.shape)
+
+
+@torch.library.register_fake(f"{_NS}::rational_attention_packed")
+def _(qkv, slopes, scale, eps, key_mask, mask_tokens):
+    B, T, _, H, D = qkv.shape
+    return qkv.new_empty((B, T, H * D))
+
+
+@torch.library.register_fake(f"{_NS}::attn_fwd_packed")
+def _(qkv, slopes, scale, eps, key_mask, residual):
+    B, T, _, H, D = qkv.shape
+    out = qkv.new_empty((B, T, H, D)).permute(0, 2, 1, 3)
+    lo = torch.empty_like(out) if qkv.element_size() == 2 and residual else qkv.new_empty(0)
+    return out, qkv.new_empty((B, H, T), dtype=torch.float32), lo
+
+
+@torch.library.register_fake(f"{_NS}::attn_bwd_packed")
+def _(qkv, out, out_lo, L, d_out, slopes, scale, eps, key_mask):
+    return qkv.new_empty(qkv.shape)
 
 
 @torch.library.register_fake(f"{_NS}::norm_fwd")

@@ -270,6 +270,9 @@ FAT_API int fat_attn_bwd(const void* q, const void* k, const void* v, const void
 FAT_API int fat_key_mask_words(int T);
 FAT_API int fat_pack_key_mask(const uint8_t* mask, uint32_t* bits, int B, int T, int64_t mask_batch_stride,
                  int64_t mask_token_stride, void* stream);
+/* The same from a mask of integers of 1, 2, 4 or 8 bytes (any bit set = the key takes part). */
+FAT_API int fat_pack_key_mask_elems(const void* mask, int element_bytes, uint32_t* bits, int B, int T, int64_t mask_batch_stride,
+                 int64_t mask_token_stride, void* stream);
 FAT_API int fat_attn_fwd_masked(const void* q, const void* k, const void* v, const float* slopes, const uint32_t* key_mask_bits,
                  void* out, void* out_lo, float* L, int B, int H, int T, int D,
                  const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides, const int64_t* out_strides,

@@ -453,3 +453,41 @@ def test_head_loss_without_logits_vs_oracle(shape, dtype):
     with torch.no_grad():                              # loss only: no gradient buffers, same number
         loss3 = fat().head_shifted_cross_entropy(y.to(DEV), w.to(DEV), labels.to(DEV), -100)
     assert float(loss3) == float(loss.detach())
+
+
+@pytest.mark.parametrize("n", [64, 7, 1365])
+@pytest.mark.parametrize("use", ["plain", "slices", "non_leaf", "hook", "retain_grad", "grad_of_half", "grad_of_half_and_whole", "other_use",
+                                 "twice"])
+def test_swiglu_of_the_halves_of_a_packed_tensor(n, use):
+    """gate and value taken from one tensor: the backward may hand the packed tensor one gradient and skip the halves, but
+    not when somebody looks at the halves' gradients.  float64 against the oracle formula through plain autograd."""
+    x, go = gen(61, (5, 2 * n), (5, n), dtype=torch.float64)
+    results = []
+    for fn in (fat().rational_swiglu, oracle.rational_swiglu):
+        leaf = x.to(DEV).requires_grad_(True)
+        whole = leaf * 1.5 if use == "non_leaf" else leaf
+        gate, value = (whole[..., :n], whole[..., n:]) if use == "slices" else whole.chunk(2, dim=-1)
+        out, d_out, seen = fn(gate, value), go.to(DEV), []
+        if use == "hook":
+            gate.register_hook(lambda t: seen.append(t.clone()))
+        if use == "retain_grad":
+            value.retain_grad()
+        if use == "other_use":
+            out = out + gate.sin()
+        if use.startswith("grad_of_half"):
+            results.append(torch.autograd.grad(out, (gate, leaf) if use.endswith("whole") else (gate,), d_out))
+            continue
+        if use == "twice":
+            out.backward(d_out, retain_graph=True)
+        out.backward(d_out)
+        results.append([leaf.grad, *seen] + ([value.grad] if use == "retain_grad" else []))
+    assert len(results[0]) == len(results[1])
+    for got, want in zip(*results):
+        assert norm_max_err(got, want) < 1e-12          # float64: a few roundings of 1.1e-16 per element
+
+
+@pytest.mark.parametrize("dtype", [torch.bool, torch.uint8, torch.int16, torch.int32, torch.int64, torch.float32])
+def test_key_mask_of_every_element_type_packs_alike(dtype):
+    from fastalgebraictransformer_b200 import ops
+    mask = torch.arange(2 * 133).view(2, 133) % 3 != 0
+    assert torch.equal(ops.pack_key_mask(mask.to(dtype).to(DEV)), ops.pack_key_mask(mask.to(DEV)))
