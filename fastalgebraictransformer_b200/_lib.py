@@ -52,6 +52,8 @@ PROTOTYPES = {
     "fat_pack_key_mask_elems": (_int, [_ptr, _int, _ptr, _int, _int, _i64, _i64, _ptr]),
     "fat_attn_fwd_masked": (_int, [_ptr] * 8 + [_int] * 4 + [_p64] * 4 + [_dbl, _dbl, _int, _int, _int, _ptr, _ptr]),
     "fat_attn_bwd_masked": (_int, [_ptr] * 13 + [_sz] + [_int] * 4 + [_p64] * 8 + [_dbl, _dbl, _int, _int, _int, _ptr, _ptr]),
+    "fat_lm_decode_workspace_bytes": (_sz, [_int] * 9),
+    "fat_lm_decode_step": (_int, [_ptr, _int, _ptr, _i64] + [_ptr] * 5 + [_p64, _int, _ptr, _sz] + [_int] * 7 + [_dbl] * 3 + [_int, _ptr, _ptr]),
     "fat_attn_decode": (_int, [_ptr] * 8 + [_int] * 4 + [_p64] * 6 + [_dbl, _dbl, _int, _ptr, _ptr]),
 }
 

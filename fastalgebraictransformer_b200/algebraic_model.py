@@ -69,6 +69,7 @@ class KVCache:
         self.v = [torch.empty(batch, n_head, capacity, d_head, dtype=dtype, device=device) for _ in range(n_layers)]
         self.lengths = torch.zeros(batch, dtype=torch.int32, device=device)
         self.seen = 0                                   # host copy of the (common) length
+        self.step = None                                # the fused decode step of the model that fills this cache (_DecodeStep)
 
     def layer(self, i: int):
         return self.k[i], self.v[i], self
@@ -152,6 +153,68 @@ class AlgebraicBlock(nn.Module):
             x, y = add_mean_error_norm(x, pending, self.norm1.weight, self.norm1.eps)
         x, y = add_mean_error_norm(x, self.attn(y, mask, cache), self.norm2.weight, self.norm2.eps)
         return x, self.ffn(y)
+
+
+class _DecodeStep:
+    """What ``lm_decode_step`` (one launch for a whole decode step) needs of a model and a cache, gathered once per cache,
+    and the conditions under which it stands for the modules' own forward passes: stock modules without hooks, nothing
+    that drops out.  ``None`` from ``make`` means the step runs module by module."""
+
+    def __init__(self, parameters, rest, watch, hooks, model):
+        self.parameters, self.rest, self.watch, self.hooks, self.model = parameters, rest, watch, hooks, model
+        self.expected = [d.get(k) for d, k in watch]
+
+    @staticmethod
+    def make(model, cache):
+        stock = {AlgebraicBlock: ("attn", "ffn", "norm1", "norm2"), AlgebraicAttention: ("qkv", "out", "dropout"),
+                 RationalSwiGLU: ("w_gate_val", "w_out", "dropout"), RationalMR: (), nn.Linear: (), nn.Dropout: ()}
+        watch, hooks, modules = [], [], [model.norm, model.head, *model.blocks]
+        for m in modules:                                # (grows while it is walked)
+            if type(m) not in stock or (type(m) is nn.Linear and m.bias is not None):
+                return None
+            modules += [getattr(m, n) for n in stock[type(m)]]
+            watch += [(m._modules, n) for n in stock[type(m)]] + [(m._parameters, n) for n in m._parameters] + [(m.__dict__, "forward")]
+            watch += [(m._buffers, n) for n in m._buffers] + ([(m.__dict__, "training"), (m.__dict__, "p")] if type(m) is nn.Dropout else [])
+            hooks += [m._forward_hooks, m._forward_pre_hooks]
+            if type(m) is nn.Dropout and m.training and m.p > 0:
+                return None
+        if type(model.embed) is not nn.Embedding or model.embed.max_norm is not None:
+            return None
+        watch += [(model._modules, n) for n in ("embed", "norm", "head", "blocks")] + [(model.blocks._modules, n) for n in model.blocks._modules]
+        watch += [(model.embed._parameters, "weight"), (model.embed.__dict__, "forward")]
+        hooks += [model.embed._forward_hooks, model.embed._forward_pre_hooks, torch.nn.modules.module._global_forward_hooks,
+                  torch.nn.modules.module._global_forward_pre_hooks]
+        first, norms = model.blocks[0], [model.norm] + [n for b in model.blocks for n in (b.norm1, b.norm2)]
+        params = [w for b in model.blocks for w in (b.norm1.weight, b.attn.qkv.weight, b.attn.out.weight, b.norm2.weight,
+                                                    b.ffn.w_gate_val.weight, b.ffn.w_out.weight)]
+        tops = [model.embed.weight, model.norm.weight, model.head.weight]
+        slopes = [b.attn.alibi_slopes for b in model.blocks]
+        dtype, device = tops[2].dtype, tops[2].device
+        if (any(w.dtype != dtype or w.device != device or not w.is_contiguous() for w in params + tops) or cache.k[0].dtype != dtype or
+                any(s.dtype not in (dtype, torch.float32) or s.dtype != slopes[0].dtype for s in slopes) or len({n.eps for n in norms}) > 1 or
+                len({(b.attn.n_head, b.attn.scale, *b.ffn.w_out.weight.shape) for b in model.blocks}) > 1):
+            return None
+        B, H, capacity, D = cache.k[0].shape
+        nbytes = torch.ops.algebraic.lm_decode_workspace_bytes(B, tops[2].shape[1], H, D, first.ffn.w_out.weight.shape[1], tops[2].shape[0],
+                                                               len(params) // 6, capacity, dtype)
+        if nbytes == 0:
+            return None
+        workspace = torch.zeros(nbytes, dtype=torch.uint8, device=device)
+        step = _DecodeStep((*tops, params, slopes), (workspace, float(first.attn.scale), float(model.norm.eps), float(EPS)), watch, hooks, model)
+        return step if step.stands(model) else None
+
+    def stands(self, model) -> bool:
+        """Whether the model is still the one this step was made of (a parameter may be changed in place or moved; the
+        launch takes its address anew)."""
+        if model is not self.model or any(self.hooks) or torch.is_autocast_enabled("cuda"):
+            return False
+        for have, want in zip([d.get(k) for d, k in self.watch], self.expected):
+            if have is not want:
+                return False
+        return True
+
+    def __call__(self, input_ids, cache):
+        return torch.ops.algebraic.lm_decode_step(input_ids, *self.parameters, cache.k, cache.v, cache.lengths, *self.rest)
 
 
 class AlgebraicTransformerLM(nn.Module):
@@ -239,7 +302,17 @@ class AlgebraicTransformerLM(nn.Module):
         """Logits [B, V] of the LAST position of ``input_ids`` given the tokens already in ``cache``.  With an empty cache
         ``input_ids`` is the prompt (any length); afterwards it is the one token per sequence that was sampled last.
         Same arithmetic as ``forward`` on the concatenated sequence: keys and values of earlier positions do not
-        depend on later tokens (causal attention, relative bias), so they are kept instead of recomputed."""
+        depend on later tokens (causal attention, relative bias), so they are kept instead of recomputed.  A step of one
+        token per sequence runs as one launch where the fused step covers the model (``_DecodeStep``)."""
+        if cache.seen > 0 and input_ids.dim() == 2 and input_ids.size(1) == 1 and input_ids.dtype == torch.int64 and input_ids.is_cuda:
+            if cache.seen >= cache.capacity:
+                raise RuntimeError(f"key/value cache is full ({cache.capacity} tokens)")
+            if cache.step is None or (cache.step is not False and not cache.step.stands(self)):
+                cache.step = _DecodeStep.make(self, cache) or False
+            if cache.step and input_ids.size(0) == cache.lengths.numel():
+                logits = cache.step(input_ids, cache)
+                cache.seen += 1                          # (the launch has advanced the device-side lengths)
+                return logits
         x = self.embed(input_ids)
         pending = None
         for i, block in enumerate(self.blocks):

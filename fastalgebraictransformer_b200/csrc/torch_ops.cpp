@@ -471,6 +471,48 @@ Tensor attn_decode(const Tensor& q_in, const Tensor& k_new_in, const Tensor& v_n
   return out;
 }
 
+// Bytes of the (zeroed) workspace lm_decode_step needs, 0 when it does not cover the shape.
+int64_t lm_decode_workspace_bytes(int64_t B, int64_t C, int64_t H, int64_t D, int64_t F, int64_t V, int64_t n_layers, int64_t capacity,
+                                  at::ScalarType dtype) {
+  const int tag = dtype == at::kBFloat16 ? FAT_BF16 : dtype == at::kHalf ? FAT_F16 : -1;
+  return int64_t(fat_lm_decode_workspace_bytes(int(B), int(C), int(H), int(D), int(F), int(V), int(n_layers), int(capacity), tag));
+}
+
+// Logits [B, V] of the tokens ids [B, 1] that follow the cached ones; appends to the caches and advances `lengths`.
+// params: norm1, qkv, out, norm2, gate_val, down of every layer in turn; slopes, k, v: one per layer.
+Tensor lm_decode_step(const Tensor& ids, const Tensor& embed, const Tensor& norm, const Tensor& head, at::TensorList params, at::TensorList slopes,
+                      at::TensorList k, at::TensorList v, Tensor& lengths, Tensor& workspace, double scale, double eps_norm, double eps_attn) {
+  const int64_t L = int64_t(k.size()), B = ids.size(0), C = norm.size(0), V = head.size(0);
+  TORCH_CHECK(L >= 1 && L <= FAT_LM_MAX_LAYERS && int64_t(params.size()) == 6 * L && int64_t(slopes.size()) == L && int64_t(v.size()) == L, "one set of tensors per layer expected");
+  const int64_t H = k[0].size(1), cap = k[0].size(2), D = k[0].size(3), F = params[5].size(1);
+  const auto dtype = head.scalar_type();
+  auto param = [&](const Tensor& t, at::IntArrayRef shape) {
+    TORCH_CHECK(t.is_cuda() && t.device() == head.device() && t.scalar_type() == dtype && t.is_contiguous() && t.sizes() == shape, "parameters must be dense CUDA tensors of the model's dtype and shapes");
+    return t.data_ptr();
+  };
+  TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.dim() == 2 && ids.size(1) == 1, "ids must be int64 [B, 1]");
+  TORCH_CHECK(lengths.is_cuda() && lengths.scalar_type() == at::kInt && lengths.is_contiguous() && lengths.numel() == B, "lengths must be int32 [B]");
+  const int slopes_f32 = slopes[0].scalar_type() == at::kFloat;
+  const auto cs = strides3(k[0]);
+  std::array<fat_lm_layer, FAT_LM_MAX_LAYERS> layers;
+  for (int64_t i = 0; i < L; ++i) {
+    const Tensor* w = &params[6 * i];
+    TORCH_CHECK(slopes[i].is_cuda() && slopes[i].is_contiguous() && slopes[i].numel() == H && slopes[i].scalar_type() == (slopes_f32 ? at::kFloat : dtype), "one dense slope per head expected");
+    for (const Tensor* c : {&k[i], &v[i]})
+      TORCH_CHECK(c->is_cuda() && c->scalar_type() == dtype && c->stride(3) == 1 && c->sizes() == k[0].sizes() && c->strides() == k[0].strides(), "the layers' caches must be alike");
+    layers[i] = {param(w[0], {C}), param(w[1], {3 * C, C}), param(w[2], {C, C}), param(w[3], {C}), param(w[4], {2 * F, C}), param(w[5], {C, F}),
+                 k[i].data_ptr(), v[i].data_ptr(), slopes[i].data_ptr()};
+  }
+  TORCH_CHECK(k[0].size(0) == B && C == H * D, "the caches must be [B,H,capacity,D] of the model");
+  Tensor logits = empty_of({B, V}, head);
+  c10::cuda::CUDAGuard guard(head.device());
+  check(fat_lm_decode_step(layers.data(), int(L), ids.data_ptr<int64_t>(), ids.stride(0), param(embed, {V, C}), param(norm, {C}), param(head, {V, C}),
+                           logits.data_ptr(), lengths.data_ptr<int>(), cs.data(), slopes_f32, workspace.data_ptr(), size_t(workspace.numel()),
+                           int(B), int(C), int(H), int(D), int(F), int(V), int(cap), scale, eps_norm, eps_attn, dtype_tag(head),
+                           status_word(head.get_device()).data_ptr<int>(), stream_of(head)));
+  return logits;
+}
+
 }  // namespace
 
 TORCH_LIBRARY(algebraic, m) {
@@ -497,6 +539,10 @@ TORCH_LIBRARY(algebraic, m) {
   m.def("pack_key_mask(Tensor mask) -> Tensor");
   m.def("attn_decode(Tensor q, Tensor k_new, Tensor v_new, Tensor(a!) k_cache, Tensor(b!) v_cache, Tensor n_cached, Tensor slopes, "
         "float scale, float eps) -> Tensor");
+  m.def("lm_decode_workspace_bytes(int B, int C, int H, int D, int F, int V, int n_layers, int capacity, ScalarType dtype) -> int",
+        &lm_decode_workspace_bytes);
+  m.def("lm_decode_step(Tensor ids, Tensor embed, Tensor norm, Tensor head, Tensor[] params, Tensor[] slopes, Tensor[] k, Tensor[] v, "
+        "Tensor(a!) lengths, Tensor(b!) workspace, float scale, float eps_norm, float eps_attn) -> Tensor");
   m.def("device_status(int device) -> Tensor", &device_status);
 }
 
@@ -520,4 +566,5 @@ TORCH_LIBRARY_IMPL(algebraic, CUDA, m) {
   m.impl("attn_bwd_packed", &attn_bwd_packed);
   m.impl("attn_decode", &attn_decode);
   m.impl("pack_key_mask", &pack_key_mask);
+  m.impl("lm_decode_step", &lm_decode_step);
 }

@@ -307,6 +307,30 @@ FAT_API int fat_attn_decode(const void* q, const void* k_new, const void* v_new,
                  const int64_t* out_strides, const int64_t* k_cache_strides, const int64_t* v_cache_strides,
                  double scale, double eps, int dtype, int* status, void* stream);
 
+/* ------------------------------------------------------------------------------------
+ * One decode step of the whole language model over its key/value caches, as one cooperative launch: logits[b] of the token
+ * ids[b * ids_stride] that follows the n_cached[b] tokens already in the caches.  Same arithmetic as
+ * AlgebraicTransformerLM.forward on the last position (algebraic_model.py:209-227 with the blocks of 139-152): the new key
+ * and value rows are appended to every layer's caches and n_cached[b] is incremented.
+ * Parameters are dense row-major in the nn.Linear convention ([out, in]): qkv [3C, C], out [C, C], gate_val [2F, C],
+ * down [C, F], head [V, C], embed [V, C]; C = H * D.  Caches [B, H, capacity, D] with the given (batch, head, token)
+ * element strides, the same for all layers.  slopes: H values per layer, float32 (slopes_f32) or of the tensor dtype.
+ * workspace: fat_lm_decode_workspace_bytes bytes (0: the shape is not covered), zeroed once before its first use, used by
+ * one step at a time.  Covered: 1-16 sequences, D in {64, 128}, up to FAT_LM_MAX_LAYERS layers, activation rows that fit
+ * shared memory.  An id outside [0, V) gives that sequence NaN logits.  dtypes: BF16, F16.
+ * ---------------------------------------------------------------------------------- */
+#define FAT_LM_MAX_LAYERS 48
+typedef struct fat_lm_layer {
+  const void *norm1, *qkv, *out, *norm2, *gate_val, *down;
+  void *k_cache, *v_cache;
+  const void* slopes;
+} fat_lm_layer;
+FAT_API size_t fat_lm_decode_workspace_bytes(int B, int C, int H, int D, int F, int V, int n_layers, int capacity, int dtype);
+FAT_API int fat_lm_decode_step(const fat_lm_layer* layers, int n_layers, const int64_t* ids, int64_t ids_stride, const void* embed,
+                 const void* norm, const void* head, void* logits, int32_t* n_cached, const int64_t* cache_strides,
+                 int slopes_f32, void* workspace, size_t workspace_bytes, int B, int C, int H, int D, int F, int V,
+                 int capacity, double scale, double eps_norm, double eps_attn, int dtype, int* status, void* stream);
+
 /* Which kernel family FAT_PATH_AUTO would pick for these arguments (FAT_PATH_SIMT or
  * FAT_PATH_TENSOR), for the forward (backward = 0) or the backward (backward = 1) launch.
  * Host-only, no launch. */

@@ -195,3 +195,61 @@ def test_decode_first_token_of_an_empty_cache(dtype):
     else:
         assert bf16_violations(got, want)[0] == 0.0
     assert torch.equal(kd[:, :, 0].cpu(), k_new) and torch.equal(vd[:, :, 0].cpu(), v_new)
+
+
+@pytest.mark.parametrize("dtype,d_model,n_head,d_ffn,vocab,B,prompt", [
+    (torch.bfloat16, 256, 4, None, 1000, 8, 70),        # d_ffn 682: rows of the down projection only 4-byte aligned; keys shared by CTAs
+    (torch.bfloat16, 512, 8, None, 509, 1, 300),        # d_ffn 1365: 2-byte aligned, ragged last units; many key shares
+    (torch.float16, 768, 6, 2048, 1000, 9, 40),         # nine tokens: the second half of the MMA rows; heads of 128
+    (torch.bfloat16, 768, 12, 2048, 777, 16, 33),       # more (batch, head) pairs than SMs
+    (torch.float16, 64, 1, 40, 64, 2, 1),               # less than one unit per warp group
+])
+def test_fused_decode_step_equals_the_modules_and_the_oracle(dtype, d_model, n_head, d_ffn, vocab, B, prompt):
+    """The whole step as one launch: logits, caches and lengths against the module-by-module step on the same caches, and
+    the logits against the float32 oracle of the full forward."""
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM, check_device_status
+    torch.manual_seed(19)
+    model = AlgebraicTransformerLM(vocab_size=vocab, d_model=d_model, n_head=n_head, n_layers=2, d_ffn=d_ffn, dropout=0.0, block_size=512)
+    n = prompt + 4
+    ids = torch.randint(0, vocab, (B, n))
+    state = {k: v.detach().to(dtype).float() for k, v in model.state_dict().items() if k != "embed.weight" and not k.endswith("alibi_slopes")}
+    want, _ = oracle.lm_forward(state, ids, n_head)
+    model, ids = model.to(DEV).to(dtype).eval(), ids.to(DEV)
+    caches, logits = [model.new_cache(B, n) for _ in range(2)], []
+    for fused, cache in enumerate(caches):
+        model.forward_cached(ids[:, :prompt], cache)
+        if not fused:
+            cache.step = False                          # module by module
+        logits.append([model.forward_cached(ids[:, t:t + 1], cache) for t in range(prompt, n)])
+    assert caches[1].step and not caches[0].step
+    check_device_status()
+    assert caches[1].lengths.tolist() == [n] * B and caches[1].seen == n
+    # the two round at the same places and differ in the order of float32 sums: now and then a 16-bit rounding falls to the
+    # other side (2^-9 or 2^-11 of one element), which two layers turn into a few times that of the largest logit
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in zip(*logits):
+        assert norm_max_err(b, a) < 4 * eps
+    for t, got in enumerate(logits[1]):
+        assert norm_max_err(got, want[:, prompt + t]) < 3e-2
+    for side in ("k", "v"):
+        for a, b in zip(getattr(caches[0], side), getattr(caches[1], side)):
+            assert norm_max_err(b, a) < 4 * eps
+
+
+def test_fused_decode_step_yields_to_hooks_and_replaced_modules():
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM
+    torch.manual_seed(3)
+    model = AlgebraicTransformerLM(vocab_size=64, d_model=128, n_head=2, n_layers=2, dropout=0.0, block_size=64).to(DEV).to(torch.bfloat16).eval()
+    ids = torch.randint(0, 64, (2, 12), device=DEV)
+    cache = model.new_cache(2, 12)
+    model.forward_cached(ids[:, :4], cache)
+    model.forward_cached(ids[:, 4:5], cache)
+    assert cache.step
+    calls = []
+    handle = model.blocks[1].attn.qkv.register_forward_hook(lambda *a: calls.append(1))
+    model.forward_cached(ids[:, 5:6], cache)
+    assert calls == [1]
+    handle.remove()
+    model.blocks[0].ffn.w_out = torch.nn.Sequential(model.blocks[0].ffn.w_out)
+    model.forward_cached(ids[:, 6:7], cache)
+    assert cache.step is False and cache.lengths.tolist() == [7, 7] and cache.seen == 7
