@@ -2,111 +2,173 @@
 // (tensor cores cannot hold the 1e-5 bar in one pass), for head sizes the tcgen05 kernels
 // do not cover, and the on-device cross-check of the tcgen05 path.
 //
-// Tiling: 64 queries x 64 keys per step, 256 threads as a 16x16 grid.  Thread (ty,tx) owns
-// score rows {ty+16i} and score columns {tx+16j}; Q/K/V tiles live in shared memory as
-// float with rows padded by 4 floats, so every 128-bit shared load is conflict free.
-// Forward keeps a running sum of sigma^4 only (sigma^4 <= 1, nothing to rescale).  Backward
-// is two kernels without atomics: a query-major one (Delta, d_q) and a key-major one
-// (d_k, d_v), each recomputing the scores it needs.
+// What bounds it: the FMA pipe, as long as shared memory, issue slots and latencies keep up.  A CTA owns kOwn = 32 queries
+// (forward, d_q) or keys (d_k/d_v) and streams tiles of kStream = 64 rows of the other side.  Short own tiles, handed out
+// longest first over all heads, because small problems have few of them: 2x12 heads of 512 tokens are 384 CTAs of 1-8 steps;
+// 64-row tiles left 192 for 148 SMs and twice the longest one's time.  128 threads; a warp covers 16 x 32 scores, a thread
+// 4 x 4 (rows 4 apart, columns 8 apart), so that no shared load has bank conflicts.  FMAs are issued as float32 pairs
+// (fma.rn.f32x2: same pipe time, half the issue slots): along the head dimension in the score products, along the output
+// columns in the others, whose weights lie doubled (w, w) in shared memory so that no register moves build the pairs.
+// float32 tiles arrive by cp.async, each while a contraction that does not need its buffer runs.
+// 2x12 heads, 512 tokens, D = 64, float32: forward 97 -> 57 us, d_q 133 -> 79 us, d_k/d_v 152 -> 78 us (64-row tiles of 256
+// threads with synchronous loads before).  FMA pipe 40-45 % busy on an active SM at 8 warps per SM (before: 15-20 %): latency of
+// the shared loads, and an SM's share of the CTAs (71 % of the longest SM's time on average).
+// Backward is two kernels without atomics: a query-major one (Delta, d_q) and a key-major one (d_k, d_v), each
+// recomputing the scores it needs.  No running maximum anywhere (sigma^4 <= 1).
 #include "attn_common.cuh"
 
 namespace fat {
 namespace {
 
-constexpr int BM = 64, BN = 64, NT = 256;
-constexpr int LDP = BN + 4;
+constexpr int kOwn = 32, kStream = 64, NT = 128;
+constexpr int kPairLd = 2 * kStream + 4;        // pitch of the doubled weights [kOwn][kStream] in floats
 
-template <typename T, int DP>
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void upk2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+
+// This thread's place: score rows row(i) of the own tile, score columns col(j) of the streamed tile.
+struct Lane {
+  int ly, lx, wy, wx;
+  __device__ __forceinline__ Lane() : ly((threadIdx.x & 31) >> 3), lx(threadIdx.x & 7), wy(threadIdx.x >> 6), wx((threadIdx.x >> 5) & 1) {}
+  __device__ __forceinline__ int row(int i) const { return wy * 16 + ly + 4 * i; }
+  __device__ __forceinline__ int col(int j) const { return wx * 32 + lx + 8 * j; }
+};
+
+// The CTA's tile: the grid runs over (tile, batch, head) with the tile slowest, whatever the caller wants first.
+struct Tile { int b, h, tile; };
+__device__ __forceinline__ Tile this_tile(const AttnParams& p) {
+  const int tiles = (p.T + kOwn - 1) / kOwn, group = gridDim.x / tiles;         // H * B, or H with the batch on the y axis
+  const int bh = blockIdx.y * group + blockIdx.x % group;
+  return Tile{bh / p.H, bh % p.H, int(blockIdx.x) / group};
+}
+
+// dst[ROWS][DP + 4] = rows row0.. of base as float, zeros beyond T_len and D.  float32 rows that can be moved in 16-byte
+// pieces are copied asynchronously (the caller waits with copies_done), everything else is there on return.
+template <typename T, int DP, int ROWS>
 __device__ __forceinline__ void load_tile(float* __restrict__ dst, const T* __restrict__ base,
                                           int64_t row_stride, int row0, int T_len, int D, bool vec) {
   constexpr int LD = DP + 4;
   constexpr int W = 16 / sizeof(T);
   if (vec) {
     constexpr int PPR = DP / W;
-    for (int idx = threadIdx.x; idx < BM * PPR; idx += NT) {
-      const int r = idx / PPR, c = (idx % PPR) * W, row = row0 + r;
-      float vals[W];
-      if (row < T_len && c < D) {
-        load_pack_cached<T, W>(base + int64_t(row) * row_stride + c, vals);
-      } else {
-#pragma unroll
-        for (int j = 0; j < W; ++j) vals[j] = 0.f;
+    if constexpr (sizeof(T) == 4) {
+      const uint32_t s0 = uint32_t(__cvta_generic_to_shared(dst));
+#pragma unroll 4
+      for (int idx = threadIdx.x; idx < ROWS * PPR; idx += NT) {
+        const int r = idx / PPR, c = (idx % PPR) * W, row = row0 + r;
+        const bool in = row < T_len && c < D;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s0 + uint32_t(r * LD + c) * 4u),
+                     "l"(base + (in ? int64_t(row) * row_stride + c : 0)), "r"(in ? 16u : 0u) : "memory");
       }
+    } else {
+#pragma unroll 2
+      for (int idx = threadIdx.x; idx < ROWS * PPR; idx += NT) {
+        const int r = idx / PPR, c = (idx % PPR) * W, row = row0 + r;
+        float vals[W];
+        if (row < T_len && c < D) {
+          load_pack_cached<T, W>(base + int64_t(row) * row_stride + c, vals);
+        } else {
 #pragma unroll
-      for (int j = 0; j < W; j += 4)
-        *reinterpret_cast<float4*>(&dst[r * LD + c + j]) = make_float4(vals[j], vals[j + 1], vals[j + 2], vals[j + 3]);
+          for (int j = 0; j < W; ++j) vals[j] = 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < W; j += 4)
+          *reinterpret_cast<float4*>(&dst[r * LD + c + j]) = make_float4(vals[j], vals[j + 1], vals[j + 2], vals[j + 3]);
+      }
     }
   } else {
-    for (int idx = threadIdx.x; idx < BM * DP; idx += NT) {
+    for (int idx = threadIdx.x; idx < ROWS * DP; idx += NT) {
       const int r = idx / DP, c = idx % DP, row = row0 + r;
       dst[r * LD + c] = (row < T_len && c < D) ? Elem<T>::to_c(base[int64_t(row) * row_stride + c]) : 0.f;
     }
   }
 }
+// Every copy of this thread has landed / those of all threads are visible.
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void copies_visible() { copies_done(); __syncthreads(); }
 
-// acc[i][j] += sum_d A[ty+16i][d] * Bm[tx+16j][d]
+// s[i][j] = sum_d A[row(i)][d] * Bm[col(j)][d]     (A is [kOwn][DP+4], Bm is [kStream][DP+4])
 template <int DP>
-__device__ __forceinline__ void gemm_nt(float (&acc)[4][4], const float* __restrict__ A,
-                                        const float* __restrict__ Bm, int ty, int tx) {
+__device__ __forceinline__ void gemm_nt(float (&s)[4][4], const float* __restrict__ A, const float* __restrict__ Bm, const Lane& ln) {
   constexpr int LD = DP + 4;
-#pragma unroll 2
+  f32x2 acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+  const float* a0 = A + ln.row(0) * LD;
+  const float* b0 = Bm + ln.col(0) * LD;
+#pragma unroll 4
   for (int d = 0; d < DP; d += 4) {
-    float4 a[4], b[4];
+    ulonglong2 a[4], b[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(&A[(ty + 16 * i) * LD + d]);
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a0 + 4 * i * LD + d);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(&Bm[(tx + 16 * j) * LD + d]);
+    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(b0 + 8 * j * LD + d);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-        acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-        acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-        acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
-      }
+      for (int j = 0; j < 4; ++j) acc[i][j] = fma2(a[i].x, b[j].x, acc[i][j]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = fma2(a[i].y, b[j].y, acc[i][j]);
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float lo, hi;
+      upk2(acc[i][j], lo, hi);
+      s[i][j] = lo + hi;
+    }
 }
 
-// Column ownership of the [64][DP] output tiles: thread tx owns VW consecutive columns in
-// each of NCH chunks, chunk c starting at column c*16*VW.
+// Columns of the [kOwn][DP] outputs: a warp has one half of them, a lane VW neighbours in each of NCH chunks.
 template <int DP> struct OutCols {
   static constexpr int VW = DP >= 64 ? 4 : 2;
   static constexpr int NCH = DP / 16 / VW;
-  static constexpr int N = DP / 16;
-  static __device__ __forceinline__ int col(int tx, int c, int e) { return c * 16 * VW + tx * VW + e; }
+  static constexpr int NP = DP / 32;                                            // pairs per thread and row
+  static __device__ __forceinline__ int col(const Lane& ln, int c) { return ln.wx * (DP / 2) + c * 8 * VW + ln.lx * VW; }
 };
+template <int DP> struct Out { f32x2 v[4][OutCols<DP>::NP]; };
+template <int DP> __device__ __forceinline__ void clear(Out<DP>& o) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int n = 0; n < OutCols<DP>::NP; ++n) o.v[i][n] = 0ull;
+}
 
-// o[i][*] += sum_k P[ty+16i][k] * V[k][cols(tx)]     (P is [64][LDP], V is [64][DP+4])
+// o[row(i)][*] += sum_k W[row(i)][k] * V[k][*]     (W doubled, V is [kStream][DP+4])
 template <int DP>
-__device__ __forceinline__ void gemm_nn(float (&o)[4][DP / 16], const float* __restrict__ P,
-                                        const float* __restrict__ V, int ty, int tx) {
+__device__ __forceinline__ void gemm_nn(Out<DP>& o, const float* __restrict__ W, const float* __restrict__ V, const Lane& ln) {
   using OC = OutCols<DP>;
   constexpr int LD = DP + 4;
-#pragma unroll 2
-  for (int k = 0; k < BN; k += 4) {
-    float4 p4[4];
+  const float* w0 = W + ln.row(0) * kPairLd;
+#pragma unroll 4
+  for (int k = 0; k < kStream; k += 2) {
+    ulonglong2 w[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) p4[i] = *reinterpret_cast<const float4*>(&P[(ty + 16 * i) * LDP + k]);
+    for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const ulonglong2*>(w0 + 4 * i * kPairLd + 2 * k);
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      float vv[OC::N];
+    for (int kk = 0; kk < 2; ++kk) {
+      f32x2 v[OC::NP];
 #pragma unroll
       for (int c = 0; c < OC::NCH; ++c) {
+        const float* at = V + (k + kk) * LD + OC::col(ln, c);
         if constexpr (OC::VW == 4) {
-          const float4 t = *reinterpret_cast<const float4*>(&V[(k + kk) * LD + OC::col(tx, c, 0)]);
-          vv[c * 4 + 0] = t.x; vv[c * 4 + 1] = t.y; vv[c * 4 + 2] = t.z; vv[c * 4 + 3] = t.w;
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(at);
+          v[2 * c] = t.x;
+          v[2 * c + 1] = t.y;
         } else {
-          const float2 t = *reinterpret_cast<const float2*>(&V[(k + kk) * LD + OC::col(tx, c, 0)]);
-          vv[c * 2 + 0] = t.x; vv[c * 2 + 1] = t.y;
+          v[c] = *reinterpret_cast<const f32x2*>(at);
         }
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float pv = kk == 0 ? p4[i].x : kk == 1 ? p4[i].y : kk == 2 ? p4[i].z : p4[i].w;
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int n = 0; n < OC::N; ++n) o[i][n] = fmaf(pv, vv[n], o[i][n]);
-      }
+        for (int n = 0; n < OC::NP; ++n) o.v[i][n] = fma2(kk ? w[i].y : w[i].x, v[n], o.v[i][n]);
     }
   }
 }
@@ -114,26 +176,31 @@ __device__ __forceinline__ void gemm_nn(float (&o)[4][DP / 16], const float* __r
 // Writes o*mul to `base`; when `lo` is given also writes the rounding residual round(o*mul - stored).
 template <typename T, int DP>
 __device__ __forceinline__ void store_rows(T* __restrict__ base, int64_t row_stride, int row0, int T_len, int D,
-                                           const float (&o)[4][DP / 16], const float (&mul)[4], int ty, int tx,
-                                           T* __restrict__ lo = nullptr) {
+                                           const Out<DP>& o, const float (&mul)[4], const Lane& ln, T* __restrict__ lo = nullptr) {
   using OC = OutCols<DP>;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int row = row0 + ty + 16 * i;
+    const int row = row0 + ln.row(i);
     if (row >= T_len) continue;
 #pragma unroll
-    for (int c = 0; c < OC::NCH; ++c)
+    for (int n = 0; n < OC::NP; ++n) {
+      float val[2];
+      upk2(o.v[i][n], val[0], val[1]);
+      const int col = OC::col(ln, 2 * n / OC::VW) + 2 * n % OC::VW;
 #pragma unroll
-      for (int e = 0; e < OC::VW; ++e) {
-        const int col = OC::col(tx, c, e);
-        if (col < D) {
-          const float val = o[i][c * OC::VW + e] * mul[i];
-          const T hi = Elem<T>::from_c(val);
-          base[int64_t(row) * row_stride + col] = hi;
-          if (lo) lo[int64_t(row) * row_stride + col] = Elem<T>::from_c(val - Elem<T>::to_c(hi));
+      for (int e = 0; e < 2; ++e)
+        if (col + e < D) {
+          const float x = val[e] * mul[i];
+          const T hi = Elem<T>::from_c(x);
+          base[int64_t(row) * row_stride + col + e] = hi;
+          if (lo) lo[int64_t(row) * row_stride + col + e] = Elem<T>::from_c(x - Elem<T>::to_c(hi));
         }
-      }
+    }
   }
+}
+
+__device__ __forceinline__ void put_pair(float* W, int row, int col, float w) {
+  *reinterpret_cast<float2*>(W + row * kPairLd + 2 * col) = make_float2(w, w);
 }
 
 struct Score { float f, k; };   // f = sigma^4, k = 2 sigma^3 r^2 (derivative of f w.r.t. the score)
@@ -148,138 +215,159 @@ __device__ __forceinline__ Score score_terms(float qk, float scale, float slope,
 
 // ------------------------------------------------------------------ forward
 template <typename T, int DP>
-__global__ void __launch_bounds__(NT) attn_fwd_simt_kernel(AttnParams p, bool vec) {
+__global__ void __launch_bounds__(NT, DP > 64 ? 2 : 4) attn_fwd_simt_kernel(AttnParams p, bool vec) {
   extern __shared__ __align__(16) float smem[];
   constexpr int LD = DP + 4;
-  float* Qs = smem; float* Ks = Qs + BM * LD; float* Vs = Ks + BN * LD; float* Ps = Vs + BN * LD;
-  const int b = blockIdx.z, h = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;   // long rows first
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const int q0 = qt * BM;
+  float* Qs = smem; float* Ks = Qs + kOwn * LD; float* Vs = Ks + kStream * LD; float* Ps = Vs + kStream * LD;
+  const Lane ln;
+  const Tile tl = this_tile(p);
+  const int b = tl.b, h = tl.h, n_tiles = (p.T + kOwn - 1) / kOwn;
+  const int q0 = (n_tiles - 1 - tl.tile) * kOwn;                               // long rows first
   const T* qb = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const T* kb = static_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* vb = static_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
   T* ob = static_cast<T*>(p.out) + b * p.os[0] + h * p.os[1];
   const float slope = p.slopes[h];
 
-  load_tile<T, DP>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
-  float o[4][DP / 16] = {};
+  load_tile<T, DP, kOwn>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
+  load_tile<T, DP, kStream>(Ks, kb, p.ks[2], 0, p.T, p.D, vec);
+  Out<DP> o;
+  clear(o);
   float l[4] = {0.f, 0.f, 0.f, 0.f};
-  const int n_kt = p.causal ? qt + 1 : (p.T + BN - 1) / BN;
-  for (int kt = 0; kt < n_kt; ++kt) {
-    const int k0 = kt * BN;
-    load_tile<T, DP>(Ks, kb, p.ks[2], k0, p.T, p.D, vec);
-    load_tile<T, DP>(Vs, vb, p.vs[2], k0, p.T, p.D, vec);
-    __syncthreads();
-    float acc[4][4] = {};
-    gemm_nt<DP>(acc, Qs, Ks, ty, tx);
+  const int k_end = p.causal ? min(p.T, q0 + kOwn) : p.T;
+#pragma unroll 1
+  for (int k0 = 0; k0 < k_end; k0 += kStream) {
+    copies_visible();                                                          // K is there, V and the weights are free
+    load_tile<T, DP, kStream>(Vs, vb, p.vs[2], k0, p.T, p.D, vec);
+    float s[4][4];
+    gemm_nt<DP>(s, Qs, Ks, ln);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = q0 + ty + 16 * i;
+    for (int j = 0; j < 4; ++j) {
+      const int col = k0 + ln.col(j);
+      const bool kept = col < p.T && key_kept(p, b, col);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = k0 + tx + 16 * j;
-        const bool live = col < p.T && row < p.T && (!p.causal || col <= row) && key_kept(p, b, col);
-        const float f = live ? score_terms(acc[i][j], p.scale, slope, row, col).f : 0.f;
+      for (int i = 0; i < 4; ++i) {
+        const int row = q0 + ln.row(i);
+        const bool live = kept && row < p.T && (!p.causal || col <= row);
+        const float f = live ? score_terms(s[i][j], p.scale, slope, row, col).f : 0.f;
         l[i] += f;
-        Ps[(ty + 16 * i) * LDP + tx + 16 * j] = f;
+        put_pair(Ps, ln.row(i), ln.col(j), f);
       }
     }
-    __syncthreads();
-    gemm_nn<DP>(o, Ps, Vs, ty, tx);
-    __syncthreads();
+    copies_visible();                                                          // V is there, K is free
+    if (k0 + kStream < k_end) load_tile<T, DP, kStream>(Ks, kb, p.ks[2], k0 + kStream, p.T, p.D, vec);
+    gemm_nn<DP>(o, Ps, Vs, ln);
   }
+  // a row's sum: over the eight lanes that share it, then over the two warps
+  float* part = Qs;                                                            // (every score has been formed)
   float inv[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
 #pragma unroll
-    for (int m = 8; m > 0; m >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], m);
-    inv[i] = 1.f / (l[i] + p.eps);
-    const int row = q0 + ty + 16 * i;
-    if (tx == 0 && row < p.T) p.L[(int64_t(b) * p.H + h) * p.T + row] = l[i];
+    for (int m = 4; m > 0; m >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], m);
+    if (ln.lx == 0) part[ln.wx * kOwn + ln.row(i)] = l[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float sum = part[ln.row(i)] + part[kOwn + ln.row(i)];
+    inv[i] = 1.f / (sum + p.eps);
+    const int row = q0 + ln.row(i);
+    if (ln.wx == 0 && ln.lx == 0 && row < p.T) p.L[(int64_t(b) * p.H + h) * p.T + row] = sum;
   }
   T* olo = p.out_lo ? static_cast<T*>(p.out_lo) + b * p.os[0] + h * p.os[1] : nullptr;
-  store_rows<T, DP>(ob, p.os[2], q0, p.T, p.D, o, inv, ty, tx, olo);
+  store_rows<T, DP>(ob, p.os[2], q0, p.T, p.D, o, inv, ln, olo);
 }
 
 // ------------------------------------------------------------------ backward, query-major: Delta and d_q
 template <typename T, int DP>
-__global__ void __launch_bounds__(NT) attn_bwd_dq_simt_kernel(AttnParams p, bool vec) {
+__global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_bwd_dq_simt_kernel(AttnParams p, bool vec) {
   extern __shared__ __align__(16) float smem[];
   constexpr int LD = DP + 4;
-  float* Qs = smem; float* dOs = Qs + BM * LD; float* Ks = dOs + BM * LD; float* Vs = Ks + BN * LD;
-  float* dSs = Vs + BN * LD; float* rowInv = dSs + BM * LDP; float* rowD = rowInv + BM;
-  const int b = blockIdx.z, h = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  float* Qs = smem; float* dOs = Qs + kOwn * LD; float* Ks = dOs + kOwn * LD; float* Vs = Ks + kStream * LD;
+  float* dSs = Vs + kStream * LD; float* rowInv = dSs + kOwn * kPairLd; float* rowD = rowInv + kOwn;
+  const Lane ln;
+  const Tile tl = this_tile(p);
+  const int b = tl.b, h = tl.h, n_tiles = (p.T + kOwn - 1) / kOwn;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = qt * BM;
+  const int q0 = (n_tiles - 1 - tl.tile) * kOwn;
   const T* qb = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const T* kb = static_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* vb = static_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
   const T* ob = static_cast<const T*>(p.out) + b * p.os[0] + h * p.os[1];
+  const T* olo = p.out_lo ? static_cast<const T*>(p.out_lo) + b * p.os[0] + h * p.os[1] : nullptr;
   const T* dob = static_cast<const T*>(p.d_out) + b * p.dos[0] + h * p.dos[1];
   T* dqb = static_cast<T*>(p.d_q) + b * p.dqs[0] + h * p.dqs[1];
   const int64_t stat0 = (int64_t(b) * p.H + h) * p.T;
   const float slope = p.slopes[h];
 
-  load_tile<T, DP>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
-  load_tile<T, DP>(dOs, dob, p.dos[2], q0, p.T, p.D, vec);
-  load_tile<T, DP>(Ks, ob, p.os[2], q0, p.T, p.D, vec);          // the O tile, parked in the K buffer
-  const bool has_lo = p.out_lo != nullptr;                        // and its rounding residual in the V buffer
-  if (has_lo) load_tile<T, DP>(Vs, static_cast<const T*>(p.out_lo) + b * p.os[0] + h * p.os[1], p.os[2], q0, p.T, p.D, vec);
-  __syncthreads();
-  for (int r = warp * 8; r < warp * 8 + 8; ++r) {
+  load_tile<T, DP, kOwn>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
+  load_tile<T, DP, kOwn>(dOs, dob, p.dos[2], q0, p.T, p.D, vec);
+  load_tile<T, DP, kStream>(Ks, kb, p.ks[2], 0, p.T, p.D, vec);
+  load_tile<T, DP, kStream>(Vs, vb, p.vs[2], 0, p.T, p.D, vec);
+#pragma unroll 2
+  for (int r = warp * 8; r < warp * 8 + 8; ++r) {                              // Delta = d_out . (out + its rounding residual)
+    const int row = q0 + r;
     float s = 0.f;
-    for (int d = lane; d < DP; d += 32) s = fmaf(dOs[r * LD + d], has_lo ? Ks[r * LD + d] + Vs[r * LD + d] : Ks[r * LD + d], s);
+    if (row < p.T) {
+#pragma unroll
+      for (int d = lane; d < DP; d += 32)
+        if (d < p.D) {
+          float o = Elem<T>::to_c(ob[int64_t(row) * p.os[2] + d]);
+          if (olo) o += Elem<T>::to_c(olo[int64_t(row) * p.os[2] + d]);
+          s = fmaf(Elem<T>::to_c(dob[int64_t(row) * p.dos[2] + d]), o, s);
+        }
+    }
     s = warp_sum(s);
     if (lane == 0) {
-      const int row = q0 + r;
       rowD[r] = s;
       rowInv[r] = row < p.T ? 1.f / (p.L[stat0 + row] + p.eps) : 0.f;
       if (row < p.T) p.delta[stat0 + row] = s;
     }
   }
-  __syncthreads();
 
-  float dq[4][DP / 16] = {};
-  const int n_kt = p.causal ? qt + 1 : (p.T + BN - 1) / BN;
-  for (int kt = 0; kt < n_kt; ++kt) {
-    const int k0 = kt * BN;
-    load_tile<T, DP>(Ks, kb, p.ks[2], k0, p.T, p.D, vec);
-    load_tile<T, DP>(Vs, vb, p.vs[2], k0, p.T, p.D, vec);
-    __syncthreads();
-    float s[4][4] = {}, dp[4][4] = {};
-    gemm_nt<DP>(s, Qs, Ks, ty, tx);
-    gemm_nt<DP>(dp, dOs, Vs, ty, tx);
+  Out<DP> dq;
+  clear(dq);
+  const int k_end = p.causal ? min(p.T, q0 + kOwn) : p.T;
+#pragma unroll 1
+  for (int k0 = 0; k0 < k_end; k0 += kStream) {
+    copies_visible();
+    float s[4][4], dp[4][4];
+    gemm_nt<DP>(s, Qs, Ks, ln);
+    gemm_nt<DP>(dp, dOs, Vs, ln);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rl = ty + 16 * i, row = q0 + rl;
-      const float dlt = rowD[rl], inv = rowInv[rl];
+    for (int j = 0; j < 4; ++j) {
+      const int col = k0 + ln.col(j);
+      const bool kept = col < p.T && key_kept(p, b, col);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = k0 + tx + 16 * j;
-        const bool live = col < p.T && row < p.T && (!p.causal || col <= row) && key_kept(p, b, col);
-        dSs[rl * LDP + tx + 16 * j] =
-            live ? score_terms(s[i][j], p.scale, slope, row, col).k * (dp[i][j] - dlt) * inv : 0.f;
+      for (int i = 0; i < 4; ++i) {
+        const int rl = ln.row(i), row = q0 + rl;
+        const bool live = kept && row < p.T && (!p.causal || col <= row);
+        put_pair(dSs, rl, ln.col(j), live ? score_terms(s[i][j], p.scale, slope, row, col).k * (dp[i][j] - rowD[rl]) * rowInv[rl] : 0.f);
       }
     }
-    __syncthreads();
-    gemm_nn<DP>(dq, dSs, Ks, ty, tx);
-    __syncthreads();
+    __syncthreads();                                                           // dS is there, V is free
+    const bool more = k0 + kStream < k_end;
+    if (more) load_tile<T, DP, kStream>(Vs, vb, p.vs[2], k0 + kStream, p.T, p.D, vec);
+    gemm_nn<DP>(dq, dSs, Ks, ln);
+    __syncthreads();                                                           // K and dS are free
+    if (more) load_tile<T, DP, kStream>(Ks, kb, p.ks[2], k0 + kStream, p.T, p.D, vec);
   }
+  copies_done();
   const float mul[4] = {p.scale, p.scale, p.scale, p.scale};
-  store_rows<T, DP>(dqb, p.dqs[2], q0, p.T, p.D, dq, mul, ty, tx);
+  store_rows<T, DP>(dqb, p.dqs[2], q0, p.T, p.D, dq, mul, ln);
 }
 
 // ------------------------------------------------------------------ backward, key-major: d_k and d_v
 template <typename T, int DP>
-__global__ void __launch_bounds__(NT) attn_bwd_dkv_simt_kernel(AttnParams p, bool vec) {
+__global__ void __launch_bounds__(NT, 2) attn_bwd_dkv_simt_kernel(AttnParams p, bool vec) {
   extern __shared__ __align__(16) float smem[];
   constexpr int LD = DP + 4;
-  float* Ks = smem; float* Vs = Ks + BN * LD; float* Qs = Vs + BN * LD; float* dOs = Qs + BM * LD;
-  float* PsT = dOs + BM * LD; float* dSsT = PsT + BN * LDP; float* rowInv = dSsT + BN * LDP; float* rowD = rowInv + BM;
-  const int b = blockIdx.z, h = blockIdx.y, kt = blockIdx.x;                    // early key tiles are the long ones
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const int k0 = kt * BN;
+  float* Ks = smem; float* Vs = Ks + kOwn * LD; float* Qs = Vs + kOwn * LD; float* dOs = Qs + kStream * LD;
+  float* PsT = dOs + kStream * LD; float* dSsT = PsT + kOwn * kPairLd;
+  const Lane ln;
+  const Tile tl = this_tile(p);                                                // early key tiles are the long ones
+  const int b = tl.b, h = tl.h, k0 = tl.tile * kOwn;
   const T* qb = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const T* kb = static_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* vb = static_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
@@ -289,45 +377,60 @@ __global__ void __launch_bounds__(NT) attn_bwd_dkv_simt_kernel(AttnParams p, boo
   const int64_t stat0 = (int64_t(b) * p.H + h) * p.T;
   const float slope = p.slopes[h];
 
-  load_tile<T, DP>(Ks, kb, p.ks[2], k0, p.T, p.D, vec);
-  load_tile<T, DP>(Vs, vb, p.vs[2], k0, p.T, p.D, vec);
-  float dk[4][DP / 16] = {}, dv[4][DP / 16] = {};
-  const int n_qt = (p.T + BM - 1) / BM;
-  for (int qt = p.causal ? kt : 0; qt < n_qt; ++qt) {
-    const int q0 = qt * BM;
-    load_tile<T, DP>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
-    load_tile<T, DP>(dOs, dob, p.dos[2], q0, p.T, p.D, vec);
-    if (threadIdx.x < BM) {
-      const int row = q0 + threadIdx.x;
-      rowInv[threadIdx.x] = row < p.T ? 1.f / (p.L[stat0 + row] + p.eps) : 0.f;
-      rowD[threadIdx.x] = row < p.T ? p.delta[stat0 + row] : 0.f;
+  int q0 = p.causal ? k0 / kStream * kStream : 0;
+  load_tile<T, DP, kOwn>(Ks, kb, p.ks[2], k0, p.T, p.D, vec);
+  load_tile<T, DP, kOwn>(Vs, vb, p.vs[2], k0, p.T, p.D, vec);
+  load_tile<T, DP, kStream>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
+  load_tile<T, DP, kStream>(dOs, dob, p.dos[2], q0, p.T, p.D, vec);
+  bool kept[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int col = k0 + ln.row(i);
+    kept[i] = col < p.T && key_kept(p, b, col);
+  }
+  Out<DP> dk, dv;
+  clear(dk);
+  clear(dv);
+#pragma unroll 1
+  for (; q0 < p.T; q0 += kStream) {
+    float L[4], dlt[4];                                                        // of this thread's four queries
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int row = q0 + ln.col(j);
+      L[j] = row < p.T ? p.L[stat0 + row] : 0.f;
+      dlt[j] = row < p.T ? p.delta[stat0 + row] : 0.f;
     }
-    __syncthreads();
-    float s[4][4] = {}, dp[4][4] = {};
-    gemm_nt<DP>(s, Qs, Ks, ty, tx);
-    gemm_nt<DP>(dp, dOs, Vs, ty, tx);
+    copies_visible();
+    float s[4][4], dp[4][4];
+    gemm_nt<DP>(s, Ks, Qs, ln);
+    gemm_nt<DP>(dp, Vs, dOs, ln);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rl = ty + 16 * i, row = q0 + rl;
-      const float dlt = rowD[rl], inv = rowInv[rl];
+    for (int j = 0; j < 4; ++j) {
+      const int row = q0 + ln.col(j);
+      const float inv = 1.f / (L[j] + p.eps);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int cl = tx + 16 * j, col = k0 + cl;
-        const bool live = col < p.T && row < p.T && (!p.causal || col <= row) && key_kept(p, b, col);
-        Score sc = score_terms(s[i][j], p.scale, slope, row, col);
-        PsT[cl * LDP + rl] = live ? sc.f * inv : 0.f;
-        dSsT[cl * LDP + rl] = live ? sc.k * (dp[i][j] - dlt) * inv : 0.f;
+      for (int i = 0; i < 4; ++i) {
+        const int cl = ln.row(i), col = k0 + cl;
+        const bool live = kept[i] && row < p.T && (!p.causal || col <= row);
+        const Score sc = score_terms(s[i][j], p.scale, slope, row, col);
+        put_pair(PsT, cl, ln.col(j), live ? sc.f * inv : 0.f);
+        put_pair(dSsT, cl, ln.col(j), live ? sc.k * (dp[i][j] - dlt[j]) * inv : 0.f);
       }
     }
     __syncthreads();
-    gemm_nn<DP>(dv, PsT, dOs, ty, tx);
-    gemm_nn<DP>(dk, dSsT, Qs, ty, tx);
-    __syncthreads();
+    gemm_nn<DP>(dv, PsT, dOs, ln);
+    __syncthreads();                                                           // dO is free
+    const bool more = q0 + kStream < p.T;
+    if (more) load_tile<T, DP, kStream>(dOs, dob, p.dos[2], q0 + kStream, p.T, p.D, vec);
+    gemm_nn<DP>(dk, dSsT, Qs, ln);
+    __syncthreads();                                                           // Q and the weights are free
+    if (more) load_tile<T, DP, kStream>(Qs, qb, p.qs[2], q0 + kStream, p.T, p.D, vec);
   }
+  copies_done();
   const float one[4] = {1.f, 1.f, 1.f, 1.f};
   const float mul[4] = {p.scale, p.scale, p.scale, p.scale};
-  store_rows<T, DP>(dvb, p.dvs[2], k0, p.T, p.D, dv, one, ty, tx);
-  store_rows<T, DP>(dkb, p.dks[2], k0, p.T, p.D, dk, mul, ty, tx);
+  store_rows<T, DP>(dvb, p.dvs[2], k0, p.T, p.D, dv, one, ln);
+  store_rows<T, DP>(dkb, p.dks[2], k0, p.T, p.D, dk, mul, ln);
 }
 
 template <typename T>
@@ -343,27 +446,29 @@ bool tiles_vectorisable(const AttnParams& p, bool bwd) {
 }
 
 template <typename Kern>
-int launch(Kern kern, const AttnParams& p, bool vec, int tiles, size_t smem, cudaStream_t st, const char* what) {
+int launch(Kern kern, const AttnParams& p, bool vec, size_t smem, cudaStream_t st, const char* what) {
   if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, what)) return rc;
-  dim3 grid(tiles, p.H, p.B);
+  const int64_t column = int64_t((p.T + kOwn - 1) / kOwn) * p.H;
+  const bool flat = column * p.B < (int64_t(1) << 31);                          // (otherwise the longest go first within a batch element)
+  const dim3 grid(unsigned(flat ? column * p.B : column), unsigned(flat ? 1 : p.B));
   kern<<<grid, NT, smem, st>>>(p, vec);
   return check_launch(what);
 }
 
 template <typename T, int DP>
 int fwd_t(const AttnParams& p, cudaStream_t st) {
-  constexpr size_t smem = (size_t(3) * BM * (DP + 4) + BM * LDP) * sizeof(float);
-  return launch(attn_fwd_simt_kernel<T, DP>, p, tiles_vectorisable<T>(p, false), (p.T + BM - 1) / BM, smem, st, "attn_fwd_simt");
+  constexpr size_t smem = (size_t(kOwn + 2 * kStream) * (DP + 4) + kOwn * kPairLd) * sizeof(float);
+  return launch(attn_fwd_simt_kernel<T, DP>, p, tiles_vectorisable<T>(p, false), smem, st, "attn_fwd_simt");
 }
 
 template <typename T, int DP>
 int bwd_t(const AttnParams& p, cudaStream_t st) {
   const bool vec = tiles_vectorisable<T>(p, true);
-  const int tiles = (p.T + BM - 1) / BM;
-  constexpr size_t smem_dq = (size_t(4) * BM * (DP + 4) + BM * LDP + 2 * BM) * sizeof(float);
-  constexpr size_t smem_dkv = (size_t(4) * BM * (DP + 4) + 2 * BM * LDP + 2 * BM) * sizeof(float);
-  if (int rc = launch(attn_bwd_dq_simt_kernel<T, DP>, p, vec, tiles, smem_dq, st, "attn_bwd_dq_simt")) return rc;
-  return launch(attn_bwd_dkv_simt_kernel<T, DP>, p, vec, tiles, smem_dkv, st, "attn_bwd_dkv_simt");
+  constexpr size_t tiles = size_t(2) * (kOwn + kStream) * (DP + 4);
+  constexpr size_t smem_dq = (tiles + kOwn * kPairLd + 2 * kOwn) * sizeof(float);
+  constexpr size_t smem_dkv = (tiles + 2 * kOwn * kPairLd) * sizeof(float);
+  if (int rc = launch(attn_bwd_dq_simt_kernel<T, DP>, p, vec, smem_dq, st, "attn_bwd_dq_simt")) return rc;
+  return launch(attn_bwd_dkv_simt_kernel<T, DP>, p, vec, smem_dkv, st, "attn_bwd_dkv_simt");
 }
 
 template <typename T>

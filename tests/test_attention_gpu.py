@@ -62,6 +62,20 @@ def test_fp32_vs_oracle(shape):
             assert norm_max_err(got, w) < FP32_TOL, f"{name}: {norm_max_err(got, w):.2e}"
 
 
+# own tiles of 32 rows, streamed tiles of 64: one row short of, at and beyond each edge; D = 30 and 34 take element-wise
+# copies (rows are no multiple of 16 bytes), 100 leaves columns of the tile empty
+@pytest.mark.parametrize("T", [31, 32, 33, 96, 97, 161])
+@pytest.mark.parametrize("D,causal", [(64, True), (128, False), (30, True), (34, False), (100, True)])
+def test_cuda_core_tile_edges(T, D, causal):
+    B, H = 2, 3
+    q, k, v, go = gen_qkv(27, B, H, T, D)
+    slopes = oracle.compute_alibi_slopes(H)
+    got = run_attention(q, k, v, go, slopes, 0.2, causal=causal, path=1)
+    want = oracle.rational_attention_grads(q, k, v, go, slopes, 0.2, causal=causal)
+    for g, w, name in zip(got, want, ("out", "dq", "dk", "dv")):
+        assert norm_max_err(g, w) < FP32_TOL, f"{name}: {norm_max_err(g, w):.2e}"
+
+
 def test_config1_fp32_closed_form_slopes():
     """Benchmark configuration 1: B=2,H=12,S=512,D=64 float32, slopes 2^(-8(i+1)/12)."""
     B, H, T, D = 2, 12, 512, 64
