@@ -10,6 +10,7 @@
 // kernels (one block per row, two passes, scalar accesses) that accept anything.
 #include <initializer_list>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -88,6 +89,14 @@ swiglu_fwd_kernel(const T* __restrict__ gate, const T* __restrict__ value, T* __
   }
 }
 
+template <typename C>
+__device__ __forceinline__ void swiglu_grads(C o, C a, C b, C& d_gate, C& d_value) {
+  const C r = rcp1p_abs(a);
+  const C s = rsigmoid(a, r);
+  d_value = o * a * s;                                  // d_out * gate * sigma
+  d_gate = o * b * (s + a * C(0.5) * r * r);            // d_out * value * (sigma + gate sigma')
+}
+
 template <typename T, int W>
 __global__ void __launch_bounds__(kThreads)
 swiglu_bwd_kernel(const T* __restrict__ d_out, const T* __restrict__ gate, const T* __restrict__ value,
@@ -106,16 +115,85 @@ swiglu_bwd_kernel(const T* __restrict__ d_out, const T* __restrict__ gate, const
       load_pack<T, W>(g + pk * W, a);
       load_pack<T, W>(v + pk * W, b);
 #pragma unroll
-      for (int i = 0; i < W; ++i) {
-        const C r = rcp1p_abs(a[i]);
-        const C s = rsigmoid(a[i], r);
-        rb[i] = o[i] * a[i] * s;                              // d_value = d_out * gate * sigma
-        ra[i] = o[i] * b[i] * (s + a[i] * C(0.5) * r * r);    // d_gate  = d_out * value * (sigma + gate sigma')
-      }
+      for (int i = 0; i < W; ++i) swiglu_grads(o[i], a[i], b[i], ra[i], rb[i]);
       store_pack<T, W>(dg + pk * W, ra);
       store_pack<T, W>(dv + pk * W, rb);
     }
   }
+}
+
+// Rows that do not start on 16-byte boundaries (the halves of a packed projection of odd or merely even width): packs of 8, 4
+// or 2 bytes, whatever all the addresses share.  G threads share a row and take up to U packs of it each, G packs apart, all
+// loads before the first use (one element of one row at a time left a thread two loads of 2 bytes in flight).  What bounds it
+// next is issuing instructions (84 % of the slots), so the packs stay as they come until they are used and their addresses are
+// one pointer per tensor plus constants: numbering the packs of all rows through, with a division per thread and a product
+// per access, took 40 and 64 us.  [8192, 2 x 2730] bfloat16, forward and backward: 76 and 99 -> 27 and 41 us (floor 21 and 34).
+template <typename T, int W>
+struct RaggedPack {
+  using Raw = std::conditional_t<W * sizeof(T) == 8, uint2, std::conditional_t<W * sizeof(T) == 4, uint32_t, uint16_t>>;
+  Raw raw;
+  __device__ __forceinline__ void load(const T* p) { raw = __ldcs(reinterpret_cast<const Raw*>(p)); }
+  __device__ __forceinline__ void store(T* p) const { __stcs(reinterpret_cast<Raw*>(p), raw); }
+  __device__ __forceinline__ typename Elem<T>::C get(int i) const { return Elem<T>::to_c(reinterpret_cast<const T*>(&raw)[i]); }
+  __device__ __forceinline__ void put(int i, typename Elem<T>::C v) { reinterpret_cast<T*>(&raw)[i] = Elem<T>::from_c(v); }
+};
+
+template <typename T, int W, int U>
+__global__ void __launch_bounds__(kThreads)
+swiglu_fwd_ragged_kernel(const T* __restrict__ gate, const T* __restrict__ value, T* __restrict__ out,
+                         int64_t n_rows, int64_t packs_per_row, int64_t gs, int64_t vs, int64_t os, int G) {
+  const int t = threadIdx.x & (G - 1), rows_per_block = kThreads / G;
+  for (int64_t row = int64_t(blockIdx.x) * rows_per_block + threadIdx.x / G; row < n_rows; row += int64_t(gridDim.x) * rows_per_block)
+    for (int64_t seg = int64_t(blockIdx.y) * U * G; seg < packs_per_row; seg += int64_t(gridDim.y) * U * G) {
+      const int left = int(packs_per_row - seg < U * G ? packs_per_row - seg : U * G) - t;       // packs from this thread's first on
+      const int64_t at = (seg + t) * W;
+      const T* g = gate + row * gs + at; const T* v = value + row * vs + at; T* o = out + row * os + at;
+      RaggedPack<T, W> a[U], b[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u * G < left) { a[u].load(g + u * G * W); b[u].load(v + u * G * W); }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u * G < left) {
+          RaggedPack<T, W> r;
+#pragma unroll
+          for (int i = 0; i < W; ++i) { const auto x = a[u].get(i); r.put(i, x * rsigmoid(x, rcp1p_abs(x)) * b[u].get(i)); }
+          r.store(o + u * G * W);
+        }
+    }
+}
+
+template <typename T, int W, int U>
+__global__ void __launch_bounds__(kThreads)
+swiglu_bwd_ragged_kernel(const T* __restrict__ d_out, const T* __restrict__ gate, const T* __restrict__ value,
+                         T* __restrict__ d_gate, T* __restrict__ d_value, int64_t n_rows, int64_t packs_per_row,
+                         int64_t dos, int64_t gs, int64_t vs, int64_t dgs, int64_t dvs, int G) {
+  const int t = threadIdx.x & (G - 1), rows_per_block = kThreads / G;
+  for (int64_t row = int64_t(blockIdx.x) * rows_per_block + threadIdx.x / G; row < n_rows; row += int64_t(gridDim.x) * rows_per_block)
+    for (int64_t seg = int64_t(blockIdx.y) * U * G; seg < packs_per_row; seg += int64_t(gridDim.y) * U * G) {
+      const int left = int(packs_per_row - seg < U * G ? packs_per_row - seg : U * G) - t;
+      const int64_t at = (seg + t) * W;
+      const T* go = d_out + row * dos + at; const T* g = gate + row * gs + at; const T* v = value + row * vs + at;
+      T* dg = d_gate + row * dgs + at; T* dv = d_value + row * dvs + at;
+      RaggedPack<T, W> o[U], a[U], b[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u * G < left) { o[u].load(go + u * G * W); a[u].load(g + u * G * W); b[u].load(v + u * G * W); }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u * G < left) {
+          RaggedPack<T, W> ra, rb;
+#pragma unroll
+          for (int i = 0; i < W; ++i) {
+            typename Elem<T>::C x, y;
+            swiglu_grads(o[u].get(i), a[u].get(i), b[u].get(i), x, y);
+            ra.put(i, x);
+            rb.put(i, y);
+          }
+          ra.store(dg + u * G * W);
+          rb.store(dv + u * G * W);
+        }
+    }
 }
 
 // =====================================================================================
@@ -713,21 +791,57 @@ RowPlan plan_rows(int64_t n_rows, int64_t n_cols, std::initializer_list<const vo
     default: { constexpr int VPT = 8; __VA_ARGS__; } break;       \
   }
 
+// Bytes that every address of the rows is a multiple of (at most 16): rows at `ptrs`, their strides, and the end of a row.
+inline int shared_alignment(std::initializer_list<const void*> ptrs, std::initializer_list<int64_t> row_strides, int64_t n_cols, int64_t n_rows, int elem_bytes) {
+  uint64_t bits = 16 | uint64_t(n_cols) * elem_bytes;
+  for (const void* p : ptrs) bits |= reinterpret_cast<uintptr_t>(p);
+  if (n_rows > 1)
+    for (int64_t s : row_strides) bits |= uint64_t(s) * elem_bytes;
+  return int(bits & (~bits + 1));
+}
+
+// launch(pack width W, packs per thread U, threads per row G, grid) for rows that share an alignment of less than 16 bytes.
+// G: enough threads for a row of up to U packs each; longer rows are cut into segments of U * 256 packs.
+template <typename T, typename Launch>
+void ragged_launch(int align, int64_t n_rows, int64_t n_cols, Launch&& launch) {
+  auto go = [&](auto w, auto u) {
+    const int64_t ppr = n_cols / w;
+    int G = 32;
+    while (G < kThreads && int64_t(G) * u < ppr) G <<= 1;
+    const int64_t blocks = (n_rows + kThreads / G - 1) / (kThreads / G), segs = (ppr + u * G - 1) / (u * G), cap = (int64_t(1) << 31) - 1;
+    launch(w, u, G, dim3(unsigned(blocks < cap ? blocks : cap), unsigned(segs < 65535 ? segs : 65535)));
+  };
+  if constexpr (sizeof(T) == 2) {
+    if (align >= 8) return go(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
+    if (align >= 4) return go(std::integral_constant<int, 2>{}, std::integral_constant<int, 6>{});
+    return go(std::integral_constant<int, 1>{}, std::integral_constant<int, 8>{});
+  } else if constexpr (sizeof(T) == 4) {
+    if (align >= 8) return go(std::integral_constant<int, 2>{}, std::integral_constant<int, 4>{});
+    return go(std::integral_constant<int, 1>{}, std::integral_constant<int, 6>{});
+  } else {
+    return go(std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{});
+  }
+}
+
 template <typename T>
 int swiglu_fwd_t(const void* gate, const void* value, void* out, int64_t n_rows, int64_t n_cols,
                  int64_t gs, int64_t vs, int64_t os, cudaStream_t st) {
   constexpr int W = 16 / sizeof(T);
   if (gs == n_cols && vs == n_cols && os == n_cols) { n_cols *= n_rows; n_rows = 1; gs = vs = os = n_cols; }
-  const bool vec = aligned16(gate) && aligned16(value) && aligned16(out) && n_cols % W == 0 &&
-                   gs % W == 0 && vs % W == 0 && os % W == 0;
-  const int64_t ppr = vec ? n_cols / W : n_cols;
-  int64_t gx = (ppr + kThreads - 1) / kThreads;
-  const int64_t cap = int64_t(FAT_SWIGLU_BPS) * num_sms();
-  if (gx > cap) gx = cap;
-  int64_t gy = n_rows < (cap + gx - 1) / gx ? n_rows : (cap + gx - 1) / gx;
-  dim3 grid((unsigned)gx, (unsigned)gy);
-  if (vec) swiglu_fwd_kernel<T, W><<<grid, kThreads, 0, st>>>((const T*)gate, (const T*)value, (T*)out, n_rows, ppr, gs, vs, os);
-  else     swiglu_fwd_kernel<T, 1><<<grid, kThreads, 0, st>>>((const T*)gate, (const T*)value, (T*)out, n_rows, ppr, gs, vs, os);
+  const int align = shared_alignment({gate, value, out}, {gs, vs, os}, n_cols, n_rows, sizeof(T));
+  if (align == 16) {
+    const int64_t ppr = n_cols / W;
+    int64_t gx = (ppr + kThreads - 1) / kThreads;
+    const int64_t cap = int64_t(FAT_SWIGLU_BPS) * num_sms();
+    if (gx > cap) gx = cap;
+    int64_t gy = n_rows < (cap + gx - 1) / gx ? n_rows : (cap + gx - 1) / gx;
+    dim3 grid((unsigned)gx, (unsigned)gy);
+    swiglu_fwd_kernel<T, W><<<grid, kThreads, 0, st>>>((const T*)gate, (const T*)value, (T*)out, n_rows, ppr, gs, vs, os);
+  } else {
+    ragged_launch<T>(align, n_rows, n_cols, [&](auto w, auto u, int G, dim3 grid) {
+      swiglu_fwd_ragged_kernel<T, w, u><<<grid, kThreads, 0, st>>>((const T*)gate, (const T*)value, (T*)out, n_rows, n_cols / w, gs, vs, os, G);
+    });
+  }
   return check_launch("swiglu_fwd");
 }
 
@@ -739,16 +853,21 @@ int swiglu_bwd_t(const void* d_out, const void* gate, const void* value, void* d
   if (dos == n_cols && gs == n_cols && vs == n_cols && dgs == n_cols && dvs == n_cols) {
     n_cols *= n_rows; n_rows = 1; dos = gs = vs = dgs = dvs = n_cols;
   }
-  const bool vec = aligned16(d_out) && aligned16(gate) && aligned16(value) && aligned16(d_gate) && aligned16(d_value) &&
-                   n_cols % W == 0 && dos % W == 0 && gs % W == 0 && vs % W == 0 && dgs % W == 0 && dvs % W == 0;
-  const int64_t ppr = vec ? n_cols / W : n_cols;
-  int64_t gx = (ppr + kThreads - 1) / kThreads;
-  const int64_t cap = int64_t(FAT_SWIGLU_BPS) * num_sms();
-  if (gx > cap) gx = cap;
-  int64_t gy = n_rows < (cap + gx - 1) / gx ? n_rows : (cap + gx - 1) / gx;
-  dim3 grid((unsigned)gx, (unsigned)gy);
-  if (vec) swiglu_bwd_kernel<T, W><<<grid, kThreads, 0, st>>>((const T*)d_out, (const T*)gate, (const T*)value, (T*)d_gate, (T*)d_value, n_rows, ppr, dos, gs, vs, dgs, dvs);
-  else     swiglu_bwd_kernel<T, 1><<<grid, kThreads, 0, st>>>((const T*)d_out, (const T*)gate, (const T*)value, (T*)d_gate, (T*)d_value, n_rows, ppr, dos, gs, vs, dgs, dvs);
+  const int align = shared_alignment({d_out, gate, value, d_gate, d_value}, {dos, gs, vs, dgs, dvs}, n_cols, n_rows, sizeof(T));
+  if (align == 16) {
+    const int64_t ppr = n_cols / W;
+    int64_t gx = (ppr + kThreads - 1) / kThreads;
+    const int64_t cap = int64_t(FAT_SWIGLU_BPS) * num_sms();
+    if (gx > cap) gx = cap;
+    int64_t gy = n_rows < (cap + gx - 1) / gx ? n_rows : (cap + gx - 1) / gx;
+    dim3 grid((unsigned)gx, (unsigned)gy);
+    swiglu_bwd_kernel<T, W><<<grid, kThreads, 0, st>>>((const T*)d_out, (const T*)gate, (const T*)value, (T*)d_gate, (T*)d_value, n_rows, ppr, dos, gs, vs, dgs, dvs);
+  } else {
+    ragged_launch<T>(align, n_rows, n_cols, [&](auto w, auto u, int G, dim3 grid) {
+      swiglu_bwd_ragged_kernel<T, w, u><<<grid, kThreads, 0, st>>>((const T*)d_out, (const T*)gate, (const T*)value, (T*)d_gate, (T*)d_value,
+                                                                   n_rows, n_cols / w, dos, gs, vs, dgs, dvs, G);
+    });
+  }
   return check_launch("swiglu_bwd");
 }
 

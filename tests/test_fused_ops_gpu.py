@@ -105,6 +105,24 @@ def test_swiglu_vs_oracle(shape, dtype):
     compare(dv, wdv, dtype, "swiglu dvalue")
 
 
+# halves of a packed tensor whose rows start on 8-, 4- and 2-byte boundaries (and 8- and 4-byte ones in float32); rows shorter
+# than a block's share of packs, one pack long, and longer than several shares
+@pytest.mark.parametrize("rows,n", [(1, 1), (3, 5), (301, 12), (7, 510), (5, 1365), (33, 2730), (2, 8188), (3, 4097)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32, torch.float64])
+def test_swiglu_of_ragged_rows(rows, n, dtype):
+    (x, go) = gen(47, (rows, 2 * n), (rows, n))
+    x, go = x.to(dtype), go.to(dtype)
+    xd = x.to(DEV).requires_grad_(True)
+    out = fat().rational_swiglu(*xd.chunk(2, dim=-1))
+    out.backward(go.to(DEV))
+    a, c = oracle_inputs([x, go], dtype)
+    a.requires_grad_(True)
+    want = oracle.rational_swiglu(*a.chunk(2, dim=-1))
+    want.backward(c)
+    compare(out.detach(), want.detach(), dtype, "out")
+    compare(xd.grad, a.grad, dtype, "d_x")
+
+
 def test_swiglu_reads_packed_halves_in_place():
     """gate / value as the two halves of one [rows, 2*ffn] projection (the model's layout)."""
     (gv, go) = gen(13, (4, 96, 2 * 344), (4, 96, 344))
