@@ -20,7 +20,14 @@
 // 65536 and more are clamped to 65504 and reported in bit 29 of the status word).  S = Q K^T uses
 // q and k as they are.
 //
+// A launch with about as many CTAs as SMs lasts as long as its longest CTA (16 key tiles for the last queries of 2000 tokens,
+// while the average is 9).  There the kernel runs in clusters of two CTAs, and the two share the keys of one of the longest
+// query blocks: the sums of the halves simply add, so each CTA sends the accumulator and row sums of one of its two query tiles
+// to the other one's shared memory (over the K stages, free by then) and finishes the other tile.  Shorter blocks stay whole,
+// one per CTA of a cluster.  How many blocks are shared is decided at launch_fwd.
+//
 // TMEM columns: S0/P0 [0,128)  S1/P1 [128,256)  O0 [256,256+D)  O1 [256+D,256+2D).
+#include <algorithm>
 #include <type_traits>
 
 #include "attn_tc_common.cuh"
@@ -163,16 +170,38 @@ __device__ __forceinline__ uint32_t convert_v(unsigned char* base, int lane) {
   return flag;
 }
 
-template <typename T, int D>
+// Every thread of both CTAs: what was written before is visible after, in either CTA's shared memory.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_addr(const void* own, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(own)), "r"(rank));
+  return r;
+}
+
+// PAIRS: clusters of two CTAs; the `n_shared` longest query blocks of every (batch, head) have a cluster each, the others a CTA.
+template <typename T, int D, bool PAIRS>
 __global__ void __launch_bounds__(kFwdThreads, 1)
-attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
+attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p, int n_shared) {
   extern __shared__ unsigned char smem_raw[];
   using S = FwdSmem<D>;
   S& sm = *reinterpret_cast<S*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5;
   const int n_qb = (p.T + 2 * BLK - 1) / (2 * BLK);
   int rank, bh;
-  if (!banded_tile(n_qb, p.B * p.H, kFwdBands, rank, bh)) return;      // padding block of the banded order
+  bool shared = false;                                       // the same in both CTAs of a cluster
+  const uint32_t half = PAIRS ? blockIdx.x % 2 : 0;          // of a shared block: which half of the keys; also the query tile to finish
+  if (PAIRS) {
+    const int n_bh = p.B * p.H, cluster = blockIdx.x / 2;
+    shared = cluster < n_shared * n_bh;
+    const int unit = shared ? cluster : 2 * (cluster - n_shared * n_bh) + int(half);
+    rank = unit / n_bh + (shared ? 0 : n_shared);
+    bh = unit % n_bh;
+    if (rank >= n_qb) return;                                // (the last whole block may lack a neighbour)
+  } else if (!banded_tile(n_qb, p.B * p.H, kFwdBands, rank, bh)) {
+    return;                                                  // padding block of the banded order
+  }
   const int b = bh / p.H, h = bh % p.H;
   const int qb = n_qb - 1 - rank;                            // long query blocks first
   const int n_kv_total = (p.T + BLK - 1) / BLK;
@@ -180,6 +209,17 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
   int n_tiles[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) n_tiles[t] = (2 * qb + t) * BLK < p.T ? (p.causal ? min(2 * qb + t + 1, n_kv_total) : n_kv_total) : 0;
+  int j0 = 0;                                                // first key tile of this CTA; n_tiles counts from it
+  bool mine[2] = {true, true};
+  if (PAIRS && shared) {
+    const int all = max(n_tiles[0], n_tiles[1]), mid = (all + 1) / 2;
+    j0 = half ? mid : 0;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      mine[t] = int(half) == t;
+      n_tiles[t] = max(0, min(n_tiles[t], half ? all : mid) - j0);
+    }
+  }
   const int n_max = max(n_tiles[0], n_tiles[1]);
   Guard g{&sm.abort_flag, p.status};
   constexpr bool kConvertV = !std::is_same<T, __half>::value;
@@ -210,14 +250,14 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
       for (int j = 0; j < n_max; ++j) {
         const int st = j % kStages, vst = j % kVStages;
         if (!g.wait(&sm.k_empty[st], ((j / kStages) & 1) ^ 1, 10)) break;
-        load_tile_tma<D>(sm.k[st], &maps.k, &sm.k_full[st], j * BLK, h, b);
+        load_tile_tma<D>(sm.k[st], &maps.k, &sm.k_full[st], (j0 + j) * BLK, h, b);
         if (!g.wait(&sm.v_empty[vst], ((j / kVStages) & 1) ^ 1, 11)) break;
 #ifdef FAT_TEST_WITHHOLD_V_TILE
         // test builds only (never the shipped library): this V tile is not loaded, so every wait that depends on it
         // runs out, which is how the give-up path (status word, teardown, TMEM release) gets exercised
         if (j == FAT_TEST_WITHHOLD_V_TILE) continue;
 #endif
-        load_tile_tma<D>(sm.v[vst], &maps.v, &sm.v_full[vst], j * BLK, h, b);
+        load_tile_tma<D>(sm.v[vst], &maps.v, &sm.v_full[vst], (j0 + j) * BLK, h, b);
       }
     }
   } else if (warp == kEwWarps + 1) {
@@ -284,7 +324,7 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
         const int st = j % kVStages;
         if (!g.wait(&sm.v_full[st], (j / kVStages) & 1, 40)) break;
         unsigned char* base = sm.v[st] + part * kPartBytes;
-        if (j / 2 == qb) out_of_range |= convert_v<kPartBytes, true>(base, lane);
+        if ((j0 + j) / 2 == qb) out_of_range |= convert_v<kPartBytes, true>(base, lane);
         else             convert_v<kPartBytes, false>(base, lane);
         fence_async_smem();
         mbar_arrive(&sm.v_ready[st]);
@@ -307,17 +347,18 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
     for (int j = 0; j < n; ++j) {
       if (!(ok = g.wait(&sm.s_full[t], j & 1, 30))) break;
       tc_fence_after();
-      const bool diag = (j == 2 * qb + t);
-      // bias of column c of this tile: -slope |row - (j BLK + c)|.  Keys up to the query: slope * c + slope (j BLK - row);
+      const int jt = j0 + j;                                 // the key tile
+      const bool diag = (jt == 2 * qb + t);
+      // bias of column c of this tile: -slope |row - (jt BLK + c)|.  Keys up to the query: slope * c + slope (jt BLK - row);
       // keys after it (non-causal only): the same with the sign flipped; the diagonal tile of a non-causal problem
       // takes the absolute value element by element.
-      const float sl = (!p.causal && j > 2 * qb + t) ? -slope : slope;
-      const float base = sl * float(j * BLK - row);
+      const float sl = (!p.causal && jt > 2 * qb + t) ? -slope : slope;
+      const float base = sl * float(jt * BLK - row);
       const f32x2 step2 = pk2(2.f * sl, 2.f * sl);
       const uint32_t trow = tmem_addr(tmem, lane_base, t * BLK + part * kColsPerWg);
       if (p.key_mask) {
         // (bits of keys beyond T are clear, so a ragged last tile needs no limit of its own)
-        const uint32_t* kw = p.key_mask + int64_t(b) * p.mask_words + j * (BLK / 32);
+        const uint32_t* kw = p.key_mask + int64_t(b) * p.mask_words + jt * (BLK / 32);
         if (p.causal && diag) softmax_tile<true, false, true>(trow, part * kChunks, r, scale2, four2, step2, sl, base, l2, kw);
         else if (diag)        softmax_tile<false, true, true>(trow, part * kChunks, 0, scale2, four2, step2, sl, base, l2, kw);
         else                  softmax_tile<false, false, true>(trow, part * kChunks, 0, scale2, four2, step2, sl, base, l2, kw);
@@ -326,7 +367,7 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
         else      softmax_tile<false, false>(trow, part * kChunks, r, scale2, four2, step2, sl, base, l2);
       } else {
         // zero-filled keys beyond T are not neutral (sigma(bias)^4 > 0): the last tile of a ragged sequence masks them
-        const int last_col = p.T - 1 - j * BLK;
+        const int last_col = p.T - 1 - jt * BLK;
         const bool tail = last_col < BLK - 1;
         if (diag && tail)  softmax_tile<true, true>(trow, part * kChunks, last_col, scale2, four2, step2, sl, base, l2);
         else if (diag)     softmax_tile<false, true>(trow, part * kChunks, 0, scale2, four2, step2, sl, base, l2);
@@ -351,7 +392,33 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
 #pragma unroll
       for (int i = 0; i < kSplit; ++i) l_sum += sm.l_part[t][i][r];
     }
-    if (n > 0 && !g.aborted()) {
+    float* parts = reinterpret_cast<float*>(sm.k);            // [D / 4][BLK][4]: the other half's accumulator
+    if (PAIRS && shared) {
+      cluster_sync();                                        // both CTAs' MMAs have run: their K stages are free
+      if (int(half) != t) {
+        const uint32_t to = peer_addr(parts, half ^ 1u) + uint32_t(r) * 16u;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t oreg[32];
+          if (n > 0) {
+            tmem_ld32(tmem_addr(tmem, lane_base, 2 * BLK + t * D + c * 32), oreg);
+            tmem_wait_ld();
+          } else {                                           // (no key of this half is visible to the tile, or the tile does not exist)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) oreg[i] = 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + uint32_t((c * 8 + i) * BLK * 16)),
+                         "r"(oreg[4 * i]), "r"(oreg[4 * i + 1]), "r"(oreg[4 * i + 2]), "r"(oreg[4 * i + 3]) : "memory");
+        }
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_addr(&sm.l_part[t][0][r], half ^ 1u)), "f"(l_sum) : "memory");
+      }
+      cluster_sync();
+      if (int(half) == t) l_sum += sm.l_part[t][0][r];
+    }
+    if (mine[t] && n > 0 && !g.aborted()) {
       // -------------------------------------------------------------- epilogue: O / (L + eps), hi + residual
       tc_fence_after();
       const float inv = (1.0f / kPUnit) / (l_sum + p.eps);     // the accumulator holds kPUnit sigma^4 V
@@ -365,6 +432,16 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
           uint32_t oreg[32];
           tmem_ld32(tmem_addr(tmem, lane_base, 2 * BLK + t * D + c * 32), oreg);
           tmem_wait_ld();
+          if (PAIRS && shared) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 o = *reinterpret_cast<const float4*>(parts + ((c * 8 + i) * BLK + r) * 4);
+              oreg[4 * i] = __float_as_uint(__uint_as_float(oreg[4 * i]) + o.x);
+              oreg[4 * i + 1] = __float_as_uint(__uint_as_float(oreg[4 * i + 1]) + o.y);
+              oreg[4 * i + 2] = __float_as_uint(__uint_as_float(oreg[4 * i + 2]) + o.z);
+              oreg[4 * i + 3] = __float_as_uint(__uint_as_float(oreg[4 * i + 3]) + o.w);
+            }
+          }
           uint32_t w[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -394,9 +471,65 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
       if (r == 0 && part == 0) tma_store_wait_all();
     }
   }
+  if (PAIRS && shared && warp >= kEwWarps) {                 // (the softmax warpgroups meet the other CTA above)
+    __syncwarp();
+    cluster_sync();
+    cluster_sync();
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == kEwWarps) tmem_dealloc(tmem, kTmemCols);
+}
+
+// How many of the longest query blocks per (batch, head) two CTAs should share (0: none, no clusters).  A CTA costs about
+// 5.5 us (6 with the exchange) and 2.05 us per key tile of its 256 queries; the first num_sms() CTAs start at once and the
+// rest, the shortest ones, behind the first to finish.  Sharing every block is not the best where that makes a second wave.
+// us for none / the rule's choice / all shared (bfloat16, causal): 16 x 2000 x 128: 43.5 / 35.0 / 37.0; 8 x 4096 x 128:
+// 76.9 / 51.7 / 51.9; 2 x 8192 x 128: 143.7 / 78.3 / 78.4; 24 x 1024 x 64: 22.6 / 16.6 / 20.7; 24 x 1500 x 128: 35.0 / 30.9 / 35.0;
+// 4 x 1024 x 128: 24.7 / 18.5 / 18.5; 48 x 777 x 64 (192 CTAs): 26.7 / none shared / 32.9.
+int shared_blocks(const AttnParams& p) {
+  const int n_qb = (p.T + 2 * BLK - 1) / (2 * BLK), n_kv = (p.T + BLK - 1) / BLK, sms = num_sms();
+  const int64_t n_bh = int64_t(p.B) * p.H;
+  if (n_qb * n_bh > 2 * sms || n_kv < 4) return 0;
+  auto whole = [&](int rank) { return 5.5 + 2.05 * (p.causal ? std::min(2 * (n_qb - rank), n_kv) : n_kv); };
+  auto halved = [&](int rank) { return 6.0 + 2.05 * (((p.causal ? std::min(2 * (n_qb - rank), n_kv) : n_kv) + 1) / 2); };
+  auto span = [&](int shared) {
+    double t = shared < n_qb ? whole(shared) : 0.0;
+    if (shared > 0) t = std::max(t, halved(0));
+    const int64_t ctas = (n_qb + shared) * n_bh;
+    if (ctas > 2 * sms) return 1e9;
+    if (ctas > sms) {                                        // the first CTA of the second wave follows the shortest one of the first
+      auto at = [&](int64_t i) { return i < 2 * shared * n_bh ? halved(int(i / (2 * n_bh))) : whole(int((i - shared * n_bh) / n_bh)); };
+      t = std::max(t, at(sms - 1) + at(sms));
+    }
+    return t;
+  };
+  int best = 0;
+  double best_t = 0.92 * span(0);                            // (clusters have to gain something)
+  for (int s = 1; s <= n_qb; ++s)
+    if (const double t = span(s); t < best_t) { best = s; best_t = t; }
+  return best;
+}
+
+template <typename T, int D, bool PAIRS>
+int launch_fwd_grid(const FwdMaps& maps, const AttnParams& p, int n_shared, cudaStream_t st) {
+  auto kern = attn_fwd_tc_kernel<T, D, PAIRS>;
+  const size_t smem = sizeof(FwdSmem<D>) + 1024;
+  if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, "attn_fwd_tc")) return rc;
+  const int n_qb = (p.T + 2 * BLK - 1) / (2 * BLK), n_bh = p.B * p.H;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = 2;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(PAIRS ? 2 * unsigned(n_shared * n_bh + ((n_qb - n_shared) * n_bh + 1) / 2) : banded_grid(n_qb, n_bh, kFwdBands));
+  cfg.blockDim = dim3(kFwdThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = PAIRS ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, maps, p, n_shared);
+  return check_launch("attn_fwd_tc");
 }
 
 template <typename T, int D>
@@ -412,12 +545,8 @@ int launch_fwd(const AttnParams& p, cudaStream_t st) {
   } else {
     maps.out_lo = maps.out;
   }
-  auto kern = attn_fwd_tc_kernel<T, D>;
-  const size_t smem = sizeof(FwdSmem<D>) + 1024;
-  if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, "attn_fwd_tc")) return rc;
-  const dim3 grid(banded_grid((p.T + 2 * BLK - 1) / (2 * BLK), p.B * p.H, kFwdBands));
-  kern<<<grid, kFwdThreads, smem, st>>>(maps, p);
-  return check_launch("attn_fwd_tc");
+  const int n_shared = shared_blocks(p);
+  return n_shared ? launch_fwd_grid<T, D, true>(maps, p, n_shared, st) : launch_fwd_grid<T, D, false>(maps, p, 0, st);
 }
 
 }  // namespace

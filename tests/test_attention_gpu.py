@@ -181,6 +181,27 @@ def test_low_precision_vs_oracle(shape, dtype, path):
     assert_16bit_bar(got, want)
 
 
+# few (batch, head) pairs of many tokens: two CTAs share the keys of a query block - of every block (1-4 pairs), of the longest
+# ones (16 pairs: some; 19: an odd number of whole blocks).  An even and an odd number of key tiles, a last query block of one
+# tile (1100, 1600) and of two (2000), a ragged last tile
+@pytest.mark.parametrize("shape", [(1, 2, 1024, 64), (1, 1, 1100, 128), (2, 2, 1600, 64), (1, 3, 2000, 128), (1, 16, 2000, 64), (1, 19, 1700, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("causal,masked", [(True, False), (False, False), (True, True)])
+def test_forward_with_shared_keys(shape, dtype, causal, masked):
+    B, H, T, D = shape
+    q, k, v, _ = gen_qkv(28, B, H, T, D, dtype)
+    slopes = oracle.compute_alibi_slopes(H)
+    keep = (torch.arange(T)[None] < torch.tensor([[T - 77 * (i + 1)] for i in range(B)])).to(torch.int64) if masked else None
+    f = fat()
+    with torch.no_grad():
+        out = f.rational_attention(q.to(DEV), k.to(DEV), v.to(DEV), slopes.to(DEV), 0.1, causal=causal,
+                                   key_mask=keep.to(DEV) if masked else None)
+    f.check_device_status()
+    want = oracle.rational_attention(q.float(), k.float(), v.float(), slopes, 0.1, causal=causal, key_mask=keep)
+    bad, nme = bf16_violations(out.float(), want)
+    assert bad == 0.0, f"{bad:.2e} of elements outside the bar (norm max err {nme:.2e})"
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("path", [0, 3])
 @pytest.mark.parametrize("gscale", [1e-6, 1e-2, 1e2, 1e4, 1e6])
