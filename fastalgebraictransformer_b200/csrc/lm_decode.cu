@@ -26,11 +26,12 @@
 // over 8 or 16 warps and summed in shared memory in a fixed order (results are reproducible).  tcgen05 has nothing to give
 // here: at 8-16 rows the tensor pipe idles either way, and registers can be filled before the wait.  The order of K inside
 // an MMA is free, so a lane takes 8 consecutive elements (one 16-byte load) of a weight row as its share of two MMAs.
-// Roundings: the first kRoundedLayers blocks round h, qkv, o, gate/value and pending to 16 bits where the operator-by-operator
-// path does; later blocks keep them in float32 (operands of the contractions, cached rows and logits are 16-bit everywhere).
-// Two 16-bit evaluations of twelve blocks drift apart because one differing rounding early moves every later one; with the
-// early roundings in common the logits stay 0.016 from the operator path's (0.019 if every block rounds, 0.021 if none does;
-// either path is 0.020 from exact arithmetic, this one 0.016).
+// Roundings: h, qkv, o, gate, value and pending are rounded to 16 bits where the operator-by-operator path rounds them (operands,
+// cached rows and logits are 16-bit anyway), in every block, so that a step may run either way.  The two differ in the order of
+// float32 sums; now and then that tips a rounding, which moves every later one: two such evaluations drift apart while both keep
+// their distance from the exact result.  bfloat16 logits of 16-32 steps, 2-norm, this kernel / operators against 64 bits, and
+// against each other: 2 blocks of width 768 0.0095 / 0.0095, 0.0062; 5 blocks 0.0142 / 0.0143, 0.0112; 12 blocks 0.0205 / 0.0205,
+// 0.0187; 8 blocks of 1024 0.0220 / 0.0224, 0.0180.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -43,7 +44,6 @@ constexpr int kLmThreads = 512, kLmWarps = kLmThreads / 32;
 constexpr int kPieces = 4;                      // 16-byte pieces per chunk; a thread's ring holds 4, 2 or 1 chunks, whatever shared memory leaves
 constexpr size_t kChunkBytes = size_t(kPieces) * kLmThreads * 16;
 constexpr size_t kLmSmemLimit = 220 * 1024;
-constexpr int kRoundedLayers = 2;
 constexpr int kPollLimit = 1 << 21;             // about a second
 
 struct LmLayerArgs {
@@ -144,13 +144,13 @@ struct Poller {
   }
 };
 
-template <typename T> __device__ __forceinline__ float as_stored(float v, bool rounded) { return rounded ? Elem<T>::to_c(Elem<T>::from_c(v)) : v; }
+template <typename T> __device__ __forceinline__ float as_stored(float v) { return Elem<T>::to_c(Elem<T>::from_c(v)); }
 
 // A[token][0..C) = norm(h) for all tokens, h = the tokens' embedding rows (add == nullptr) or h + add; every CTA keeps the residual
 // stream h [token][C] for itself in shared memory.  16 / (8 MR) warps per token; a thread owns the same columns every time.
 template <typename T, int MR>
 __device__ __forceinline__ void norm_into(unsigned char* A, int a_stride, float* h, float* sums, const LmArgs& p, const Poller& poll, const uint2* add,
-                                          unsigned tag, const void* weight, bool rounded) {
+                                          unsigned tag, const void* weight) {
   constexpr int WPT = 2 / MR, NT = 32 * WPT, NB = 6;
   const int warp = threadIdx.x >> 5, tok = warp / WPT, idx = threadIdx.x % NT, C2 = p.C / 2;
   float sum = 0.f;
@@ -177,8 +177,8 @@ __device__ __forceinline__ void norm_into(unsigned char* A, int a_stride, float*
           const int c = c0 + i * NT;
           if (c < C2) {
             float2 a = hr[c];
-            a.x = as_stored<T>(a.x + __uint_as_float(v[i].x), rounded);
-            a.y = as_stored<T>(a.y + __uint_as_float(v[i].z), rounded);
+            a.x = as_stored<T>(a.x + __uint_as_float(v[i].x));
+            a.y = as_stored<T>(a.y + __uint_as_float(v[i].z));
             sum += fabsf(a.x) + fabsf(a.y);
             hr[c] = a;
           }
@@ -545,7 +545,6 @@ lm_decode_kernel(const __grid_constant__ LmArgs p) {
   for (int step = 0; step <= 4 * p.L; ++step) {
     const int li = step >> 2, ph = step & 3;
     const LmLayerArgs& ly = p.layer[li < p.L ? li : 0];
-    const bool rounded = li < kRoundedLayers;
     const unsigned tag = launch + li * 8 + 1;    // qkv words; + 1 attention, + 2 o, + 3 act, + 4 pending
     const int64_t odd = li & 1;
     uint2 *att = p.att + odd * B * C / 2, *part = p.part + odd * items * (D + 2), *act = p.act + odd * B * p.act_words;
@@ -565,7 +564,7 @@ lm_decode_kernel(const __grid_constant__ LmArgs p) {
       }
     } else {
       const void* w = li == p.L ? p.norm : ph == 0 ? ly.norm1 : ly.norm2;
-      norm_into<T, MR>(A, as, h, sums, p, poll, add, ph == 0 ? tag - 4 : tag + 2, w, rounded);        // (tag - 4: the pending words of the layer before)
+      norm_into<T, MR>(A, as, h, sums, p, poll, add, ph == 0 ? tag - 4 : tag + 2, w);        // (tag - 4: the pending words of the layer before)
     }
     __syncthreads();
     // ---- this step's contraction
@@ -629,11 +628,11 @@ lm_decode_kernel(const __grid_constant__ LmArgs p) {
               if (n + 1 < p.V) out[1] = Elem<T>::from_c(v0.y);
             }
           } else {
-            v0.x = as_stored<T>(v0.x, rounded);
-            v0.y = as_stored<T>(v0.y, rounded);
+            v0.x = as_stored<T>(v0.x);
+            v0.y = as_stored<T>(v0.y);
             if (ph == 2) {
-              const float a0 = v0.x * rsigmoid(v0.x, rcp1p_abs(v0.x)) * as_stored<T>(v1.x, rounded);
-              const float a1 = v0.y * rsigmoid(v0.y, rcp1p_abs(v0.y)) * as_stored<T>(v1.y, rounded);
+              const float a0 = v0.x * rsigmoid(v0.x, rcp1p_abs(v0.x)) * as_stored<T>(v1.x);
+              const float a1 = v0.y * rsigmoid(v0.y, rcp1p_abs(v0.y)) * as_stored<T>(v1.y);
               st_word(act + int64_t(tok) * p.act_words + n / 2, Pair16<T>::put(a0, a1), tag + 3);
             } else {
               uint2* out = ph == 0 ? p.qkv + odd * B * 3 * C : ph == 1 ? p.o + odd * B * C : p.pend + odd * B * C;

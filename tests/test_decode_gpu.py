@@ -236,6 +236,70 @@ def test_fused_decode_step_equals_the_modules_and_the_oracle(dtype, d_model, n_h
             assert norm_max_err(b, a) < 4 * eps
 
 
+def _both_ways(model, ids, prompt):
+    """Logits of the steps after the prompt and the caches, operator by operator and as one launch."""
+    B, n = ids.shape
+    caches, logits = [model.new_cache(B, n) for _ in range(2)], []
+    for fused, cache in enumerate(caches):
+        model.forward_cached(ids[:, :prompt], cache)
+        if not fused:
+            cache.step = False
+        logits.append([model.forward_cached(ids[:, t:t + 1], cache) for t in range(prompt, n)])
+    assert caches[1].step and not caches[0].step
+    return caches, logits
+
+
+# more blocks than there are word buffers (two, used in turn).  The keys of a (batch, head) pair whole and shared out; heads of 128
+# for up to eight sequences; 16 sequences at width 1024, which leave room for one chunk in flight
+@pytest.mark.parametrize("dtype,d_model,n_head,n_layers,vocab,B,prompt", [
+    (torch.bfloat16, 768, 12, 5, 1000, 8, 150), (torch.bfloat16, 512, 8, 12, 509, 1, 300), (torch.float16, 768, 6, 3, 500, 4, 90),
+    (torch.bfloat16, 1024, 16, 3, 300, 16, 40), (torch.float16, 512, 4, 4, 200, 3, 33),
+])
+def test_fused_decode_step_of_many_blocks(dtype, d_model, n_head, n_layers, vocab, B, prompt):
+    """Two 16-bit evaluations drift apart with depth, so each is held against the 64-bit one: the fused step may be no further
+    off than the operators are, up to the scatter of such errors (2-norms over thousands of elements: 3-4 % here, 15 % allowed)."""
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM, check_device_status
+    torch.manual_seed(23)
+    model = AlgebraicTransformerLM(vocab_size=vocab, d_model=d_model, n_head=n_head, n_layers=n_layers, dropout=0.0, block_size=512)
+    ids = torch.randint(0, vocab, (B, prompt + 6))
+    state = {k: v.detach().to(dtype).double() for k, v in model.state_dict().items() if k != "embed.weight" and not k.endswith("alibi_slopes")}
+    exact, _ = oracle.lm_forward(state, ids, n_head)
+    model, ids = model.to(DEV).to(dtype).eval(), ids.to(DEV)
+    caches, logits = _both_ways(model, ids, prompt)
+    check_device_status()
+    exact = exact[:, prompt:]
+    off = [((torch.stack(x, 1).double().cpu() - exact).norm() / exact.norm()).item() for x in logits]
+    assert off[1] < 1.15 * off[0], f"{off[1]:.5f} from the exact logits, the operators {off[0]:.5f}"
+    assert off[0] < 3e-2
+    for side in ("k", "v"):
+        for a, b in zip(*(getattr(c, side) for c in caches)):
+            assert norm_max_err(b, a) < 3e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n_head", [1, 2])
+def test_fused_decode_step_rounds_where_the_operators_round(dtype, n_head):
+    """Weights with one power of two per row make every contraction exact, so the order of sums does not matter and both ways
+    have to agree to the bit, in every block: the residual stream, whose sums are rounded block by block, included."""
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM
+    torch.manual_seed(5)
+    C, n_layers = 128, 6
+    model = AlgebraicTransformerLM(vocab_size=96, d_model=C, n_head=n_head, n_layers=n_layers, d_ffn=192, dropout=0.0, block_size=64)
+    with torch.no_grad():
+        for block in model.blocks:
+            for w in (block.attn.qkv.weight, block.attn.out.weight, block.ffn.w_gate_val.weight, block.ffn.w_out.weight):
+                col = torch.randint(0, w.shape[1], (w.shape[0], 1))
+                w.zero_().scatter_(1, col, (2.0 ** torch.randint(-2, 2, col.shape)) * (1 - 2 * torch.randint(0, 2, col.shape)))
+        model.head.weight.copy_(torch.randint(1, 9, (96, C)) / 8.0 * (1 - 2 * torch.randint(0, 2, (96, C))))
+    model = model.to(DEV).to(dtype).eval()
+    caches, logits = _both_ways(model, torch.randint(0, 96, (3, 8), device=DEV), 1)
+    for side in ("k", "v"):
+        for i, (a, b) in enumerate(zip(*(getattr(c, side) for c in caches))):
+            assert torch.equal(a, b), f"{side} of block {i}"
+    for a, b in zip(*logits):                         # (the head's weights are dense: its sums may still round either way)
+        assert norm_max_err(b, a) < (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10)
+
+
 def test_fused_decode_step_yields_to_hooks_and_replaced_modules():
     from fastalgebraictransformer_b200 import AlgebraicTransformerLM
     torch.manual_seed(3)
