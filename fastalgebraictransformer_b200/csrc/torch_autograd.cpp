@@ -244,15 +244,16 @@ struct RationalAttentionBackward : Node {
 };
 
 struct RationalAttentionPackedBackward : Node {
-  SavedVariable qkv, out, L, lo, slopes, bits;          // out: [B,H,T,D]; the caller holds a [B,T,H*D] view of the same memory
+  SavedVariable qkv, out, L, lo, slopes, bits;          // out: the result [B,T,H*D] itself, so that a change in place is noticed
   double scale = 0, eps = 0;
   std::string name() const override { return "RationalAttentionPackedBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined()) return {Tensor()};
-    const Tensor pt = qkv.unpack(), ot = out.unpack(), Lt = L.unpack(), lt = lo.unpack(), st = slopes.unpack(), bt = bits.unpack();
+    const Tensor pt = qkv.unpack(), tokens = out.unpack(shared_from_this()), Lt = L.unpack(), lt = lo.unpack(), st = slopes.unpack(), bt = bits.unpack();
     BackwardScope scope;
-    const Tensor d = grads[0].reshape({pt.size(0), pt.size(1), pt.size(3), pt.size(4)}).permute({0, 2, 1, 3});
+    auto heads = [&](const Tensor& t) { return t.reshape({pt.size(0), pt.size(1), pt.size(3), pt.size(4)}).permute({0, 2, 1, 3}); };
+    const Tensor ot = heads(tokens), d = heads(grads[0]);
     return {op_attn_bwd_packed(pt, ot, lt, Lt, d, st, scale, eps, bt.defined() ? optional<Tensor>(bt) : optional<Tensor>())};
   }
   void release_variables() override {
@@ -395,7 +396,7 @@ Tensor attention_packed_autograd(const Tensor& qkv, const Tensor& slopes, double
   }
   if (node) {
     set_history(tokens, node);
-    node->out = SavedVariable(out, false);
+    node->out = SavedVariable(tokens, true);
     node->L = SavedVariable(L, false);
     node->lo = SavedVariable(lo, false);
     if (bits) node->bits = SavedVariable(*bits, false);

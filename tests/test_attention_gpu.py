@@ -261,6 +261,51 @@ def test_packed_projection_bf16_tensor_path(shape):
     assert_16bit_bar((got_out, gq, gk, gv), want)
 
 
+@pytest.mark.parametrize("shape,dtype", [((2, 4, 333, 64), torch.bfloat16), ((1, 3, 77, 128), torch.float16), ((2, 3, 65, 32), torch.float32),
+                                         ((2, 1, 40, 64), torch.bfloat16)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_packed_projection_through_the_operator(shape, dtype, masked):
+    """rational_attention_packed, the call the model makes: result and gradient of the packed tensor against the oracle."""
+    from fastalgebraictransformer_b200.backward import rational_attention_packed
+    B, H, T, D = shape
+    g = torch.Generator().manual_seed(44)
+    packed = torch.randn(B, T, 3, H, D, generator=g).to(dtype)
+    go = torch.randn(B, T, H * D, generator=g).to(dtype)
+    keep = (torch.arange(T)[None] < torch.tensor([[T - 9 * (i + 1)] for i in range(B)])).to(torch.int64) if masked else None
+    slopes = oracle.compute_alibi_slopes(H)
+    pd = packed.to(DEV).requires_grad_(True)
+    out = rational_attention_packed(pd, slopes.to(DEV), 0.125, key_mask=keep.to(DEV) if masked else None)
+    assert out.shape == (B, T, H * D) and out.is_contiguous()
+    out.backward(go.to(DEV))
+    fat().check_device_status()
+    q, k, v = packed.float().permute(2, 0, 3, 1, 4).unbind(0)
+    want = oracle.rational_attention_grads(q, k, v, go.float().view(B, T, H, D).permute(0, 2, 1, 3), slopes, 0.125, key_mask=keep)
+    got = (out.detach().view(B, T, H, D).permute(0, 2, 1, 3), *pd.grad.permute(2, 0, 3, 1, 4).unbind(0))
+    if dtype == torch.float32:
+        for x, w, name in zip(got, want, ("out", "dq", "dk", "dv")):
+            assert norm_max_err(x, w) < FP32_TOL, name
+    else:
+        assert_16bit_bar(got, want)
+
+
+@pytest.mark.parametrize("change", ["result", "view", "module"])
+def test_a_result_changed_in_place_is_not_differentiated(change):
+    """The backward reads the result: after a change in place it must refuse, not form a gradient from the new numbers."""
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM
+    from fastalgebraictransformer_b200.backward import rational_attention_packed
+    with pytest.raises(RuntimeError, match="in-?place"):
+        if change == "module":                       # heads scaled in place on their way into the output projection
+            model = AlgebraicTransformerLM(vocab_size=64, d_model=128, n_head=2, n_layers=1, dropout=0.0, block_size=32).to(DEV)
+            model.blocks[0].attn.out.register_forward_pre_hook(lambda m, args: (args[0].mul_(2.0),))
+            ids = torch.randint(0, 64, (2, 16), device=DEV)
+            model(ids, labels=ids)[1].backward()
+        else:
+            qkv = torch.randn(2, 16, 3, 2, 64, device=DEV, requires_grad=True)
+            out = rational_attention_packed(qkv, oracle.compute_alibi_slopes(2).to(DEV), 0.125)
+            (out if change == "result" else out.view(2, 16, 2, 64)[:, :, 1]).mul_(2.0)
+            out.sum().backward()
+
+
 def test_deterministic():
     """The CUDA-core path and the deterministic tensor path (no atomics anywhere): two runs give bit-identical outputs
     and gradients."""
