@@ -132,6 +132,9 @@ def build_ops(force: bool = False, verbose: bool = False) -> str:
     cmds = [[cxx, *flags, "-c", src, "-o", obj] for src, obj in zip(OPS_SRCS, objs) if force or _stale(obj, [src, header])]
     link = [cxx, "-shared", *objs, "-o", OPS_LIB] + ["-L" + p for p in ce.library_paths()]
     link += ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-L" + PKG, "-lfat_b200", "-Wl,-rpath,$ORIGIN"]
+    # the C++ library of the process, by name: a compiler that only has the static one would put a second copy into this module,
+    # whose stream facets are not the process's (writing a number into an error text crashed)
+    link.append("-l:libstdc++.so.6")
 
     def run(cmd):
         return subprocess.run(cmd, capture_output=True, text=True)
