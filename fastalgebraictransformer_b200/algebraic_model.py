@@ -191,6 +191,7 @@ class _DecodeStep:
         slopes = [b.attn.alibi_slopes for b in model.blocks]
         dtype, device = tops[2].dtype, tops[2].device
         if (any(w.dtype != dtype or w.device != device or not w.is_contiguous() for w in params + tops) or cache.k[0].dtype != dtype or
+                any(t.device != device for t in slopes + cache.k + cache.v + [cache.lengths]) or
                 any(s.dtype not in (dtype, torch.float32) or s.dtype != slopes[0].dtype for s in slopes) or len({n.eps for n in norms}) > 1 or
                 len({(b.attn.n_head, b.attn.scale, *b.ffn.w_out.weight.shape) for b in model.blocks}) > 1):
             return None
@@ -304,7 +305,8 @@ class AlgebraicTransformerLM(nn.Module):
         Same arithmetic as ``forward`` on the concatenated sequence: keys and values of earlier positions do not
         depend on later tokens (causal attention, relative bias), so they are kept instead of recomputed.  A step of one
         token per sequence runs as one launch where the fused step covers the model (``_DecodeStep``)."""
-        if cache.seen > 0 and input_ids.dim() == 2 and input_ids.size(1) == 1 and input_ids.dtype == torch.int64 and input_ids.is_cuda:
+        if (cache.seen > 0 and input_ids.dim() == 2 and input_ids.size(1) == 1 and input_ids.dtype == torch.int64 and
+                input_ids.is_cuda and input_ids.device == self.head.weight.device):
             if cache.seen >= cache.capacity:
                 raise RuntimeError(f"key/value cache is full ({cache.capacity} tokens)")
             if cache.step is None or (cache.step is not False and not cache.step.stands(self)):

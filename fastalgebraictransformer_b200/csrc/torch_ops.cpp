@@ -486,20 +486,22 @@ Tensor lm_decode_step(const Tensor& ids, const Tensor& embed, const Tensor& norm
   TORCH_CHECK(L >= 1 && L <= FAT_LM_MAX_LAYERS && int64_t(params.size()) == 6 * L && int64_t(slopes.size()) == L && int64_t(v.size()) == L, "one set of tensors per layer expected");
   const int64_t H = k[0].size(1), cap = k[0].size(2), D = k[0].size(3), F = params[5].size(1);
   const auto dtype = head.scalar_type();
+  auto here = [&](const Tensor& t) { return t.is_cuda() && t.device() == head.device(); };
   auto param = [&](const Tensor& t, at::IntArrayRef shape) {
-    TORCH_CHECK(t.is_cuda() && t.device() == head.device() && t.scalar_type() == dtype && t.is_contiguous() && t.sizes() == shape, "parameters must be dense CUDA tensors of the model's dtype and shapes");
+    TORCH_CHECK(here(t) && t.scalar_type() == dtype && t.is_contiguous() && t.sizes() == shape, "parameters must be dense tensors of the model's dtype, shapes and GPU");
     return t.data_ptr();
   };
-  TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.dim() == 2 && ids.size(1) == 1, "ids must be int64 [B, 1]");
-  TORCH_CHECK(lengths.is_cuda() && lengths.scalar_type() == at::kInt && lengths.is_contiguous() && lengths.numel() == B, "lengths must be int32 [B]");
+  TORCH_CHECK(here(ids) && ids.scalar_type() == at::kLong && ids.dim() == 2 && ids.size(1) == 1, "ids must be int64 [B, 1] on the model's GPU");
+  TORCH_CHECK(here(lengths) && lengths.scalar_type() == at::kInt && lengths.is_contiguous() && lengths.numel() == B, "lengths must be int32 [B] on the model's GPU");
+  TORCH_CHECK(here(workspace) && workspace.scalar_type() == at::kByte && workspace.is_contiguous(), "the workspace must be dense bytes on the model's GPU");
   const int slopes_f32 = slopes[0].scalar_type() == at::kFloat;
   const auto cs = strides3(k[0]);
   std::array<fat_lm_layer, FAT_LM_MAX_LAYERS> layers;
   for (int64_t i = 0; i < L; ++i) {
     const Tensor* w = &params[6 * i];
-    TORCH_CHECK(slopes[i].is_cuda() && slopes[i].is_contiguous() && slopes[i].numel() == H && slopes[i].scalar_type() == (slopes_f32 ? at::kFloat : dtype), "one dense slope per head expected");
+    TORCH_CHECK(here(slopes[i]) && slopes[i].is_contiguous() && slopes[i].numel() == H && slopes[i].scalar_type() == (slopes_f32 ? at::kFloat : dtype), "one dense slope per head on the model's GPU expected");
     for (const Tensor* c : {&k[i], &v[i]})
-      TORCH_CHECK(c->is_cuda() && c->scalar_type() == dtype && c->stride(3) == 1 && c->sizes() == k[0].sizes() && c->strides() == k[0].strides(), "the layers' caches must be alike");
+      TORCH_CHECK(here(*c) && c->scalar_type() == dtype && c->stride(3) == 1 && c->sizes() == k[0].sizes() && c->strides() == k[0].strides(), "the layers' caches must be alike and on the model's GPU");
     layers[i] = {param(w[0], {C}), param(w[1], {3 * C, C}), param(w[2], {C, C}), param(w[3], {C}), param(w[4], {2 * F, C}), param(w[5], {C, F}),
                  k[i].data_ptr(), v[i].data_ptr(), slopes[i].data_ptr()};
   }

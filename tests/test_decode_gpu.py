@@ -300,6 +300,40 @@ def test_fused_decode_step_rounds_where_the_operators_round(dtype, n_head):
         assert norm_max_err(b, a) < (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10)
 
 
+def _half_model(n_layers=2, d_model=128, n_head=2, vocab=64, **kw):
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM
+    torch.manual_seed(3)
+    kw = {"dropout": 0.0, "block_size": 64, **kw}
+    return AlgebraicTransformerLM(vocab_size=vocab, d_model=d_model, n_head=n_head, n_layers=n_layers, **kw).to(DEV).to(torch.bfloat16).eval()
+
+
+@pytest.mark.parametrize("what", ["ids", "lengths", "workspace", "slopes", "k", "v", "workspace dtype", "lengths dtype"])
+def test_decode_step_operator_refuses_tensors_from_elsewhere(what):
+    """Every tensor of the step has to be on the model's GPU (here: one on the host); refused before anything is launched."""
+    model = _half_model()
+    cache = model.new_cache(2, 12)
+    ids = torch.randint(0, 64, (2, 5), device=DEV)
+    model.forward_cached(ids[:, :4], cache)
+    model.forward_cached(ids[:, 4:], cache)
+    blocks = model.blocks
+    args = dict(ids=ids[:, :1], embed=model.embed.weight, norm=model.norm.weight, head=model.head.weight,
+                params=[w for b in blocks for w in (b.norm1.weight, b.attn.qkv.weight, b.attn.out.weight, b.norm2.weight, b.ffn.w_gate_val.weight, b.ffn.w_out.weight)],
+                slopes=[b.attn.alibi_slopes for b in blocks], k=list(cache.k), v=list(cache.v), lengths=cache.lengths.clone(),
+                workspace=torch.zeros(1 << 20, dtype=torch.uint8, device=DEV))
+    step = lambda: torch.ops.algebraic.lm_decode_step(*args.values(), 0.125, 1e-6, 1e-6)          # noqa: E731
+    assert step().shape == (2, 64)
+    torch.cuda.synchronize()
+    if what.endswith("dtype"):
+        name = what.split()[0]
+        args[name] = args[name].to(torch.int64)
+    elif isinstance(args[what], list):
+        args[what][1] = args[what][1].cpu()
+    else:
+        args[what] = args[what].cpu()
+    with pytest.raises(RuntimeError, match="model's GPU"):
+        step()
+
+
 def test_fused_decode_step_yields_to_hooks_and_replaced_modules():
     from fastalgebraictransformer_b200 import AlgebraicTransformerLM
     torch.manual_seed(3)
