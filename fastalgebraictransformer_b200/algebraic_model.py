@@ -157,8 +157,8 @@ class AlgebraicBlock(nn.Module):
 
 class _DecodeStep:
     """What ``lm_decode_step`` (one launch for a whole decode step) needs of a model and a cache, gathered once per cache,
-    and the conditions under which it stands for the modules' own forward passes: stock modules without hooks, nothing
-    that drops out.  ``None`` from ``make`` means the step runs module by module."""
+    and the conditions under which it stands for the modules' own forward passes: stock modules without hooks or methods
+    of their own, nothing that drops out, the constants they had.  ``None`` from ``make`` means the step runs module by module."""
 
     def __init__(self, parameters, rest, watch, hooks, model):
         self.parameters, self.rest, self.watch, self.hooks, self.model = parameters, rest, watch, hooks, model
@@ -168,20 +168,25 @@ class _DecodeStep:
     def make(model, cache):
         stock = {AlgebraicBlock: ("attn", "ffn", "norm1", "norm2"), AlgebraicAttention: ("qkv", "out", "dropout"),
                  RationalSwiGLU: ("w_gate_val", "w_out", "dropout"), RationalMR: (), nn.Linear: (), nn.Dropout: ()}
-        watch, hooks, modules = [], [], [model.norm, model.head, *model.blocks]
+        constants = {AlgebraicAttention: ("scale", "n_head", "d_head"), RationalMR: ("eps",), nn.Dropout: ("training", "p")}
+        watch, hooks, modules, own = [(globals(), "EPS")], [], [model.norm, model.head, *model.blocks], [(model.embed.__dict__, "forward")]
         for m in modules:                                # (grows while it is walked)
             if type(m) not in stock or (type(m) is nn.Linear and m.bias is not None):
                 return None
             modules += [getattr(m, n) for n in stock[type(m)]]
-            watch += [(m._modules, n) for n in stock[type(m)]] + [(m._parameters, n) for n in m._parameters] + [(m.__dict__, "forward")]
-            watch += [(m._buffers, n) for n in m._buffers] + ([(m.__dict__, "training"), (m.__dict__, "p")] if type(m) is nn.Dropout else [])
+            watch += [(m._modules, n) for n in stock[type(m)]] + [(m._parameters, n) for n in m._parameters]
+            watch += [(m._buffers, n) for n in m._buffers] + [(m.__dict__, n) for n in constants.get(type(m), ())]
+            own += [(m.__dict__, "forward"), (m.__dict__, "forward_deferred")]
             hooks += [m._forward_hooks, m._forward_pre_hooks]
             if type(m) is nn.Dropout and m.training and m.p > 0:
                 return None
-        if type(model.embed) is not nn.Embedding or model.embed.max_norm is not None:
+        if type(model.embed) is not nn.Embedding or model.embed.max_norm is not None or any(n in d for d, n in own):
             return None
+        if any(getattr(c, n) is not f for c, n, f in _STOCK_METHODS):
+            return None
+        watch += own + [(vars(c), n) for c, n, _ in _STOCK_METHODS]
         watch += [(model._modules, n) for n in ("embed", "norm", "head", "blocks")] + [(model.blocks._modules, n) for n in model.blocks._modules]
-        watch += [(model.embed._parameters, "weight"), (model.embed.__dict__, "forward")]
+        watch += [(model.embed._parameters, "weight"), (model.embed.__dict__, "max_norm")]
         hooks += [model.embed._forward_hooks, model.embed._forward_pre_hooks, torch.nn.modules.module._global_forward_hooks,
                   torch.nn.modules.module._global_forward_pre_hooks]
         first, norms = model.blocks[0], [model.norm] + [n for b in model.blocks for n in (b.norm1, b.norm2)]
@@ -193,7 +198,8 @@ class _DecodeStep:
         if (any(w.dtype != dtype or w.device != device or not w.is_contiguous() for w in params + tops) or cache.k[0].dtype != dtype or
                 any(t.device != device for t in slopes + cache.k + cache.v + [cache.lengths]) or
                 any(s.dtype not in (dtype, torch.float32) or s.dtype != slopes[0].dtype for s in slopes) or len({n.eps for n in norms}) > 1 or
-                len({(b.attn.n_head, b.attn.scale, *b.ffn.w_out.weight.shape) for b in model.blocks}) > 1):
+                len({(b.attn.n_head, b.attn.scale, *b.ffn.w_out.weight.shape) for b in model.blocks}) > 1 or
+                (first.attn.n_head, first.attn.d_head) != (cache.k[0].shape[1], cache.k[0].shape[3])):
             return None
         B, H, capacity, D = cache.k[0].shape
         nbytes = torch.ops.algebraic.lm_decode_workspace_bytes(B, tops[2].shape[1], H, D, first.ffn.w_out.weight.shape[1], tops[2].shape[0],
@@ -216,6 +222,11 @@ class _DecodeStep:
 
     def __call__(self, input_ids, cache):
         return torch.ops.algebraic.lm_decode_step(input_ids, *self.parameters, cache.k, cache.v, cache.lengths, *self.rest)
+
+
+# what the fused step stands for; a class that has been given another method since is run as it is
+_STOCK_METHODS = [(c, n, getattr(c, n)) for c, n in ((AlgebraicBlock, "forward_deferred"), (AlgebraicAttention, "forward"), (RationalSwiGLU, "forward"),
+                                                    (RationalMR, "forward"), (nn.Linear, "forward"), (nn.Dropout, "forward"), (nn.Embedding, "forward"))]
 
 
 class AlgebraicTransformerLM(nn.Module):

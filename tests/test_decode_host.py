@@ -52,3 +52,93 @@ def test_a_cache_or_slopes_of_another_gpu_make_no_fused_step(what):
         else:
             getattr(cache, what)[1] = getattr(cache, what)[1].to("cuda:1")
         assert _DecodeStep.make(model, cache) is None
+
+
+def _scale(model):
+    model.blocks[1].attn.scale = 0.5
+
+
+def _heads(model):
+    model.blocks[0].attn.n_head = 4
+
+
+def _eps_of_a_block(model):
+    model.blocks[0].norm2.eps = 1e-3
+
+
+def _eps_of_the_last_norm(model):
+    model.norm.eps = 1e-3
+
+
+def _forward_of_an_instance(model):
+    attn = model.blocks[1].attn
+    attn.forward = lambda *a, **k: type(attn).forward(attn, *a, **k)
+
+
+def _deferred_forward_of_a_block(model):
+    block = model.blocks[0]
+    block.forward_deferred = lambda *a, **k: type(block).forward_deferred(block, *a, **k)
+
+
+def _forward_of_the_embedding(model):
+    embed = model.embed
+    embed.forward = lambda x: type(embed).forward(embed, x)
+
+
+def _clipped_embedding(model):
+    model.embed.max_norm = 1.0
+
+
+CHANGES = [_scale, _heads, _eps_of_a_block, _eps_of_the_last_norm, _forward_of_an_instance, _deferred_forward_of_a_block,
+           _forward_of_the_embedding, _clipped_embedding]
+
+
+@pytest.mark.parametrize("change", CHANGES)
+def test_a_changed_constant_or_method_ends_the_fused_step(change):
+    """What the step was made of no longer holds: it must not stand, however the change came about."""
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    with FakeTensorMode():
+        model, cache = model_and_cache()
+        step = _DecodeStep.make(model, cache)
+        assert step.stands(model)
+        change(model)
+        assert not step.stands(model)
+
+
+@pytest.mark.parametrize("change", CHANGES)
+def test_a_step_is_not_made_of_a_model_that_differs(change):
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    with FakeTensorMode():
+        model, cache = model_and_cache()
+        change(model)
+        assert _DecodeStep.make(model, cache) is None           # (scale and eps: one value for all blocks and norms)
+
+
+def test_a_method_replaced_on_the_class_ends_the_fused_step(monkeypatch):
+    from fastalgebraictransformer_b200 import algebraic_model
+    with FakeTensorMode():
+        model, cache = model_and_cache()
+        step = algebraic_model._DecodeStep.make(model, cache)
+        stock = algebraic_model.AlgebraicAttention.forward
+        monkeypatch.setattr(algebraic_model.AlgebraicAttention, "forward", lambda self, *a, **k: stock(self, *a, **k))
+        assert not step.stands(model) and algebraic_model._DecodeStep.make(model, cache) is None
+
+
+def test_heads_that_are_not_the_caches_make_no_fused_step():
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    with FakeTensorMode():
+        model, cache = model_and_cache()
+        for block in model.blocks:
+            block.attn.n_head, block.attn.d_head = 1, 128
+        assert _DecodeStep.make(model, cache) is None
+
+
+def test_constants_changed_everywhere_are_taken_over():
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    with FakeTensorMode():
+        model, cache = model_and_cache()
+        for block in model.blocks:
+            block.attn.scale = 0.5
+        for norm in [model.norm] + [n for b in model.blocks for n in (b.norm1, b.norm2)]:
+            norm.eps = 1e-3
+        assert _DecodeStep.make(model, cache).rest[1:3] == (0.5, 1e-3)
