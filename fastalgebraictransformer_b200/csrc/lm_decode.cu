@@ -94,17 +94,19 @@ __device__ __forceinline__ void copy_async(uint32_t dst, const void* src, bool i
 }
 
 // ------------------------------------------------------------------------------------------------- tagged words
-// Two neighbouring words: (value, tag, value, tag).
+// A word is one 64-bit element of every access, so that its value and its tag are seen together (a vector access promises that
+// for each of its elements, not for the whole).  Two neighbouring words: (value, tag, value, tag).
 __device__ __forceinline__ uint4 ld_words(const uint2* p) {
-  uint4 v;
-  asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
+  uint64_t a, b;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  return make_uint4(uint32_t(a), uint32_t(a >> 32), uint32_t(b), uint32_t(b >> 32));
 }
+__device__ __forceinline__ uint64_t word_of(uint32_t value, unsigned tag) { return uint64_t(tag) << 32 | value; }
 __device__ __forceinline__ void st_words(uint2* p, uint32_t a, uint32_t b, unsigned tag) {
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(a), "r"(tag), "r"(b), "r"(tag) : "memory");
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(word_of(a, tag)), "l"(word_of(b, tag)) : "memory");
 }
 __device__ __forceinline__ void st_word(uint2* p, uint32_t a, unsigned tag) {
-  asm volatile("st.volatile.global.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(a), "r"(tag) : "memory");
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(word_of(a, tag)) : "memory");
 }
 
 struct Poller {
