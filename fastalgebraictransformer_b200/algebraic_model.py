@@ -196,6 +196,7 @@ class _DecodeStep:
         slopes = [b.attn.alibi_slopes for b in model.blocks]
         dtype, device = tops[2].dtype, tops[2].device
         if (any(w.dtype != dtype or w.device != device or not w.is_contiguous() for w in params + tops) or cache.k[0].dtype != dtype or
+                tops[0].shape != tops[2].shape or
                 any(t.device != device for t in slopes + cache.k + cache.v + [cache.lengths]) or
                 any(s.dtype not in (dtype, torch.float32) or s.dtype != slopes[0].dtype for s in slopes) or len({n.eps for n in norms}) > 1 or
                 len({(b.attn.n_head, b.attn.scale, *b.ffn.w_out.weight.shape) for b in model.blocks}) > 1 or
@@ -323,9 +324,13 @@ class AlgebraicTransformerLM(nn.Module):
             if cache.step is None or (cache.step is not False and not cache.step.stands(self)):
                 cache.step = _DecodeStep.make(self, cache) or False
             if cache.step and input_ids.size(0) == cache.lengths.numel():
-                logits = cache.step(input_ids, cache)
-                cache.seen += 1                          # (the launch has advanced the device-side lengths)
-                return logits
+                try:
+                    logits = cache.step(input_ids, cache)
+                except RuntimeError:                     # refused before anything ran: rows off 16-byte boundaries, caches that
+                    cache.step = False                   # are not alike, a launch that fails
+                else:
+                    cache.seen += 1                      # (the launch has advanced the device-side lengths)
+                    return logits
         x = self.embed(input_ids)
         pending = None
         for i, block in enumerate(self.blocks):

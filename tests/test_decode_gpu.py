@@ -334,6 +334,51 @@ def test_decode_step_operator_refuses_tensors_from_elsewhere(what):
         step()
 
 
+def _unaligned(t):
+    """The same values in memory that starts two bytes after a 16-byte boundary."""
+    return torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)[1:t.numel() + 1].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("late", [False, True])
+@pytest.mark.parametrize("what", ["embedding rows", "embedding rows fewer", "parameter", "head", "slopes dtype", "cache layout", "cache alignment"])
+def test_what_the_fused_step_does_not_take_runs_module_by_module(what, late):
+    """Models and caches that the operators take and the single launch does not: same result as without it, whether they
+    differ from the start or (late) come to differ after the first fused step."""
+    results = []
+    for fused in (False, True):
+        model = _half_model(vocab=64)
+        cache = model.new_cache(2, 16)
+        ids = torch.randint(0, 60, (2, 9), generator=torch.Generator().manual_seed(4)).to(DEV)
+        model.forward_cached(ids[:, :4], cache)
+        if late:
+            if fused:
+                model.forward_cached(ids[:, 4:5], cache)
+                assert cache.step
+            else:                                    # (the same rows in the cache as the fused step leaves)
+                model.forward_cached(ids[:, 4:5], cache)
+        cache.step = None if fused else False
+        with torch.no_grad():
+            if what.startswith("embedding"):
+                rows = 60 if what.endswith("fewer") else 80
+                model.embed = torch.nn.Embedding(rows, 128).to(DEV).to(torch.bfloat16)
+                model.embed.weight.copy_(torch.randn(rows, 128, generator=torch.Generator().manual_seed(6)))
+            elif what == "parameter":
+                w = model.blocks[1].ffn.w_out.weight
+                w.data = _unaligned(w)
+            elif what == "head":
+                model.head.weight.data = _unaligned(model.head.weight)
+            elif what == "slopes dtype":
+                model.blocks[1].attn.alibi_slopes = model.blocks[1].attn.alibi_slopes.double()
+            elif what == "cache layout":
+                cache.k[1] = cache.k[1].permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3)
+            else:                                    # rows of 8 extra elements: aligned, but not alike
+                cache.v[0] = torch.cat((cache.v[0], cache.v[0][..., :8]), -1)[..., :64]
+        results.append([model.forward_cached(ids[:, t:t + 1], cache) for t in range(5 if late else 4, 9)] + [cache.lengths, *cache.k, *cache.v])
+        assert not cache.step
+    for got, want in zip(*results):
+        assert torch.equal(got[..., :9, :] if got.dim() == 4 else got, want[..., :9, :] if want.dim() == 4 else want)
+
+
 def test_fused_decode_step_yields_to_hooks_and_replaced_modules():
     from fastalgebraictransformer_b200 import AlgebraicTransformerLM
     torch.manual_seed(3)
