@@ -543,8 +543,8 @@ TORCH_LIBRARY(algebraic, m) {
         "float scale, float eps) -> Tensor");
   m.def("lm_decode_workspace_bytes(int B, int C, int H, int D, int F, int V, int n_layers, int capacity, ScalarType dtype) -> int",
         &lm_decode_workspace_bytes);
-  m.def("lm_decode_step(Tensor ids, Tensor embed, Tensor norm, Tensor head, Tensor[] params, Tensor[] slopes, Tensor[] k, Tensor[] v, "
-        "Tensor(a!) lengths, Tensor(b!) workspace, float scale, float eps_norm, float eps_attn) -> Tensor");
+  m.def("lm_decode_step(Tensor ids, Tensor embed, Tensor norm, Tensor head, Tensor[] params, Tensor[] slopes, Tensor(a!)[] k, "
+        "Tensor(b!)[] v, Tensor(c!) lengths, Tensor(d!) workspace, float scale, float eps_norm, float eps_attn) -> Tensor");
   m.def("device_status(int device) -> Tensor", &device_status);
 }
 

@@ -246,6 +246,11 @@ def _(q, k_new, v_new, k_cache, v_cache, n_cached, slopes, scale, eps):
     return q.new_empty(q.shape)
 
 
+@torch.library.register_fake(f"{_NS}::lm_decode_step")
+def _(ids, embed, norm, head, params, slopes, k, v, lengths, workspace, scale, eps_norm, eps_attn):
+    return head.new_empty((ids.shape[0], head.shape[0]))
+
+
 # ----------------------------------------------------------------------------- autograd formulas
 def _swiglu_setup(ctx, inputs, output):
     ctx.save_for_backward(*inputs)

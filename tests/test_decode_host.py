@@ -142,3 +142,15 @@ def test_constants_changed_everywhere_are_taken_over():
         for norm in [model.norm] + [n for b in model.blocks for n in (b.norm1, b.norm2)]:
             norm.eps = 1e-3
         assert _DecodeStep.make(model, cache).rest[1:3] == (0.5, 1e-3)
+
+
+def test_decode_step_operator_declares_what_it_writes_and_its_shape():
+    """The caches' rows, the lengths and the workspace; the result is [B, V] of the head's dtype."""
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    schema = torch.ops.algebraic.lm_decode_step.default._schema
+    written = {a.name for a in schema.arguments if a.alias_info is not None and a.alias_info.is_write}
+    assert written == {"k", "v", "lengths", "workspace"}
+    with FakeTensorMode():
+        model, cache = model_and_cache()
+        logits = _DecodeStep.make(model, cache)(torch.zeros(2, 1, dtype=torch.int64, device="cuda:0"), cache)
+        assert logits.shape == (2, 64) and logits.dtype == torch.bfloat16
