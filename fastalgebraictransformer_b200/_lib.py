@@ -130,6 +130,13 @@ def check_device_status(device=None) -> None:
                            f"(code {(v >> 24) & 0xf}: a bounded wait inside a kernel ran out, detail {v & 0xffffff})")
 
 
+def check_waits(device) -> None:
+    """Synchronise and raise if a bounded wait inside a kernel has run out on `device`; whatever else the status word holds
+    stays for ``check_device_status``."""
+    if (int(device_status(torch.device(device)).item()) >> 24) & 0xf:
+        check_device_status(device)
+
+
 class device_guard:
     """Make ``device`` current for the duration of a launch (no-op when it already is)."""
 

@@ -19,7 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.utils.checkpoint import checkpoint
 
-from . import ops
+from . import _lib, ops
 from .backward import rational_attention_packed
 from .forward import compute_alibi_slopes
 from .fused_ops import (EPS, add_mean_error_norm, head_shifted_cross_entropy, mean_error_norm, rational_swiglu,
@@ -381,6 +381,8 @@ class AlgebraicTransformerLM(nn.Module):
                     cache.seen += 1
                 else:
                     logits = self.forward_cached(nxt, cache)
+            if cache.step:
+                _lib.check_waits(idx.device)            # (a step that gave up waiting has NaN logits)
             return idx
         for _ in range(max_new_tokens):
             idx_cond = idx if idx.size(1) <= self.block_size else idx[:, -self.block_size:]

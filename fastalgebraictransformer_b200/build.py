@@ -81,16 +81,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 WAIT_TEST_LIB = os.path.join(PKG, "..", "tests", "_build", "libfat_b200_waittest.so")
-WAIT_TEST_FLAGS = ["-DFAT_TEST_WITHHOLD_V_TILE=0", "-DFAT_TEST_CE_WITHHOLD_ROW=4", "-DFAT_WAIT_HINT_NS=100000", "-DFAT_WAIT_SPINS=30"]
-WAIT_TEST_SOURCES = ("attn_tc_fwd.cu", "loss.cu")
+WAIT_TEST_FLAGS = ["-DFAT_TEST_WITHHOLD_V_TILE=0", "-DFAT_TEST_CE_WITHHOLD_ROW=4", "-DFAT_TEST_LM_WITHHOLD_UNIT=0", "-DFAT_WAIT_HINT_NS=100000",
+                   "-DFAT_WAIT_SPINS=30", "-DFAT_LM_POLL_LIMIT=4096"]
+WAIT_TEST_SOURCES = ("attn_tc_fwd.cu", "loss.cu", "lm_decode.cu")
 
 
 def build_wait_test(force: bool = False, verbose: bool = False) -> str:
     """A TEST-ONLY variant of the library (tests/_build/, never loaded by the package): the attention forward is compiled
     so that its producer leaves out one V tile, the staged loss kernel so that its first block never requests the copy of
-    one row, and every bounded wait gives up after ~3 ms.  tests/test_wait_timeout.py uses it to run the give-up paths
-    once (status word or NaN losses, teardown, TMEM release).  Only those two sources are recompiled; the other objects
-    are the shipped ones."""
+    one row, the language model's decode step so that one unit of its first projection is never handed on, and every bounded
+    wait gives up after ~3 ms.  tests/test_wait_timeout.py uses it to run the give-up paths once (status word, NaN losses or
+    logits, teardown, TMEM release).  Only those sources are recompiled; the other objects are the shipped ones."""
     srcs = [os.path.join(CSRC, n) for n in WAIT_TEST_SOURCES]
     headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + sorted(glob.glob(os.path.join(PKG, "..", "include", "*.h")))
     out_dir = os.path.dirname(WAIT_TEST_LIB)
@@ -102,9 +103,16 @@ def build_wait_test(force: bool = False, verbose: bool = False) -> str:
         return WAIT_TEST_LIB
     nvcc = _nvcc()
     cmds = [[nvcc, *NVCC_FLAGS, *WAIT_TEST_FLAGS, "-c", src, "-o", obj] for src, obj in zip(srcs, objs)]
-    cmds.append([nvcc, "-shared", "-o", WAIT_TEST_LIB, *objs, *others, "-gencode", "arch=compute_100a,code=sm_100a"])
-    for cmd in cmds:
-        r = subprocess.run(cmd, capture_output=True, text=True)
+    link = [nvcc, "-shared", "-o", WAIT_TEST_LIB, *objs, *others, "-gencode", "arch=compute_100a,code=sm_100a"]
+
+    def run(cmd):
+        return subprocess.run(cmd, capture_output=True, text=True)
+
+    with cf.ThreadPoolExecutor(max_workers=len(cmds)) as ex:
+        results = list(ex.map(run, cmds))
+    if all(r.returncode == 0 for r in results):
+        results.append(run(link))
+    for r in results:
         if verbose or r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
         if r.returncode:

@@ -44,7 +44,11 @@ constexpr int kLmThreads = 512, kLmWarps = kLmThreads / 32;
 constexpr int kPieces = 4;                      // 16-byte pieces per chunk; a thread's ring holds 4, 2 or 1 chunks, whatever shared memory leaves
 constexpr size_t kChunkBytes = size_t(kPieces) * kLmThreads * 16;
 constexpr size_t kLmSmemLimit = 220 * 1024;
+#ifdef FAT_LM_POLL_LIMIT                        // (test builds only)
+constexpr int kPollLimit = FAT_LM_POLL_LIMIT;
+#else
 constexpr int kPollLimit = 1 << 21;             // about a second
+#endif
 
 struct LmLayerArgs {
   const void *norm1, *qkv, *out, *norm2, *gate_val, *down;
@@ -54,7 +58,7 @@ struct LmLayerArgs {
 struct LmArgs {
   LmLayerArgs layer[FAT_LM_MAX_LAYERS];
   const int64_t* ids; const void* embed; const void* norm; const void* head; void* logits; int* n_cached; int* status;
-  unsigned* ctl;                                // [0] launches so far, [1] CTAs that have left this one (0 between launches)
+  unsigned* ctl;                                // [0] launches so far, [1] CTAs that have left this one, [2] one of them gave up waiting (both 0 between launches)
   // tagged words, two copies each (even / odd layers): float32 values qkv [B][3C], o [B][C], pend [B][C], part [B*H][n_split]
   // [D + 2] (n_split > 1); pairs of 16-bit values att [B][C/2], act [B][act_words]
   uint2 *qkv, *o, *pend, *att, *act, *part;
@@ -522,7 +526,7 @@ template <typename T, int D, int MR, int kStages>
 __global__ void __launch_bounds__(kLmThreads, 1)
 lm_decode_kernel(const __grid_constant__ LmArgs p) {
   extern __shared__ __align__(16) unsigned char lm_smem[];
-  __shared__ int failed;
+  __shared__ int failed, last;
   __shared__ float sums[kLmWarps];
   constexpr int kTile = MR * 64;                 // partial sums of a warp: [row 0..MR*8)[col 0..8)
   unsigned char* A = lm_smem + kStages * kChunkBytes;
@@ -637,8 +641,16 @@ lm_decode_kernel(const __grid_constant__ LmArgs p) {
               const float a1 = v0.y * rsigmoid(v0.y, rcp1p_abs(v0.y)) * as_stored<T>(v1.y);
               st_word(act + int64_t(tok) * p.act_words + n / 2, Pair16<T>::put(a0, a1), tag + 3);
             } else {
+#ifdef FAT_TEST_LM_WITHHOLD_UNIT
+              // test builds only (never the shipped library): the words of this unit of the first block's projection are not written, so
+              // every wait for them runs out
+              if (li != 0 || ph != 0 || unit != FAT_TEST_LM_WITHHOLD_UNIT) {
+#else
+              {
+#endif
               uint2* out = ph == 0 ? p.qkv + odd * B * 3 * C : ph == 1 ? p.o + odd * B * C : p.pend + odd * B * C;
               st_words(out + int64_t(tok) * cn.N + n, __float_as_uint(v0.x), __float_as_uint(v0.y), ph == 0 ? tag : ph == 1 ? tag + 2 : tag + 4);
+              }
             }
           }
         }
@@ -649,13 +661,28 @@ lm_decode_kernel(const __grid_constant__ LmArgs p) {
     add = ph == 1 ? p.o + odd * B * C : ph == 3 ? p.pend + odd * B * C : nullptr;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (threadIdx.x == 0) {                        // the last CTA to leave: nobody reads the lengths and the launch number any more
+  // The last CTA to leave: nobody reads the lengths and the launch number any more.  A step in which a wait ran out (the words
+  // behind it are whatever the CTA had in its registers, and spread) gives NaN logits and does not count.
+  if (threadIdx.x == 0) {
+    if (failed) atomicExch(p.ctl + 2, 1u);
     __threadfence();
-    if (atomicAdd(p.ctl + 1, 1u) == gridDim.x - 1) {
+    last = atomicAdd(p.ctl + 1, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    const bool bad = __ldcg(p.ctl + 2) != 0u;
+    if (bad)
+#pragma unroll 1
+      for (int64_t i = threadIdx.x; i < int64_t(B) * p.V; i += kLmThreads) static_cast<T*>(p.logits)[i] = Elem<T>::from_c(__int_as_float(0x7fc00000));
+    __syncthreads();                             // (everyone has read the mark)
+    if (threadIdx.x == 0) {
+      p.ctl[2] = 0u;
       p.ctl[1] = 0u;
       p.ctl[0] += 1u;
 #pragma unroll 1
-      for (int b = 0; b < B; ++b) p.n_cached[b] += 1;
+      for (int b = 0; b < B; ++b)
+        if (!bad && p.n_cached[b] >= 0 && p.n_cached[b] < p.capacity) p.n_cached[b] += 1;      // (a sequence without room has been given no row)
     }
   }
 }

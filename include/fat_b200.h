@@ -317,7 +317,9 @@ FAT_API int fat_attn_decode(const void* q, const void* k_new, const void* v_new,
  * element strides, the same for all layers.  slopes: H values per layer, float32 (slopes_f32) or of the tensor dtype.
  * workspace: fat_lm_decode_workspace_bytes bytes (0: the shape is not covered), zeroed once before its first use, used by
  * one step at a time.  Covered: 1-16 sequences, D in {64, 128}, up to FAT_LM_MAX_LAYERS layers, activation rows that fit
- * shared memory.  An id outside [0, V) gives that sequence NaN logits.  dtypes: BF16, F16.
+ * shared memory.  An id outside [0, V) gives that sequence NaN logits.  A sequence whose cache has no room is given no row, its
+ * length stays and bit 28 of the status word is set.  When a wait inside the launch runs out, the status word says so, all
+ * logits are NaN and no length moves.  dtypes: BF16, F16.
  * ---------------------------------------------------------------------------------- */
 #define FAT_LM_MAX_LAYERS 48
 typedef struct fat_lm_layer {

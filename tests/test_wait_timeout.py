@@ -94,3 +94,95 @@ def test_a_copy_that_never_arrives_ends_in_nan_losses_and_a_usable_gpu():
     want = oracle.shifted_cross_entropy(logits.float(), labels)
     got = fat.shifted_cross_entropy(ld, lab)
     assert abs(got.item() - want.item()) < 4e-2               # (the loss comes back in the logits' dtype: bfloat16 near 8.8 has steps of 0.06)
+
+
+class LmLayer(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("norm1", "qkv", "out", "norm2", "gate_val", "down", "k_cache", "v_cache", "slopes")]
+
+
+def _lm_step(lib, model, cache, ids, workspace, lengths, logits, status):
+    """fat_lm_decode_step of `lib` on a model's parameters and a cache."""
+    from fastalgebraictransformer_b200 import _lib
+    fn = lib.fat_lm_decode_step
+    fn.restype, fn.argtypes = _lib.PROTOTYPES["fat_lm_decode_step"]
+    layers = (LmLayer * len(model.blocks))()
+    for i, b in enumerate(model.blocks):
+        layers[i] = LmLayer(*[t.data_ptr() for t in (b.norm1.weight, b.attn.qkv.weight, b.attn.out.weight, b.norm2.weight, b.ffn.w_gate_val.weight,
+                                                     b.ffn.w_out.weight, cache.k[i], cache.v[i], b.attn.alibi_slopes)])
+    B, H, capacity, D = cache.k[0].shape
+    w = model.head.weight
+    return fn(ctypes.addressof(layers), len(model.blocks), ids.data_ptr(), ids.stride(0), model.embed.weight.data_ptr(), model.norm.weight.data_ptr(),
+              w.data_ptr(), logits.data_ptr(), lengths.data_ptr(), _lib.strides3(cache.k[0]), int(model.blocks[0].attn.alibi_slopes.dtype == torch.float32),
+              workspace.data_ptr(), workspace.numel(), B, w.shape[1], H, D, model.blocks[0].ffn.w_out.weight.shape[1], w.shape[0], capacity, D ** -0.5,
+              1e-6, 1e-6, _lib.BF16, status.data_ptr(), _lib.stream_ptr(w.device))
+
+
+def _lm_case(B=2, n=9):
+    import fastalgebraictransformer_b200 as fat
+    torch.manual_seed(9)
+    model = fat.AlgebraicTransformerLM(vocab_size=300, d_model=256, n_head=4, n_layers=3, dropout=0.0, block_size=64).to("cuda").to(torch.bfloat16).eval()
+    ids = torch.randint(0, 300, (B, n), device="cuda")
+    cache = model.new_cache(B, n)
+    model.forward_cached(ids[:, :n - 1].contiguous(), cache)
+    w = model.head.weight
+    nbytes = torch.ops.algebraic.lm_decode_workspace_bytes(B, 256, 4, 64, model.blocks[0].ffn.w_out.weight.shape[1], 300, 3, n, w.dtype)
+    return model, cache, ids[:, n - 1:].contiguous(), torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+
+
+def test_words_that_never_arrive_end_in_nan_logits_and_a_usable_step():
+    """The decode step of the language model: in the test build one unit of the first projection is never handed on.  The CTAs
+    that need it give up after ~3 ms, all return, the logits are NaN, no length moves; the shipped library then takes the same
+    step in the same workspace and gives the module-by-module logits."""
+    if not os.path.exists(LIB):
+        pytest.skip("tests/_build/libfat_b200_waittest.so has not been built")
+    from fastalgebraictransformer_b200 import _lib
+    model, cache, ids, workspace = _lm_case()
+    logits = torch.zeros(2, 300, dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    lengths = cache.lengths.clone()
+    assert _lm_step(ctypes.CDLL(LIB), model, cache, ids, workspace, lengths, logits, status) == 0
+    torch.cuda.synchronize()
+    assert (status.item() >> 24) & 0xf == 1 and status.item() & 0xffffff == 300, f"status word 0x{status.item():08x}"
+    assert torch.isnan(logits).all()
+    assert torch.equal(lengths, cache.lengths)
+
+    status.zero_()
+    assert _lm_step(_lib.lib(), model, cache, ids, workspace, lengths, logits, status) == 0
+    torch.cuda.synchronize()
+    assert status.item() == 0 and lengths.tolist() == [9, 9]
+    cache.step = False
+    want = model.forward_cached(ids, cache)
+    assert ((logits.float() - want.float()).abs().max() / want.float().abs().max()).item() < 4 * 2.0 ** -8      # (as the fused step's tests)
+
+
+def test_a_sequence_without_room_keeps_its_length():
+    from fastalgebraictransformer_b200 import _lib
+    model, cache, ids, workspace = _lm_case()
+    lengths = torch.tensor([8, 9], dtype=torch.int32, device="cuda")           # the second sequence's cache is full
+    logits = torch.zeros(2, 300, dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for t in cache.k + cache.v:
+        t[:, :, 8] = 0.0
+    before = [t.clone() for t in cache.k + cache.v]
+    assert _lm_step(_lib.lib(), model, cache, ids, workspace, lengths, logits, status) == 0
+    torch.cuda.synchronize()
+    assert status.item() == 0x10000000 and lengths.tolist() == [9, 9]
+    assert torch.isfinite(logits).all()
+    for t, b in zip(cache.k + cache.v, before):
+        assert torch.equal(t[1], b[1]) and not torch.equal(t[0, :, 8], b[0, :, 8])
+
+
+def test_generate_reports_a_step_that_gave_up():
+    """The status word is read once at the end; another report in it is left for check_device_status."""
+    import fastalgebraictransformer_b200 as fat
+    from fastalgebraictransformer_b200 import _lib
+    model, _, ids, _ = _lm_case()
+    word = _lib.device_status(torch.device("cuda", 0))
+    word.fill_(1 << 24 | 300)
+    with pytest.raises(RuntimeError, match="ran out"):
+        model.generate(ids, 4, top_k=1)
+    assert word.item() == 0
+    word.fill_(0x10000000)
+    assert model.generate(ids, 4, top_k=1).shape == (2, 5)
+    with pytest.raises(RuntimeError, match="without room"):
+        fat.check_device_status()
