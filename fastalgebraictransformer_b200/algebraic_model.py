@@ -160,8 +160,8 @@ class _DecodeStep:
     and the conditions under which it stands for the modules' own forward passes: stock modules without hooks or methods
     of their own, nothing that drops out, the constants they had.  ``None`` from ``make`` means the step runs module by module."""
 
-    def __init__(self, parameters, rest, watch, hooks, model):
-        self.parameters, self.rest, self.watch, self.hooks, self.model = parameters, rest, watch, hooks, model
+    def __init__(self, parameters, rest, watch, hooks, model, replays_well):
+        self.parameters, self.rest, self.watch, self.hooks, self.model, self.replays_well = parameters, rest, watch, hooks, model, replays_well
         self.expected = [d.get(k) for d, k in watch]
 
     @staticmethod
@@ -208,8 +208,21 @@ class _DecodeStep:
         if nbytes == 0:
             return None
         workspace = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        step = _DecodeStep((*tops, params, slopes), (workspace, float(first.attn.scale), float(model.norm.eps), float(EPS)), watch, hooks, model)
+        step = _DecodeStep((*tops, params, slopes), (workspace, float(first.attn.scale), float(model.norm.eps), float(EPS)), watch, hooks, model,
+                           _DecodeStep.beats_replayed_operators(B, *reversed(first.ffn.w_out.weight.shape)))
         return step if step.stands(model) else None
+
+    @staticmethod
+    def beats_replayed_operators(B: int, d_ffn: int, d_model: int) -> bool:
+        """Whether a replay of this launch takes less than a replay of the operators' launches (issued one by one those always
+        lose).  Every CTA normalises the tokens of the whole step (8 or 16 rows) for itself, and long rows leave its ring fewer
+        chunks, so the line is drawn at the size of that tile; for one sequence the operators' contractions are matrix-vector
+        products, which only wide models with aligned rows lose to.  us, fused / operators, 512 cached tokens unless said:
+        768 x 12 blocks, 8 sequences 373 / 455, 16 sequences 566 / 465; 1024 x 24 blocks, 8: 973 / 1197, 16: 1493 / 1229;
+        512 x 8 blocks, 16: 314 / 447; 1280 x 8 blocks, 4: 463 / 463 (1800 tokens 525 / 491); 1536 x 24 blocks, 1: 1243 / 1085, 8: 1423 / 1129;
+        one sequence: 768 x 12 blocks 380 / 460, 1024 x 24 blocks 956 / 986, 512 x 8 blocks 267 / 226, 256 x 4 blocks 109 / 92.
+        Heads of 128 (768 x 12 blocks, 8 sequences): 463 / 461, with 64 cached tokens 399 / 431."""
+        return (8 if B <= 8 else 16) * d_model <= 8192 and (B > 1 or (d_model >= 768 and d_ffn % 2 == 0))
 
     def stands(self, model) -> bool:
         """Whether the model is still the one this step was made of (a parameter may be changed in place or moved; the
@@ -347,8 +360,9 @@ class AlgebraicTransformerLM(nn.Module):
         for every token; here (``use_cache``, an extension) the prompt runs once, its keys and values are kept, and each
         new token costs one decode step.  The two agree as long as the reference would not crop the prefix to
         ``block_size``; when it would (or the decode kernel does not cover the model), the reference's loop runs.
-        ``cuda_graph``: a decode step is a hundred small launches whatever the length (the cached lengths live on the
-        device), so after one step issued launch by launch it is captured once and replayed for the remaining tokens."""
+        ``cuda_graph``: a decode step is the same launches whatever the length (the cached lengths live on the device) - one,
+        or a hundred small ones -, so after one step issued launch by launch it is captured once and replayed for the
+        remaining tokens, whichever way the replay is faster (``_DecodeStep.beats_replayed_operators``)."""
         def sample(logits):
             if temperature != 1.0:
                 logits = logits / temperature
@@ -361,6 +375,11 @@ class AlgebraicTransformerLM(nn.Module):
         if use_cache and max_new_tokens > 0 and idx.size(1) > 0 and longest <= self.block_size and self.cache_supported():
             cache = self.new_cache(idx.size(0), longest)
             logits = self.forward_cached(idx, cache)
+            replayed = cuda_graph and max_new_tokens > 5    # worth a capture
+            if replayed:
+                cache.step = _DecodeStep.make(self, cache) or False
+                if cache.step and not cache.step.replays_well:
+                    cache.step = False
             graph = token = None
             for step in range(max_new_tokens):
                 nxt = sample(logits)
@@ -371,7 +390,7 @@ class AlgebraicTransformerLM(nn.Module):
                     token.copy_(nxt)
                     graph.replay()
                     cache.seen += 1                         # (the device-side lengths advance inside the graph)
-                elif cuda_graph and step == 1 and max_new_tokens - step > 4:
+                elif replayed and step == 1:
                     token, seen = nxt.clone(), cache.seen
                     graph = torch.cuda.CUDAGraph()
                     with torch.cuda.graph(graph):

@@ -379,6 +379,19 @@ def test_what_the_fused_step_does_not_take_runs_module_by_module(what, late):
         assert torch.equal(got[..., :9, :] if got.dim() == 4 else got, want[..., :9, :] if want.dim() == 4 else want)
 
 
+@pytest.mark.parametrize("B,new,fused", [(2, 12, True), (1, 12, False), (9, 12, False), (1, 4, True)])
+def test_generate_replays_the_faster_way(B, new, fused, monkeypatch):
+    """A captured step is the single launch only where its replay wins (width 768: up to 8 sequences; width 128: more than one); a
+    few tokens are stepped without a capture, where it always does."""
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    calls, stock = [], _DecodeStep.__call__
+    monkeypatch.setattr(_DecodeStep, "__call__", lambda self, *a: calls.append(1) or stock(self, *a))
+    model = _half_model(d_model=768, n_head=12) if B == 9 else _half_model()
+    prompt = torch.randint(0, 64, (B, 7), device=DEV)
+    assert model.generate(prompt, new, top_k=1).shape == (B, 7 + new)
+    assert bool(calls) == fused
+
+
 def test_fused_decode_step_yields_to_hooks_and_replaced_modules():
     from fastalgebraictransformer_b200 import AlgebraicTransformerLM
     torch.manual_seed(3)

@@ -154,3 +154,13 @@ def test_decode_step_operator_declares_what_it_writes_and_its_shape():
         model, cache = model_and_cache()
         logits = _DecodeStep.make(model, cache)(torch.zeros(2, 1, dtype=torch.int64, device="cuda:0"), cache)
         assert logits.shape == (2, 64) and logits.dtype == torch.bfloat16
+
+
+@pytest.mark.parametrize("B,d_model,d_ffn,fused", [
+    (8, 768, 2048, True), (8, 1024, 2730, True), (16, 512, 1365, True), (1, 768, 2048, True), (1, 1024, 2730, True), (2, 512, 1365, True),
+    (9, 768, 2048, False), (16, 1024, 2730, False), (1, 512, 1365, False), (1, 896, 2389, False), (4, 1280, 3413, False), (1, 1536, 4096, False),
+])
+def test_which_way_a_captured_step_goes(B, d_model, d_ffn, fused):
+    """On both sides of the line: at these sizes the launch was measured faster, or slower, than the operators' replay."""
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    assert _DecodeStep.beats_replayed_operators(B, d_ffn, d_model) == fused
