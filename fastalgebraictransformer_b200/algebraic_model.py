@@ -71,6 +71,10 @@ class KVCache:
         self.seen = 0                                   # host copy of the (common) length
         self.step = None                                # the fused decode step of the model that fills this cache (_DecodeStep)
 
+    def __getstate__(self):
+        """Copies and saved caches leave the fused step behind: it holds the model and a workspace that one cache uses at a time."""
+        return {**self.__dict__, "step": None}
+
     def layer(self, i: int):
         return self.k[i], self.v[i], self
 

@@ -164,3 +164,15 @@ def test_which_way_a_captured_step_goes(B, d_model, d_ffn, fused):
     """On both sides of the line: at these sizes the launch was measured faster, or slower, than the operators' replay."""
     from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
     assert _DecodeStep.beats_replayed_operators(B, d_ffn, d_model) == fused
+
+
+def test_copies_of_a_cache_leave_the_step_behind():
+    """A step's workspace serves one cache at a time, and a saved cache must not carry the model."""
+    import copy
+    import pickle
+    from fastalgebraictransformer_b200.algebraic_model import KVCache
+    cache = KVCache(2, 1, 2, 8, 64, torch.float32, "cpu")
+    cache.step, cache.seen = Step(), 3
+    for other in (copy.copy(cache), copy.deepcopy(cache), pickle.loads(pickle.dumps(cache))):
+        assert other.step is None and other.seen == 3 and torch.equal(other.lengths, cache.lengths)
+    assert isinstance(cache.step, Step)
