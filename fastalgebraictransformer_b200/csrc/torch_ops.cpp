@@ -9,6 +9,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
@@ -508,6 +509,8 @@ Tensor lm_decode_step(const Tensor& ids, const Tensor& embed, const Tensor& norm
   TORCH_CHECK(k[0].size(0) == B && C == H * D, "the caches must be [B,H,capacity,D] of the model");
   Tensor logits = empty_of({B, V}, head);
   c10::cuda::CUDAGuard guard(head.device());
+  // the caller does not see the workspace: it may be dropped (a changed model makes a new step) while another stream than its own uses it
+  c10::cuda::CUDACachingAllocator::recordStream(workspace.storage().data_ptr(), at::cuda::getCurrentCUDAStream(head.get_device()));
   check(fat_lm_decode_step(layers.data(), int(L), ids.data_ptr<int64_t>(), ids.stride(0), param(embed, {V, C}), param(norm, {C}), param(head, {V, C}),
                            logits.data_ptr(), lengths.data_ptr<int>(), cs.data(), slopes_f32, workspace.data_ptr(), size_t(workspace.numel()),
                            int(B), int(C), int(H), int(D), int(F), int(V), int(cap), scale, eps_norm, eps_attn, dtype_tag(head),

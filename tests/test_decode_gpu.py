@@ -392,6 +392,26 @@ def test_generate_replays_the_faster_way(B, new, fused, monkeypatch):
     assert bool(calls) == fused
 
 
+def test_workspace_outlives_its_last_launch_on_another_stream():
+    """A step dropped while its launch still waits on a side stream: its workspace must not be handed out again yet."""
+    model = _half_model()
+    cache = model.new_cache(2, 12)
+    ids = torch.randint(0, 64, (2, 8), device=DEV)
+    model.forward_cached(ids[:, :4], cache)
+    model.forward_cached(ids[:, 4:5], cache)
+    address, nbytes = cache.step.rest[0].data_ptr(), cache.step.rest[0].numel()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)               # about 50 ms
+        model.forward_cached(ids[:, 5:6], cache)
+    cache.step = None
+    taken = [torch.empty(nbytes, dtype=torch.uint8, device=DEV) for _ in range(4)]
+    still_waiting = not side.query()
+    assert still_waiting and address not in [t.data_ptr() for t in taken]
+    torch.cuda.current_stream().wait_stream(side)
+
+
 def test_fused_decode_step_yields_to_hooks_and_replaced_modules():
     from fastalgebraictransformer_b200 import AlgebraicTransformerLM
     torch.manual_seed(3)
