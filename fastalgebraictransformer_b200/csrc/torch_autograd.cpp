@@ -16,10 +16,12 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/library.h>
 
 #include <string>
 #include <tuple>
+#include <type_traits>
 
 namespace {
 
@@ -122,9 +124,43 @@ void no_forward_mode(const char* what, const Ts&... ts) {
   TORCH_CHECK_NOT_IMPLEMENTED(!any, "algebraic::", what, " does not support forward-mode automatic differentiation");
 }
 
-struct RationalSoftmaxBackward : Node {
+// What the nodes have in common.  N::attributes(f) shows f everything the backward depends on: f(SavedVariable&, is_output) and
+// f(constant).  Compiled autograd collects it and runs apply() on tensors of its own in the saved ones' place; the gradients it
+// passes have no shape yet, so an apply() hands them to its operator as they are.
+template <typename N>
+struct OperatorNode : Node {
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    self().attributes([](auto& a, bool = false) {
+      if constexpr (std::is_same_v<std::decay_t<decltype(a)>, SavedVariable>) a.reset_data();
+    });
+  }
+  void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+    const_cast<OperatorNode*>(this)->self().attributes([&](auto& a, bool is_output = false) {
+      if constexpr (std::is_same_v<std::decay_t<decltype(a)>, SavedVariable>) args.collect(a, is_output);
+      else args.collect(a);
+    });
+  }
+  variable_list apply_with_saved(const variable_list& inputs, torch::dynamo::autograd::SwapSavedVariables& saved) override {
+    self().attributes([&](auto& a, bool = false) { saved.before(a); });
+    traced = true;
+    variable_list out = this->apply(variable_list(inputs));
+    traced = false;
+    self().attributes([&](auto& a, bool = false) { saved.after(a); });
+    return out;
+  }
+
+ protected:
+  bool traced = false;
+
+ private:
+  N& self() { return static_cast<N&>(*this); }
+};
+
+struct RationalSoftmaxBackward : OperatorNode<RationalSoftmaxBackward> {
   SavedVariable x;
   double eps = 0;
+  template <typename F> void attributes(F&& f) { f(x, false); f(eps); }
   std::string name() const override { return "RationalSoftmaxBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -133,7 +169,6 @@ struct RationalSoftmaxBackward : Node {
     BackwardScope scope;
     return {op_softmax_bwd(grads[0], xt, eps)};
   }
-  void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); x.reset_data(); }
 };
 
 // The two inputs are often the halves of one packed projection, `gate, value = gv.chunk(2, -1)`.  Autograd would then
@@ -141,9 +176,10 @@ struct RationalSoftmaxBackward : Node {
 // found to be such a pair, the node has a third edge straight to the projection, and its backward sends ONE packed gradient
 // along it and nothing to the halves - unless somebody wants to see the halves' gradients themselves (hooks, retain_grad,
 // torch.autograd.grad with respect to them), in which case they get them as before.
-struct RationalSwiGLUBackward : Node {
+struct RationalSwiGLUBackward : OperatorNode<RationalSwiGLUBackward> {
   SavedVariable gate, value;
   bool halves = false;                                  // edge 2 leads to the packed tensor
+  template <typename F> void attributes(F&& f) { f(gate, false); f(value, false); f(halves); }
   std::string name() const override { return "RationalSwiGLUBackward"; }
 
   static bool watched(Node* n) {
@@ -161,7 +197,7 @@ struct RationalSwiGLUBackward : Node {
     variable_list out(num_outputs());
     if (!grads[0].defined()) return out;
     const Tensor g = gate.unpack(), v = value.unpack();
-    const bool to_packed = halves && !at::GradMode::is_enabled() && task_should_compute_output(2) &&
+    const bool to_packed = halves && !traced && !at::GradMode::is_enabled() && task_should_compute_output(2) &&
                            !watched(next_edge(0).function.get()) && !watched(next_edge(1).function.get());
     BackwardScope scope;
     if (to_packed) {
@@ -171,7 +207,6 @@ struct RationalSwiGLUBackward : Node {
     }
     return out;
   }
-  void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); gate.reset_data(); value.reset_data(); }
 };
 
 // Whether gate and value are the two halves along the last dimension of one dense tensor that they were taken from by
@@ -191,9 +226,10 @@ optional<torch::autograd::Edge> packed_edge(const Tensor& gate, const Tensor& va
   return to;
 }
 
-struct MeanErrorNormBackward : Node {
+struct MeanErrorNormBackward : OperatorNode<MeanErrorNormBackward> {
   SavedVariable x, weight, mean;
   double eps = 0;
+  template <typename F> void attributes(F&& f) { f(x, false); f(weight, false); f(mean, false); f(eps); }
   std::string name() const override { return "MeanErrorNormBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -203,12 +239,12 @@ struct MeanErrorNormBackward : Node {
     auto [dx, dw] = op_norm_bwd(grads[0], xt, wt, mt, eps);
     return {dx, dw};
   }
-  void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); x.reset_data(); weight.reset_data(); mean.reset_data(); }
 };
 
-struct AddMeanErrorNormBackward : Node {
+struct AddMeanErrorNormBackward : OperatorNode<AddMeanErrorNormBackward> {
   SavedVariable h, weight, mean;                        // h (an output), not x and residual: the backward only needs their sum
   double eps = 0;
+  template <typename F> void attributes(F&& f) { f(h, true); f(weight, false); f(mean, false); f(eps); }
   std::string name() const override { return "AddMeanErrorNormBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -220,13 +256,16 @@ struct AddMeanErrorNormBackward : Node {
     auto [ds, dw] = op_add_norm_bwd(dy, dh.defined() ? optional<Tensor>(dh) : optional<Tensor>(), ht, wt, mt, eps);
     return {ds, ds, dw};
   }
-  void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); h.reset_data(); weight.reset_data(); mean.reset_data(); }
 };
 
-struct RationalAttentionBackward : Node {
+struct RationalAttentionBackward : OperatorNode<RationalAttentionBackward> {
   SavedVariable q, k, v, out, L, lo, slopes, bits;
   double scale = 0, eps = 0;
   bool causal = true;
+  template <typename F> void attributes(F&& f) {
+    f(q, false); f(k, false); f(v, false); f(out, true); f(L, false); f(lo, false); f(slopes, false); f(bits, false);
+    f(scale); f(eps); f(causal);
+  }
   std::string name() const override { return "RationalAttentionBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -237,28 +276,19 @@ struct RationalAttentionBackward : Node {
     auto [dq, dk, dv] = op_attn_bwd(qt, kt, vt, ot, lt, Lt, grads[0], st, scale, causal, eps, bt.defined() ? optional<Tensor>(bt) : optional<Tensor>());
     return {dq, dk, dv};
   }
-  void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&q, &k, &v, &out, &L, &lo, &slopes, &bits}) s->reset_data();
-  }
 };
 
-struct RationalAttentionPackedBackward : Node {
+struct RationalAttentionPackedBackward : OperatorNode<RationalAttentionPackedBackward> {
   SavedVariable qkv, out, L, lo, slopes, bits;          // out: the result [B,T,H*D] itself, so that a change in place is noticed
   double scale = 0, eps = 0;
+  template <typename F> void attributes(F&& f) { f(qkv, false); f(out, true); f(L, false); f(lo, false); f(slopes, false); f(bits, false); f(scale); f(eps); }
   std::string name() const override { return "RationalAttentionPackedBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined()) return {Tensor()};
-    const Tensor pt = qkv.unpack(), tokens = out.unpack(shared_from_this()), Lt = L.unpack(), lt = lo.unpack(), st = slopes.unpack(), bt = bits.unpack();
+    const Tensor pt = qkv.unpack(), ot = out.unpack(shared_from_this()), Lt = L.unpack(), lt = lo.unpack(), st = slopes.unpack(), bt = bits.unpack();
     BackwardScope scope;
-    auto heads = [&](const Tensor& t) { return t.reshape({pt.size(0), pt.size(1), pt.size(3), pt.size(4)}).permute({0, 2, 1, 3}); };
-    const Tensor ot = heads(tokens), d = heads(grads[0]);
-    return {op_attn_bwd_packed(pt, ot, lt, Lt, d, st, scale, eps, bt.defined() ? optional<Tensor>(bt) : optional<Tensor>())};
-  }
-  void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&qkv, &out, &L, &lo, &slopes, &bits}) s->reset_data();
+    return {op_attn_bwd_packed(pt, ot, lt, Lt, grads[0], st, scale, eps, bt.defined() ? optional<Tensor>(bt) : optional<Tensor>())};
   }
 };
 

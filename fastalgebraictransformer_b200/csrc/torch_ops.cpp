@@ -432,12 +432,15 @@ std::tuple<Tensor, Tensor, Tensor> attn_fwd_packed(const Tensor& qkv, const Tens
   return attn_fwd(h[0], h[1], h[2], slopes, scale, true, eps, 0, true, key_mask, residual);
 }
 
+// (out and d_out either as heads, [B,H,T,D], or as the caller of the packed forward holds them, [B,T,H*D])
 Tensor attn_bwd_packed(const Tensor& qkv, const Tensor& out, const Tensor& out_lo, const Tensor& L, const Tensor& d_out,
                        const Tensor& slopes, double scale, double eps, const c10::optional<Tensor>& key_mask) {
   const auto h = heads_of(qkv);
+  const int64_t B = qkv.size(0), T = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
+  auto as_heads = [&](const Tensor& t) { return t.dim() == 3 ? t.reshape({B, T, H, D}).permute({0, 2, 1, 3}) : t; };
   Tensor packed = empty_of(qkv.sizes(), qkv);
   const auto d = heads_of(packed);
-  attn_bwd_into(h[0], h[1], h[2], out, out_lo, L, d_out, slopes, scale, true, eps, 0, key_mask, d[0], d[1], d[2]);
+  attn_bwd_into(h[0], h[1], h[2], as_heads(out), out_lo, L, as_heads(d_out), slopes, scale, true, eps, 0, key_mask, d[0], d[1], d[2]);
   return packed;
 }
 
