@@ -92,18 +92,25 @@ def rational_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, alibi_
                        causal: bool = True, eps: float = EPS, key_mask: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Memory-efficient rational attention with a custom backward (reference backward.py:386-396).  ``key_mask`` (an
     extension): padding mask [B, T], 0 = the key is padding and weighs nothing for any query."""
-    if torch.compiler.is_compiling():
+    out = NotImplemented
+    if not torch.compiler.is_compiling():
+        mask, covers = _host_mask(key_mask)
+        out = ops.host.rational_attention(q, k, v, alibi_slopes, scale, causal, eps, mask, covers)
+    if out is NotImplemented:
         return RationalAttentionFunction.apply(q, k, v, alibi_slopes, scale, causal, eps, _lib.PATH_AUTO, False, key_mask)
-    if key_mask is None or isinstance(key_mask, torch.Tensor):
-        return ops.host.rational_attention(q, k, v, alibi_slopes, scale, causal, eps, key_mask, -1)
-    return ops.host.rational_attention(q, k, v, alibi_slopes, scale, causal, eps, key_mask.bits, key_mask.n_tokens)
+    return out
 
 
 def rational_attention_packed(qkv: torch.Tensor, alibi_slopes: torch.Tensor, scale: float, eps: float = EPS, key_mask=None) -> torch.Tensor:
     """Causal rational attention of a packed projection [B, T, 3, H, D] -> [B, T, H*D]: RationalAttentionPackedFunction with
     its node in C++ (reference algebraic_model.py:89-107)."""
-    if torch.compiler.is_compiling():
-        return RationalAttentionPackedFunction.apply(qkv, alibi_slopes, scale, eps, key_mask)
-    if key_mask is None or isinstance(key_mask, torch.Tensor):
-        return ops.host.rational_attention_packed(qkv, alibi_slopes, scale, eps, key_mask, -1)
-    return ops.host.rational_attention_packed(qkv, alibi_slopes, scale, eps, key_mask.bits, key_mask.n_tokens)
+    out = NotImplemented
+    if not torch.compiler.is_compiling():
+        mask, covers = _host_mask(key_mask)
+        out = ops.host.rational_attention_packed(qkv, alibi_slopes, scale, eps, mask, covers)
+    return RationalAttentionPackedFunction.apply(qkv, alibi_slopes, scale, eps, key_mask) if out is NotImplemented else out
+
+
+def _host_mask(key_mask):
+    """None, a [B, T] mask or a PackedKeyMask as ``ops.host`` takes it: the tensor, and the tokens it covers if it is packed."""
+    return (key_mask, -1) if key_mask is None or isinstance(key_mask, torch.Tensor) else (key_mask.bits, key_mask.n_tokens)

@@ -7,6 +7,7 @@
 // node is a plain C++ Node with SavedVariables, and its backward calls the backward operator without going through the
 // interpreter.  The operators below the autograd key are the ones of torch_ops.cpp and are reached through the dispatcher,
 // so modes that watch operators (fake tensors, profilers, functionalisation) see what they saw before.
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -492,6 +493,29 @@ bool cuda_arg(const Tensor& t, const char* fn) {
   PyErr_SetString(PyExc_RuntimeError, (std::string(fn) + ": CUDA tensor required — this build has no CPU fallback").c_str());
   return false;
 }
+// Whether a call has to be seen by __torch_function__ (a mode, or a tensor of a class that defines it) or by a functorch transform:
+// the autograd Functions' business, and the caller is told so with NotImplemented.  (A plain tensor costs a type and a bit test.)
+bool not_ours(PyObject* o) {
+  const Tensor& t = THPVariable_Unpack(o);
+  if (t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper}))) return true;
+  if (THPVariable_CheckExact(o)) return false;
+  static PyObject* const disabled = [] {
+    PyObject* m = PyImport_ImportModule("torch._C");
+    PyObject* f = m ? PyObject_GetAttrString(m, "_disabled_torch_function_impl") : nullptr;
+    Py_XDECREF(m);
+    if (!f) PyErr_Clear();
+    return f;
+  }();
+  PyObject* f = PyObject_GetAttrString(reinterpret_cast<PyObject*>(Py_TYPE(o)), "__torch_function__");
+  if (!f) PyErr_Clear();
+  Py_XDECREF(f);
+  return f != nullptr && f != disabled;
+}
+template <typename... Os>
+bool not_ours(PyObject* o, Os... os) { return not_ours(o) || not_ours(os...); }
+#define FAT_LEAVE_TO_PYTHON(...) \
+  if (at::impl::torch_function_mode_enabled() || not_ours(__VA_ARGS__)) Py_RETURN_NOTIMPLEMENTED
+
 bool number_arg(PyObject* o, double& out) {
   out = PyFloat_AsDouble(o);
   return !(out == -1.0 && PyErr_Occurred());
@@ -516,6 +540,7 @@ PyObject* py_softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const Tensor* x; double eps;
   if (!count_args(n, 2, "rational_softmax") || !tensor_arg(a[0], "x", x) || !number_arg(a[1], eps) || !cuda_arg(*x, "rational_softmax")) return nullptr;
+  FAT_LEAVE_TO_PYTHON(a[0]);
   Tensor r;
   {
     pybind11::gil_scoped_release nogil;
@@ -531,6 +556,7 @@ PyObject* py_swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor *g, *v;
   if (!count_args(n, 2, "rational_swiglu") || !tensor_arg(a[0], "gate", g) || !tensor_arg(a[1], "value", v) || !cuda_arg(*g, "rational_swiglu")) return nullptr;
   if (!v->is_cuda()) { PyErr_SetString(PyExc_AssertionError, "Inputs must be on CUDA"); return nullptr; }
+  FAT_LEAVE_TO_PYTHON(a[0], a[1]);
   Tensor r;
   {
     pybind11::gil_scoped_release nogil;
@@ -546,6 +572,7 @@ PyObject* py_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor *x, *w; double eps;
   if (!count_args(n, 3, "mean_error_norm") || !tensor_arg(a[0], "x", x) || !tensor_arg(a[1], "weight", w) || !number_arg(a[2], eps) ||
       !cuda_arg(*x, "mean_error_norm")) return nullptr;
+  FAT_LEAVE_TO_PYTHON(a[0], a[1]);
   Tensor r;
   {
     pybind11::gil_scoped_release nogil;
@@ -562,6 +589,7 @@ PyObject* py_add_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!count_args(n, 4, "add_mean_error_norm") || !tensor_arg(a[0], "x", x) || !tensor_arg(a[1], "residual", res) || !tensor_arg(a[2], "weight", w) ||
       !number_arg(a[3], eps) || !cuda_arg(*x, "add_mean_error_norm")) return nullptr;
   if (!res->is_cuda()) { PyErr_SetString(PyExc_AssertionError, "Input must be on CUDA"); return nullptr; }
+  FAT_LEAVE_TO_PYTHON(a[0], a[1], a[2]);
   std::tuple<Tensor, Tensor> r;
   {
     pybind11::gil_scoped_release nogil;
@@ -588,6 +616,7 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyErr_SetString(PyExc_AssertionError, "q, k and v must be CUDA tensors of one shape");
     return nullptr;
   }
+  FAT_LEAVE_TO_PYTHON(a[0], a[1], a[2], a[3]);
   Tensor r;
   {
     pybind11::gil_scoped_release nogil;
@@ -608,6 +637,7 @@ PyObject* py_attention_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyErr_SetString(PyExc_AssertionError, "a packed projection must be a CUDA tensor [B,T,3,H,D]");
     return nullptr;
   }
+  FAT_LEAVE_TO_PYTHON(a[0], a[1]);
   Tensor r;
   {
     pybind11::gil_scoped_release nogil;

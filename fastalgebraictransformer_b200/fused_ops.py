@@ -5,7 +5,8 @@ convenience functions 606-636): same names, argument meaning and assertion behav
 work is done by the sm_100a kernels behind ``torch.ops.algebraic.*``; CPU tensors are
 rejected (this package carries no fallback implementation).  The convenience functions go
 straight to operators whose autograd nodes are C++ (``csrc/torch_autograd.cpp``); the Function
-classes are the same formulas for code that uses them by name or traces them.
+classes are the same formulas for code that uses them by name, traces them or watches them
+(``host`` answers NotImplemented for calls that ``__torch_function__`` or a functorch transform must see).
 """
 from __future__ import annotations
 
@@ -188,27 +189,23 @@ def _require_cuda(t: torch.Tensor, what: str) -> None:
 
 def rational_softmax(x: torch.Tensor, eps: float = EPS) -> torch.Tensor:
     """Apply rational softmax to the last dimension (reference fused_ops.py:606-615)."""
-    if _compiling():
-        return RationalSoftmax.apply(x, eps)
-    return _host.rational_softmax(x, eps)
+    out = NotImplemented if _compiling() else _host.rational_softmax(x, eps)
+    return RationalSoftmax.apply(x, eps) if out is NotImplemented else out
 
 
 def rational_swiglu(gate: torch.Tensor, value: torch.Tensor) -> torch.Tensor:
     """Apply the rational SwiGLU activation (reference fused_ops.py:618-626)."""
-    if _compiling():
-        return RationalSwiGLU.apply(gate, value)
-    return _host.rational_swiglu(gate, value)
+    out = NotImplemented if _compiling() else _host.rational_swiglu(gate, value)
+    return RationalSwiGLU.apply(gate, value) if out is NotImplemented else out
 
 
 def add_mean_error_norm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float = EPS):
     """(x + residual, mean_error_norm(x + residual, weight)) in one pass over the tensors."""
-    if _compiling():
-        return AddMeanErrorNorm.apply(x, residual, weight, eps)
-    return _host.add_mean_error_norm(x, residual, weight, eps)
+    out = NotImplemented if _compiling() else _host.add_mean_error_norm(x, residual, weight, eps)
+    return AddMeanErrorNorm.apply(x, residual, weight, eps) if out is NotImplemented else out
 
 
 def mean_error_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = EPS) -> torch.Tensor:
     """Apply mean-error normalisation (reference fused_ops.py:629-636)."""
-    if _compiling():
-        return MeanErrorNorm.apply(x, weight, eps)
-    return _host.mean_error_norm(x, weight, eps)
+    out = NotImplemented if _compiling() else _host.mean_error_norm(x, weight, eps)
+    return MeanErrorNorm.apply(x, weight, eps) if out is NotImplemented else out

@@ -71,3 +71,61 @@ def test_compiled_autograd_over_an_eager_forward(name):
         with compiled_autograd._enable(lambda graph: graph):
             loss.backward()
         assert same([t.grad for t in leaves], plain_grads(name))
+
+
+OPERATORS = {"softmax": "softmax_fwd", "swiglu": "swiglu_fwd", "norm": "norm_fwd", "add_norm": "add_norm_fwd", "attention": "attn_fwd",
+             "attention_packed": "attn_fwd"}
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+def test_torch_function_modes_see_the_operators(name):
+    seen = []
+
+    class Mode(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    fn, leaves, constants = case(name)
+    with Mode():
+        out = fn(*leaves, *constants)
+    assert f"algebraic.{OPERATORS[name]}" in seen
+    loss_of(out).backward()
+    assert same([t.grad for t in leaves], plain_grads(name))
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+def test_torch_function_of_a_subclass_is_asked(name):
+    seen = []
+
+    class Marked(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", str(func)))
+            return super().__torch_function__(func, types, args, kwargs or {})
+
+    fn, leaves, constants = case(name)
+    out = fn(*[t.detach().as_subclass(Marked) for t in leaves], *constants)
+    assert OPERATORS[name] in seen
+    assert type(out[0] if isinstance(out, tuple) else out) is Marked
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+@pytest.mark.parametrize("transform", ["vmap", "grad"])
+def test_functorch_transforms_stay_refused(name, transform):
+    """The operators have no functorch rules; a call under a transform raises, as their autograd Functions always did."""
+    fn, leaves, constants = case(name)
+    args = [t.detach() for t in leaves]
+    with pytest.raises(RuntimeError, match="functorch"):
+        if transform == "vmap":
+            torch.vmap(lambda x: loss_of(fn(x, *args[1:], *constants)))(torch.stack([args[0]] * 2))
+        else:
+            torch.func.grad(lambda x: loss_of(fn(x, *args[1:], *constants)))(args[0])
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+def test_forward_mode_is_refused(name):
+    import torch.autograd.forward_ad as forward_ad
+    fn, leaves, constants = case(name)
+    with forward_ad.dual_level(), pytest.raises(NotImplementedError):
+        fn(forward_ad.make_dual(leaves[0], torch.ones_like(leaves[0])), *leaves[1:], *constants)
