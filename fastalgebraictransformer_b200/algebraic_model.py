@@ -22,7 +22,7 @@ from torch.utils.checkpoint import checkpoint
 from . import _lib, ops
 from .backward import rational_attention_packed
 from .forward import compute_alibi_slopes
-from .fused_ops import (EPS, add_mean_error_norm, head_shifted_cross_entropy, mean_error_norm, rational_swiglu,
+from .fused_ops import (EPS, RationalSwiGLUPacked, add_mean_error_norm, head_shifted_cross_entropy, mean_error_norm, rational_swiglu,
                         shifted_cross_entropy)
 
 
@@ -51,7 +51,9 @@ class RationalSwiGLU(nn.Module):
         gv = self.w_gate_val(x)
         if not gv.is_cuda:
             raise RuntimeError("RationalSwiGLU: CUDA tensor required — this build has no CPU fallback")
-        return self.dropout(self.w_out(rational_swiglu(*gv.chunk(2, dim=-1))))
+        # (a tracer does not see that the halves belong together: it is given the Function with one packed gradient)
+        act = RationalSwiGLUPacked.apply(gv) if torch.compiler.is_compiling() else rational_swiglu(*gv.chunk(2, dim=-1))
+        return self.dropout(self.w_out(act))
 
 
 class KVCache:

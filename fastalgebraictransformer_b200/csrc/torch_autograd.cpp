@@ -198,7 +198,7 @@ struct RationalSwiGLUBackward : OperatorNode<RationalSwiGLUBackward> {
     variable_list out(num_outputs());
     if (!grads[0].defined()) return out;
     const Tensor g = gate.unpack(), v = value.unpack();
-    const bool to_packed = halves && !traced && !at::GradMode::is_enabled() && task_should_compute_output(2) &&
+    const bool to_packed = halves && !traced && task_should_compute_output(2) &&
                            !watched(next_edge(0).function.get()) && !watched(next_edge(1).function.get());
     BackwardScope scope;
     if (to_packed) {

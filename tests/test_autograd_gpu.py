@@ -129,3 +129,35 @@ def test_forward_mode_is_refused(name):
     fn, leaves, constants = case(name)
     with forward_ad.dual_level(), pytest.raises(NotImplementedError):
         fn(forward_ad.make_dual(leaves[0], torch.ones_like(leaves[0])), *leaves[1:], *constants)
+
+
+def test_a_graph_of_gradients_keeps_the_packed_gradient():
+    """create_graph: the halves' projection still gets one packed gradient, not a concatenation (the profiler's view of it)."""
+    x = torch.randn(64, 512, device=DEV, requires_grad=True)
+    results = []
+    for create in (False, True):
+        out = fat().rational_swiglu(*x.chunk(2, -1))
+        with torch.profiler.profile() as prof:
+            results.append(torch.autograd.grad(out, x, torch.ones_like(out), create_graph=create)[0].detach())
+        names = {e.name for e in prof.events()}
+        assert "algebraic::swiglu_bwd_packed" in names and "aten::cat" not in names, create
+    assert torch.equal(*results)
+
+
+def test_a_traced_feed_forward_block_keeps_the_packed_gradient():
+    """torch.compile of the block: the traced backward holds the packed operator and no concatenation; same gradients."""
+    from torch._dynamo.backends.common import aot_autograd
+    graphs = []
+
+    def keep(graph, inputs):
+        graphs.append({str(n.target) for n in graph.graph.nodes})
+        return graph.forward
+
+    torch.manual_seed(8)
+    block = fat().algebraic_model.RationalSwiGLU(64, 96).to(DEV)
+    x = torch.randn(2, 17, 64, device=DEV, requires_grad=True)
+    want = torch.autograd.grad(block(x).sum(), [x, *block.parameters()])
+    got = torch.autograd.grad(torch.compile(block, backend=aot_autograd(fw_compiler=keep, bw_compiler=keep))(x).sum(), [x, *block.parameters()])
+    assert same(got, want)
+    names = set().union(*graphs)
+    assert any("swiglu_bwd_packed" in n for n in names) and not any("aten.cat" in n for n in names)
