@@ -270,12 +270,12 @@ struct RationalAttentionBackward : OperatorNode<RationalAttentionBackward> {
   std::string name() const override { return "RationalAttentionBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    if (!grads[0].defined() || !(should_compute_output(0) || should_compute_output(1) || should_compute_output(2))) return {Tensor(), Tensor(), Tensor(), Tensor()};
     const Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = out.unpack(shared_from_this()), Lt = L.unpack(), lt = lo.unpack(),
                  st = slopes.unpack(), bt = bits.unpack();
     BackwardScope scope;
     auto [dq, dk, dv] = op_attn_bwd(qt, kt, vt, ot, lt, Lt, grads[0], st, scale, causal, eps, bt.defined() ? optional<Tensor>(bt) : optional<Tensor>());
-    return {dq, dk, dv};
+    return {dq, dk, dv, Tensor()};                      // (the slopes have an edge and no gradient)
   }
 };
 
@@ -286,10 +286,10 @@ struct RationalAttentionPackedBackward : OperatorNode<RationalAttentionPackedBac
   std::string name() const override { return "RationalAttentionPackedBackward"; }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    if (!grads[0].defined()) return {Tensor()};
+    if (!grads[0].defined() || !should_compute_output(0)) return {Tensor(), Tensor()};
     const Tensor pt = qkv.unpack(), ot = out.unpack(shared_from_this()), Lt = L.unpack(), lt = lo.unpack(), st = slopes.unpack(), bt = bits.unpack();
     BackwardScope scope;
-    return {op_attn_bwd_packed(pt, ot, lt, Lt, grads[0], st, scale, eps, bt.defined() ? optional<Tensor>(bt) : optional<Tensor>())};
+    return {op_attn_bwd_packed(pt, ot, lt, Lt, grads[0], st, scale, eps, bt.defined() ? optional<Tensor>(bt) : optional<Tensor>()), Tensor()};
   }
 };
 
@@ -377,10 +377,10 @@ optional<Tensor> bits_of(const optional<Tensor>& key_mask, int64_t mask_tokens, 
 
 Tensor attention_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& slopes, double scale, bool causal, double eps,
                           const optional<Tensor>& key_mask, int64_t mask_tokens) {
-  no_forward_mode("rational_attention", q, k, v);
+  no_forward_mode("rational_attention", q, k, v, slopes);
   std::shared_ptr<RationalAttentionBackward> node;
-  if (compute_requires_grad(q, k, v)) {
-    node = new_node<RationalAttentionBackward>(q, k, v);
+  if (compute_requires_grad(q, k, v, slopes)) {
+    node = new_node<RationalAttentionBackward>(q, k, v, slopes);
     node->q = SavedVariable(q, false);
     node->k = SavedVariable(k, false);
     node->v = SavedVariable(v, false);
@@ -394,7 +394,7 @@ Tensor attention_autograd(const Tensor& q, const Tensor& k, const Tensor& v, con
   {
     BelowAutograd guard;
     bits = bits_of(key_mask, mask_tokens, q.size(2));
-    std::tie(out, L, lo) = op_attn_fwd(q, k, v, slopes, scale, causal, eps, bits, bool(node));
+    std::tie(out, L, lo) = op_attn_fwd(q, k, v, slopes, scale, causal, eps, bits, node && compute_requires_grad(q, k, v));
   }
   if (node) {
     set_history(out, node);
@@ -408,10 +408,10 @@ Tensor attention_autograd(const Tensor& q, const Tensor& k, const Tensor& v, con
 
 Tensor attention_packed_autograd(const Tensor& qkv, const Tensor& slopes, double scale, double eps, const optional<Tensor>& key_mask,
                                  int64_t mask_tokens) {
-  no_forward_mode("rational_attention_packed", qkv);
+  no_forward_mode("rational_attention_packed", qkv, slopes);
   std::shared_ptr<RationalAttentionPackedBackward> node;
-  if (compute_requires_grad(qkv)) {
-    node = new_node<RationalAttentionPackedBackward>(qkv);
+  if (compute_requires_grad(qkv, slopes)) {
+    node = new_node<RationalAttentionPackedBackward>(qkv, slopes);
     node->qkv = SavedVariable(qkv, false);
     node->slopes = SavedVariable(slopes, false);
     node->scale = scale;
@@ -422,7 +422,7 @@ Tensor attention_packed_autograd(const Tensor& qkv, const Tensor& slopes, double
   {
     BelowAutograd guard;
     bits = bits_of(key_mask, mask_tokens, qkv.size(1));
-    std::tie(out, L, lo) = op_attn_fwd_packed(qkv, slopes, scale, eps, bits, bool(node));
+    std::tie(out, L, lo) = op_attn_fwd_packed(qkv, slopes, scale, eps, bits, node && compute_requires_grad(qkv));
     tokens = out.permute({0, 2, 1, 3}).reshape({qkv.size(0), qkv.size(1), qkv.size(3) * qkv.size(4)});     // a view: the memory order is [B,T,H,D]
   }
   if (node) {

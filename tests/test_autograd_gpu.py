@@ -161,3 +161,17 @@ def test_a_traced_feed_forward_block_keeps_the_packed_gradient():
     assert same(got, want)
     names = set().union(*graphs)
     assert any("swiglu_bwd_packed" in n for n in names) and not any("aten.cat" in n for n in names)
+
+
+@pytest.mark.parametrize("name", ["attention", "attention_packed"])
+@pytest.mark.parametrize("inputs", [False, True])
+def test_slopes_that_ask_for_a_gradient(name, inputs):
+    """They have none (the operator's slopes are constants), but the result belongs to their graph, as with the Functions."""
+    fn, leaves, (slopes,) = case(name)
+    slopes.requires_grad_(True)
+    leaves = [t.requires_grad_(inputs) for t in (x.detach() for x in leaves)]
+    out = fn(*leaves, slopes)
+    assert out.requires_grad
+    loss_of(out).backward()
+    assert slopes.grad is None
+    assert same([t.grad for t in leaves], plain_grads(name) if inputs else [None] * len(leaves))
