@@ -126,7 +126,7 @@ class ShiftedCrossEntropy(torch.autograd.Function):
         assert logits.is_cuda, "Input must be on CUDA"
         loss, d_logits = _alg.shifted_ce_fwd(logits, labels, ignore_index)
         ctx.save_for_backward(d_logits)
-        return loss.to(logits.dtype)
+        return loss.to(logits.dtype, copy=_compiling())      # (a tracer gives the gradient of one tensor under two names to the wrong one)
 
     @staticmethod
     def backward(ctx, grad_loss):
@@ -154,7 +154,7 @@ class HeadShiftedCrossEntropy(torch.autograd.Function):
         loss, d_y, d_w = ops.head_shifted_ce(y, weight, labels, ignore_index, want_grads=want)
         if want:
             ctx.save_for_backward(d_y, d_w)
-        return loss.to(y.dtype)
+        return loss.to(y.dtype, copy=_compiling())
 
     @staticmethod
     def backward(ctx, grad_loss):

@@ -175,3 +175,26 @@ def test_slopes_that_ask_for_a_gradient(name, inputs):
     loss_of(out).backward()
     assert slopes.grad is None
     assert same([t.grad for t in leaves], plain_grads(name) if inputs else [None] * len(leaves))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head", [False, True])
+def test_traced_loss_has_the_eager_gradients(head, dtype):
+    """torch.compile of the loss: its gradients are formed in the forward and scaled in the backward, in place when it is eager."""
+    g = torch.Generator().manual_seed(9)
+    x, w = torch.randn(2, 17, 64, generator=g).to(dtype).to(DEV), torch.randn(40, 64, generator=g).to(dtype).to(DEV)
+    labels = torch.randint(0, 40, (2, 17), generator=g).to(DEV)
+
+    def loss(x, w):
+        out = fat().head_shifted_cross_entropy(x, w, labels, -100) if head else fat().shifted_cross_entropy(x, labels, -100)
+        return out * 3.0
+
+    results = []
+    for fn in (loss, torch.compile(loss, backend="aot_eager")):
+        leaves = [x.clone().requires_grad_(True), w.clone().requires_grad_(True)]
+        fn(*leaves).backward()
+        results.append([t.grad for t in leaves])
+    assert (results[0][1] is not None) == head
+    # eager: one product with 3 in float32, rounded; traced: the same product
+    for got, want in zip(*results[::-1]):
+        assert (got is None and want is None) or torch.allclose(got, want, rtol=2.0 ** -7 if dtype == torch.bfloat16 else 1e-6, atol=0)
