@@ -5,24 +5,29 @@
 // What bounds it: the FMA pipe, as long as shared memory, issue slots and latencies keep up.  A CTA owns kOwn = 32 queries
 // (forward, d_q) or keys (d_k/d_v) and streams tiles of kStream = 64 rows of the other side.  Short own tiles, handed out
 // longest first over all heads, because small problems have few of them: 2x12 heads of 512 tokens are 384 CTAs of 1-8 steps;
-// 64-row tiles left 192 for 148 SMs and twice the longest one's time.  128 threads; a warp covers 16 x 32 scores, a thread
+// 64-row tiles left 192 for 148 SMs and twice the longest one's time.  (The backward of heads beyond 64, whose tiles leave an SM one
+// CTA of four warps, takes 64 own rows where a launch has enough of them: long_tiles.)  Four threads per own row; a warp covers 16 x 32 scores, a thread
 // 4 x 4 (rows 4 apart, columns 8 apart), so that no shared load has bank conflicts.  FMAs are issued as float32 pairs
 // (fma.rn.f32x2: same pipe time, half the issue slots): along the head dimension in the score products, along the output
 // columns in the others, whose weights lie doubled (w, w) in shared memory so that no register moves build the pairs.
-// float32 tiles arrive by cp.async, each while a contraction that does not need its buffer runs.
+// float32 tiles arrive by cp.async, each while a contraction that does not need its buffer runs; rows that cannot be moved in
+// 16-byte pieces have kernels of their own (VEC), with eight element loads in flight (D = 70, 4x16x512, forward + backward: 1647 ->
+// 852 us with the longer tiles; D = 30: 361 -> 290) and none of that code in the others.
 // 2x12 heads, 512 tokens, D = 64, float32: forward 97 -> 57 us, d_q 133 -> 79 us, d_k/d_v 152 -> 78 us (64-row tiles of 256
 // threads with synchronous loads before); eight steps of the contractions unrolled instead of four and the wider pitch of the
-// doubled weights bring forward + backward from 201 to 193 us (sixteen steps: 199, two: 208).  With four steps: FMA pipe 40-45 % busy on an active SM at 8 warps per SM (before: 15-20 %): latency of
-// the shared loads, and an SM's share of the CTAs (71 % of the longest SM's time on average).
+// doubled weights bring forward + backward from 201 to 193 us (sixteen steps: 199, two: 208).  With four steps: FMA pipe 40-45 % busy on an
+// active SM at 8 warps per SM (before: 15-20 %): latency of the shared loads, and an SM's share of the CTAs (71 % of the longest SM's time on average).
 // Backward is two kernels without atomics: a query-major one (Delta, d_q) and a key-major one (d_k, d_v), each
 // recomputing the scores it needs.  No running maximum anywhere (sigma^4 <= 1).
+#include <algorithm>
+
 #include "attn_common.cuh"
 
 namespace fat {
 namespace {
 
-constexpr int kOwn = 32, kStream = 64, NT = 128;
-constexpr int kPairLd = 2 * kStream + 16;       // pitch of the doubled weights [kOwn][kStream] in floats: neighbouring rows half the banks apart
+constexpr int kOwn = 32, kStream = 64;           // (the backward also has tiles of 64 own rows: OWN)
+constexpr int kPairLd = 2 * kStream + 16;       // pitch of the doubled weights [OWN][kStream] in floats: neighbouring rows half the banks apart
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ void upk2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
@@ -38,20 +43,21 @@ struct Lane {
 
 // The CTA's tile: the grid runs over (tile, batch, head) with the tile slowest, whatever the caller wants first.
 struct Tile { int b, h, tile; };
+template <int OWN>
 __device__ __forceinline__ Tile this_tile(const AttnParams& p) {
-  const int tiles = (p.T + kOwn - 1) / kOwn, group = gridDim.x / tiles;         // H * B, or H with the batch on the y axis
+  const int tiles = (p.T + OWN - 1) / OWN, group = gridDim.x / tiles;         // H * B, or H with the batch on the y axis
   const int bh = blockIdx.y * group + blockIdx.x % group;
   return Tile{bh / p.H, bh % p.H, int(blockIdx.x) / group};
 }
 
 // dst[ROWS][DP + 4] = rows row0.. of base as float, zeros beyond T_len and D.  float32 rows that can be moved in 16-byte
 // pieces are copied asynchronously (the caller waits with copies_done), everything else is there on return.
-template <typename T, int DP, int ROWS>
+template <typename T, int DP, int ROWS, int NT, bool VEC>
 __device__ __forceinline__ void load_tile(float* __restrict__ dst, const T* __restrict__ base,
-                                          int64_t row_stride, int row0, int T_len, int D, bool vec) {
+                                          int64_t row_stride, int row0, int T_len, int D) {
   constexpr int LD = DP + 4;
   constexpr int W = 16 / sizeof(T);
-  if (vec) {
+  if constexpr (VEC) {
     constexpr int PPR = DP / W;
     if constexpr (sizeof(T) == 4) {
       const uint32_t s0 = uint32_t(__cvta_generic_to_shared(dst));
@@ -79,6 +85,7 @@ __device__ __forceinline__ void load_tile(float* __restrict__ dst, const T* __re
       }
     }
   } else {
+#pragma unroll 8
     for (int idx = threadIdx.x; idx < ROWS * DP; idx += NT) {
       const int r = idx / DP, c = idx % DP, row = row0 + r;
       dst[r * LD + c] = (row < T_len && c < D) ? Elem<T>::to_c(base[int64_t(row) * row_stride + c]) : 0.f;
@@ -89,7 +96,7 @@ __device__ __forceinline__ void load_tile(float* __restrict__ dst, const T* __re
 __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void copies_visible() { copies_done(); __syncthreads(); }
 
-// s[i][j] = sum_d A[row(i)][d] * Bm[col(j)][d]     (A is [kOwn][DP+4], Bm is [kStream][DP+4])
+// s[i][j] = sum_d A[row(i)][d] * Bm[col(j)][d]     (A is [own][DP+4], Bm is [kStream][DP+4])
 template <int DP>
 __device__ __forceinline__ void gemm_nt(float (&s)[4][4], const float* __restrict__ A, const float* __restrict__ Bm, const Lane& ln) {
   constexpr int LD = DP + 4;
@@ -126,7 +133,7 @@ __device__ __forceinline__ void gemm_nt(float (&s)[4][4], const float* __restric
     }
 }
 
-// Columns of the [kOwn][DP] outputs: a warp has one half of them, a lane VW neighbours in each of NCH chunks.
+// Columns of the [own][DP] outputs: a warp has one half of them, a lane VW neighbours in each of NCH chunks.
 template <int DP> struct OutCols {
   static constexpr int VW = DP >= 64 ? 4 : 2;
   static constexpr int NCH = DP / 16 / VW;
@@ -215,13 +222,13 @@ __device__ __forceinline__ Score score_terms(float qk, float scale, float slope,
 }
 
 // ------------------------------------------------------------------ forward
-template <typename T, int DP>
-__global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_fwd_simt_kernel(AttnParams p, bool vec) {
+template <typename T, int DP, bool VEC>
+__global__ void __launch_bounds__(4 * kOwn, DP > 64 ? 2 : 3) attn_fwd_simt_kernel(AttnParams p) {
   extern __shared__ __align__(16) float smem[];
-  constexpr int LD = DP + 4;
+  constexpr int LD = DP + 4, NT = 4 * kOwn;
   float* Qs = smem; float* Ks = Qs + kOwn * LD; float* Vs = Ks + kStream * LD; float* Ps = Vs + kStream * LD;
   const Lane ln;
-  const Tile tl = this_tile(p);
+  const Tile tl = this_tile<kOwn>(p);
   const int b = tl.b, h = tl.h, n_tiles = (p.T + kOwn - 1) / kOwn;
   const int q0 = (n_tiles - 1 - tl.tile) * kOwn;                               // long rows first
   const T* qb = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
@@ -230,8 +237,8 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_fwd_simt_kernel(Attn
   T* ob = static_cast<T*>(p.out) + b * p.os[0] + h * p.os[1];
   const float slope = p.slopes[h];
 
-  load_tile<T, DP, kOwn>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
-  load_tile<T, DP, kStream>(Ks, kb, p.ks[2], 0, p.T, p.D, vec);
+  load_tile<T, DP, kOwn, NT, VEC>(Qs, qb, p.qs[2], q0, p.T, p.D);
+  load_tile<T, DP, kStream, NT, VEC>(Ks, kb, p.ks[2], 0, p.T, p.D);
   Out<DP> o;
   clear(o);
   float l[4] = {0.f, 0.f, 0.f, 0.f};
@@ -239,7 +246,7 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_fwd_simt_kernel(Attn
 #pragma unroll 1
   for (int k0 = 0; k0 < k_end; k0 += kStream) {
     copies_visible();                                                          // K is there, V and the weights are free
-    load_tile<T, DP, kStream>(Vs, vb, p.vs[2], k0, p.T, p.D, vec);
+    load_tile<T, DP, kStream, NT, VEC>(Vs, vb, p.vs[2], k0, p.T, p.D);
     float s[4][4];
     gemm_nt<DP>(s, Qs, Ks, ln);
 #pragma unroll
@@ -256,7 +263,7 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_fwd_simt_kernel(Attn
       }
     }
     copies_visible();                                                          // V is there, K is free
-    if (k0 + kStream < k_end) load_tile<T, DP, kStream>(Ks, kb, p.ks[2], k0 + kStream, p.T, p.D, vec);
+    if (k0 + kStream < k_end) load_tile<T, DP, kStream, NT, VEC>(Ks, kb, p.ks[2], k0 + kStream, p.T, p.D);
     gemm_nn<DP>(o, Ps, Vs, ln);
   }
   // a row's sum: over the eight lanes that share it, then over the two warps
@@ -281,17 +288,17 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_fwd_simt_kernel(Attn
 }
 
 // ------------------------------------------------------------------ backward, query-major: Delta and d_q
-template <typename T, int DP>
-__global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_bwd_dq_simt_kernel(AttnParams p, bool vec) {
+template <typename T, int DP, bool VEC, int OWN>
+__global__ void __launch_bounds__(4 * OWN, OWN > 32 ? 1 : DP > 64 ? 2 : 3) attn_bwd_dq_simt_kernel(AttnParams p) {
   extern __shared__ __align__(16) float smem[];
-  constexpr int LD = DP + 4;
-  float* Qs = smem; float* dOs = Qs + kOwn * LD; float* Ks = dOs + kOwn * LD; float* Vs = Ks + kStream * LD;
-  float* dSs = Vs + kStream * LD; float* rowInv = dSs + kOwn * kPairLd; float* rowD = rowInv + kOwn;
+  constexpr int LD = DP + 4, NT = 4 * OWN;
+  float* Qs = smem; float* dOs = Qs + OWN * LD; float* Ks = dOs + OWN * LD; float* Vs = Ks + kStream * LD;
+  float* dSs = Vs + kStream * LD; float* rowInv = dSs + OWN * kPairLd; float* rowD = rowInv + OWN;
   const Lane ln;
-  const Tile tl = this_tile(p);
-  const int b = tl.b, h = tl.h, n_tiles = (p.T + kOwn - 1) / kOwn;
+  const Tile tl = this_tile<OWN>(p);
+  const int b = tl.b, h = tl.h, n_tiles = (p.T + OWN - 1) / OWN;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = (n_tiles - 1 - tl.tile) * kOwn;
+  const int q0 = (n_tiles - 1 - tl.tile) * OWN;
   const T* qb = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const T* kb = static_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* vb = static_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
@@ -302,10 +309,10 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_bwd_dq_simt_kernel(A
   const int64_t stat0 = (int64_t(b) * p.H + h) * p.T;
   const float slope = p.slopes[h];
 
-  load_tile<T, DP, kOwn>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
-  load_tile<T, DP, kOwn>(dOs, dob, p.dos[2], q0, p.T, p.D, vec);
-  load_tile<T, DP, kStream>(Ks, kb, p.ks[2], 0, p.T, p.D, vec);
-  load_tile<T, DP, kStream>(Vs, vb, p.vs[2], 0, p.T, p.D, vec);
+  load_tile<T, DP, OWN, NT, VEC>(Qs, qb, p.qs[2], q0, p.T, p.D);
+  load_tile<T, DP, OWN, NT, VEC>(dOs, dob, p.dos[2], q0, p.T, p.D);
+  load_tile<T, DP, kStream, NT, VEC>(Ks, kb, p.ks[2], 0, p.T, p.D);
+  load_tile<T, DP, kStream, NT, VEC>(Vs, vb, p.vs[2], 0, p.T, p.D);
 #pragma unroll 2
   for (int r = warp * 8; r < warp * 8 + 8; ++r) {                              // Delta = d_out . (out + its rounding residual)
     const int row = q0 + r;
@@ -329,7 +336,7 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_bwd_dq_simt_kernel(A
 
   Out<DP> dq;
   clear(dq);
-  const int k_end = p.causal ? min(p.T, q0 + kOwn) : p.T;
+  const int k_end = p.causal ? min(p.T, q0 + OWN) : p.T;
 #pragma unroll 1
   for (int k0 = 0; k0 < k_end; k0 += kStream) {
     copies_visible();
@@ -349,10 +356,10 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_bwd_dq_simt_kernel(A
     }
     __syncthreads();                                                           // dS is there, V is free
     const bool more = k0 + kStream < k_end;
-    if (more) load_tile<T, DP, kStream>(Vs, vb, p.vs[2], k0 + kStream, p.T, p.D, vec);
+    if (more) load_tile<T, DP, kStream, NT, VEC>(Vs, vb, p.vs[2], k0 + kStream, p.T, p.D);
     gemm_nn<DP>(dq, dSs, Ks, ln);
     __syncthreads();                                                           // K and dS are free
-    if (more) load_tile<T, DP, kStream>(Ks, kb, p.ks[2], k0 + kStream, p.T, p.D, vec);
+    if (more) load_tile<T, DP, kStream, NT, VEC>(Ks, kb, p.ks[2], k0 + kStream, p.T, p.D);
   }
   copies_done();
   const float mul[4] = {p.scale, p.scale, p.scale, p.scale};
@@ -360,15 +367,15 @@ __global__ void __launch_bounds__(NT, DP > 64 ? 2 : 3) attn_bwd_dq_simt_kernel(A
 }
 
 // ------------------------------------------------------------------ backward, key-major: d_k and d_v
-template <typename T, int DP>
-__global__ void __launch_bounds__(NT, 2) attn_bwd_dkv_simt_kernel(AttnParams p, bool vec) {
+template <typename T, int DP, bool VEC, int OWN>
+__global__ void __launch_bounds__(4 * OWN, OWN > 32 ? 1 : 2) attn_bwd_dkv_simt_kernel(AttnParams p) {
   extern __shared__ __align__(16) float smem[];
-  constexpr int LD = DP + 4;
-  float* Ks = smem; float* Vs = Ks + kOwn * LD; float* Qs = Vs + kOwn * LD; float* dOs = Qs + kStream * LD;
-  float* PsT = dOs + kStream * LD; float* dSsT = PsT + kOwn * kPairLd;
+  constexpr int LD = DP + 4, NT = 4 * OWN;
+  float* Ks = smem; float* Vs = Ks + OWN * LD; float* Qs = Vs + OWN * LD; float* dOs = Qs + kStream * LD;
+  float* PsT = dOs + kStream * LD; float* dSsT = PsT + OWN * kPairLd;
   const Lane ln;
-  const Tile tl = this_tile(p);                                                // early key tiles are the long ones
-  const int b = tl.b, h = tl.h, k0 = tl.tile * kOwn;
+  const Tile tl = this_tile<OWN>(p);                                                // early key tiles are the long ones
+  const int b = tl.b, h = tl.h, k0 = tl.tile * OWN;
   const T* qb = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const T* kb = static_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* vb = static_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
@@ -379,10 +386,10 @@ __global__ void __launch_bounds__(NT, 2) attn_bwd_dkv_simt_kernel(AttnParams p, 
   const float slope = p.slopes[h];
 
   int q0 = p.causal ? k0 / kStream * kStream : 0;
-  load_tile<T, DP, kOwn>(Ks, kb, p.ks[2], k0, p.T, p.D, vec);
-  load_tile<T, DP, kOwn>(Vs, vb, p.vs[2], k0, p.T, p.D, vec);
-  load_tile<T, DP, kStream>(Qs, qb, p.qs[2], q0, p.T, p.D, vec);
-  load_tile<T, DP, kStream>(dOs, dob, p.dos[2], q0, p.T, p.D, vec);
+  load_tile<T, DP, OWN, NT, VEC>(Ks, kb, p.ks[2], k0, p.T, p.D);
+  load_tile<T, DP, OWN, NT, VEC>(Vs, vb, p.vs[2], k0, p.T, p.D);
+  load_tile<T, DP, kStream, NT, VEC>(Qs, qb, p.qs[2], q0, p.T, p.D);
+  load_tile<T, DP, kStream, NT, VEC>(dOs, dob, p.dos[2], q0, p.T, p.D);
   bool kept[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -422,10 +429,10 @@ __global__ void __launch_bounds__(NT, 2) attn_bwd_dkv_simt_kernel(AttnParams p, 
     gemm_nn<DP>(dv, PsT, dOs, ln);
     __syncthreads();                                                           // dO is free
     const bool more = q0 + kStream < p.T;
-    if (more) load_tile<T, DP, kStream>(dOs, dob, p.dos[2], q0 + kStream, p.T, p.D, vec);
+    if (more) load_tile<T, DP, kStream, NT, VEC>(dOs, dob, p.dos[2], q0 + kStream, p.T, p.D);
     gemm_nn<DP>(dk, dSsT, Qs, ln);
     __syncthreads();                                                           // Q and the weights are free
-    if (more) load_tile<T, DP, kStream>(Qs, qb, p.qs[2], q0 + kStream, p.T, p.D, vec);
+    if (more) load_tile<T, DP, kStream, NT, VEC>(Qs, qb, p.qs[2], q0 + kStream, p.T, p.D);
   }
   copies_done();
   const float one[4] = {1.f, 1.f, 1.f, 1.f};
@@ -446,37 +453,60 @@ bool tiles_vectorisable(const AttnParams& p, bool bwd) {
   return v;
 }
 
-template <typename Kern>
-int launch(Kern kern, const AttnParams& p, bool vec, size_t smem, cudaStream_t st, const char* what) {
+template <int OWN, typename Kern>
+int launch(Kern kern, const AttnParams& p, size_t smem, cudaStream_t st, const char* what) {
   if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, what)) return rc;
-  const int64_t column = int64_t((p.T + kOwn - 1) / kOwn) * p.H;
+  const int64_t column = int64_t((p.T + OWN - 1) / OWN) * p.H;
   const bool flat = column * p.B < (int64_t(1) << 31);                          // (otherwise the longest go first within a batch element)
   const dim3 grid(unsigned(flat ? column * p.B : column), unsigned(flat ? 1 : p.B));
-  kern<<<grid, NT, smem, st>>>(p, vec);
+  kern<<<grid, 4 * OWN, smem, st>>>(p);
   return check_launch(what);
 }
 
-template <typename T, int DP>
+// Whether the backward takes tiles of 64 own rows (256 threads) instead of 32.  From D = 65 on the tiles of either size leave room for
+// one CTA per SM, and 32 rows are four warps: half the streamed rows per own row and twice the warps make a 64-row tile cost 1.5
+// times a 32-row one, so it pays where a launch has enough tiles to keep every SM busy (waves of equal tiles, or the longest
+// tile against an SM's share where the tiles are triangular).  D = 128 float32 backward, us, 32 / 64 rows: 4x16x512 741 / 582,
+// 16x24x128 563 / 409, 2x8x512 175 / 251; not causal: 2x8x512 317 / 251, 2x12x512 468 / 493, 4x16x777 2800 / 2405.  D <= 64 has room for
+// two to three CTAs of 32 rows, which always win (4x16x512, D = 64: 291 / 331); so they do in the forward (D = 128: 154 / 159).
+bool long_tiles(const AttnParams& p) {
+  const int64_t n = int64_t((p.T + 63) / 64) * p.B * p.H, sms = num_sms();
+  auto waves = [&](int64_t tiles) { return p.causal ? std::max(1.0, 0.5 * double(tiles) / double(sms)) : double((tiles + sms - 1) / sms); };
+  return 1.5 * waves(n) < waves(2 * n);
+}
+
+template <typename T, int DP, bool VEC>
 int fwd_t(const AttnParams& p, cudaStream_t st) {
   constexpr size_t smem = (size_t(kOwn + 2 * kStream) * (DP + 4) + kOwn * kPairLd) * sizeof(float);
-  return launch(attn_fwd_simt_kernel<T, DP>, p, tiles_vectorisable<T>(p, false), smem, st, "attn_fwd_simt");
+  return launch<kOwn>(attn_fwd_simt_kernel<T, DP, VEC>, p, smem, st, "attn_fwd_simt");
+}
+
+template <typename T, int DP, bool VEC, int OWN>
+int bwd_own(const AttnParams& p, cudaStream_t st) {
+  constexpr size_t tiles = size_t(2) * (OWN + kStream) * (DP + 4);
+  constexpr size_t smem_dq = (tiles + OWN * kPairLd + 2 * OWN) * sizeof(float);
+  constexpr size_t smem_dkv = (tiles + 2 * OWN * kPairLd) * sizeof(float);
+  if (int rc = launch<OWN>(attn_bwd_dq_simt_kernel<T, DP, VEC, OWN>, p, smem_dq, st, "attn_bwd_dq_simt")) return rc;
+  return launch<OWN>(attn_bwd_dkv_simt_kernel<T, DP, VEC, OWN>, p, smem_dkv, st, "attn_bwd_dkv_simt");
+}
+template <typename T, int DP, bool VEC>
+int bwd_t(const AttnParams& p, cudaStream_t st) {
+  if constexpr (DP > 64)
+    if (long_tiles(p)) return bwd_own<T, DP, VEC, 64>(p, st);
+  return bwd_own<T, DP, VEC, kOwn>(p, st);
 }
 
 template <typename T, int DP>
-int bwd_t(const AttnParams& p, cudaStream_t st) {
-  const bool vec = tiles_vectorisable<T>(p, true);
-  constexpr size_t tiles = size_t(2) * (kOwn + kStream) * (DP + 4);
-  constexpr size_t smem_dq = (tiles + kOwn * kPairLd + 2 * kOwn) * sizeof(float);
-  constexpr size_t smem_dkv = (tiles + 2 * kOwn * kPairLd) * sizeof(float);
-  if (int rc = launch(attn_bwd_dq_simt_kernel<T, DP>, p, vec, smem_dq, st, "attn_bwd_dq_simt")) return rc;
-  return launch(attn_bwd_dkv_simt_kernel<T, DP>, p, vec, smem_dkv, st, "attn_bwd_dkv_simt");
+int dispatch_vec(const AttnParams& p, bool bwd, cudaStream_t st) {
+  if (tiles_vectorisable<T>(p, bwd)) return bwd ? bwd_t<T, DP, true>(p, st) : fwd_t<T, DP, true>(p, st);
+  return bwd ? bwd_t<T, DP, false>(p, st) : fwd_t<T, DP, false>(p, st);
 }
 
 template <typename T>
 int dispatch_d(const AttnParams& p, bool bwd, cudaStream_t st) {
-  if (p.D <= 32) return bwd ? bwd_t<T, 32>(p, st) : fwd_t<T, 32>(p, st);
-  if (p.D <= 64) return bwd ? bwd_t<T, 64>(p, st) : fwd_t<T, 64>(p, st);
-  if (p.D <= 128) return bwd ? bwd_t<T, 128>(p, st) : fwd_t<T, 128>(p, st);
+  if (p.D <= 32) return dispatch_vec<T, 32>(p, bwd, st);
+  if (p.D <= 64) return dispatch_vec<T, 64>(p, bwd, st);
+  if (p.D <= 128) return dispatch_vec<T, 128>(p, bwd, st);
   set_error("attention: head size %d is not supported (D <= 128)", p.D);
   return FAT_ERR_UNSUPPORTED;
 }

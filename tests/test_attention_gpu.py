@@ -76,6 +76,31 @@ def test_cuda_core_tile_edges(T, D, causal):
         assert norm_max_err(g, w) < FP32_TOL, f"{name}: {norm_max_err(g, w):.2e}"
 
 
+# 112 (batch, head) pairs: enough tiles for the backward's 64-row own tiles beyond D = 64 (128 and more tokens, or 64 and more when
+# not causal; 40 tokens stay on 32-row tiles).  One row short of, at and beyond the tile edges; D = 70 and 66 take element-wise copies
+@pytest.mark.parametrize("T", [40, 63, 64, 65, 127, 128, 129])
+@pytest.mark.parametrize("D,causal,dtype", [(128, True, torch.float32), (128, False, torch.float32), (100, True, torch.float32), (70, False, torch.float32),
+                                            (66, True, torch.float32), (128, True, torch.bfloat16), (72, False, torch.float16)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_cuda_core_long_tiles(T, D, causal, dtype, masked):
+    B, H = 8, 14
+    q, k, v, go = gen_qkv(31, B, H, T, D, dtype)
+    slopes = oracle.compute_alibi_slopes(H)
+    keep = (torch.arange(T)[None] < torch.tensor([[T - 3 * i] for i in range(B)])).to(torch.int64) if masked else None
+    from fastalgebraictransformer_b200.backward import RationalAttentionFunction
+    leaves = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]
+    out = RationalAttentionFunction.apply(*leaves, slopes.to(DEV), 0.2, causal, 1e-6, 1, False, keep.to(DEV) if masked else None)
+    out.backward(go.to(DEV))
+    fat().check_device_status()
+    got = (out.detach(), *(t.grad for t in leaves))
+    want = oracle.rational_attention_grads(*(t.float() for t in (q, k, v, go)), slopes, 0.2, causal=causal, key_mask=keep)
+    if dtype == torch.float32:
+        for g, w, name in zip(got, want, ("out", "dq", "dk", "dv")):
+            assert norm_max_err(g, w) < FP32_TOL, f"{name}: {norm_max_err(g, w):.2e}"
+    else:
+        assert_16bit_bar(got, want)
+
+
 def test_config1_fp32_closed_form_slopes():
     """Benchmark configuration 1: B=2,H=12,S=512,D=64 float32, slopes 2^(-8(i+1)/12)."""
     B, H, T, D = 2, 12, 512, 64
