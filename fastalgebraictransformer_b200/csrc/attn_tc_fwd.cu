@@ -487,6 +487,9 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p, int
 // us for none / the rule's choice / all shared (bfloat16, causal): 16 x 2000 x 128: 43.5 / 35.0 / 37.0; 8 x 4096 x 128:
 // 76.9 / 51.7 / 51.9; 2 x 8192 x 128: 143.7 / 78.3 / 78.4; 24 x 1024 x 64: 22.6 / 16.6 / 20.7; 24 x 1500 x 128: 35.0 / 30.9 / 35.0;
 // 4 x 1024 x 128: 24.7 / 18.5 / 18.5; 48 x 777 x 64 (192 CTAs): 26.7 / none shared / 32.9.
+// The constants are those of D = 128, causal; heads of 64 and calls that are not causal gain by the same rule, or nothing is shared (us
+// for none / the rule's choice): D = 64: 16 x 2000: 36.5 / 28.0; 8 x 4096: 68.8 / 50.0; 2 x 8192: 132.4 / 67.4; 12 x 1024: 20.3 / 14.6; 2 x 512: 12.3 / 10.5;
+// 24 x 1500: 28.9 / 28.3; not causal, D = 64: 4 x 1024: 21.3 / 15.1; 16 x 1024: 21.8 / 16.0; 12 x 2000: 38.8 / 38.8; D = 128: 16 x 1500: 33.0 / 33.0.
 int shared_blocks(const AttnParams& p) {
   const int n_qb = (p.T + 2 * BLK - 1) / (2 * BLK), n_kv = (p.T + BLK - 1) / BLK, sms = num_sms();
   const int64_t n_bh = int64_t(p.B) * p.H;

@@ -4,7 +4,7 @@
 // A step of generate() (algebraic_model.py:239-265) with a key/value cache moves every weight once through the GPU for 1-16
 // tokens: for the small model (110 M parameters, 8 sequences, 530 cached tokens) 219 MB of weights and 160 MB of cache,
 // 58 us at the copy bandwidth.  Issued operator by operator it is about 110 launches of 2-9 us that each wait for the one
-// before: 490 us on the GPU and 1.5-2.7 ms on the host.  What bounds it is latency, so this kernel keeps one CTA per SM
+// before: 455 us on the GPU and 2.6 ms on the host (this kernel: 373 us).  What bounds it is latency, so this kernel keeps one CTA per SM
 // resident for the whole step and the CTAs hand their results on through L2, five times per block of the model:
 //   P1  h += pending, y = norm(h) (every CTA for itself), qkv = y Wqkv^T
 //   P2  attention of the new token over the cache, one (batch, head) pair - or a share of its keys - per CTA; appends the row
@@ -13,8 +13,7 @@
 //   P5  pending = act Wdown^T
 // and, after the last block, the final norm and the head.
 // Hand-over: every 4 bytes travel with a 4-byte tag (launch, layer, phase) in one 8-byte word, and whoever needs a word polls
-// that word.  With grid-wide barriers instead (release, counter, acquire, then the loads) a step took 322 us: about 1000
-// cycles for the release, 1200-2000 for the wait and 800 for the loads, 61 times.  Buffers alternate between even and odd
+// that word; there is no grid-wide barrier.  A hand-over takes about 2.5 us of a phase's 6.  Buffers alternate between even and odd
 // layers: a word of layer l is overwritten in layer l + 2 only after a chain of all-to-all phases that contains every reader
 // of layer l (each CTA owns a P1 unit, the grid is cut to that), so no tag is lost.
 // Weights and old cache rows do not depend on the phase before: every thread streams the 16-byte pieces it will use itself

@@ -2,8 +2,9 @@
 // which the Python functions reach them.
 //
 // A call of a fused operator on a few thousand elements takes 2-4 us on the GPU; what it costs is the host.  With Python
-// autograd Functions over torch.ops, softmax forward + backward took 95 us of host time and residual add + norm 160 us
-// (of 38 and 10 us on the GPU).  Here the forward is one typed dispatcher call from a METH_FASTCALL function, the graph
+// autograd Functions over torch.ops, a pass of forward and backward took 77 us for softmax [4096, 4096], where the GPU needs 41,
+// and 123 us for residual add + norm [64, 768] (17 on the GPU); this way 48 and 83.  The forward is one typed dispatcher call from a
+// METH_FASTCALL function, the graph
 // node is a plain C++ Node with SavedVariables, and its backward calls the backward operator without going through the
 // interpreter.  The operators below the autograd key are the ones of torch_ops.cpp and are reached through the dispatcher,
 // so modes that watch operators (fake tensors, profilers, functionalisation) see what they saw before.

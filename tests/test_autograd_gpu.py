@@ -198,3 +198,48 @@ def test_traced_loss_has_the_eager_gradients(head, dtype):
     # eager: one product with 3 in float32, rounded; traced: the same product
     for got, want in zip(*results[::-1]):
         assert (got is None and want is None) or torch.allclose(got, want, rtol=2.0 ** -7 if dtype == torch.bfloat16 else 1e-6, atol=0)
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_traced_calls_have_the_eager_gradients(name):
+    """torch.compile follows the Function classes instead of the C++ nodes: same formulas, same kernels, same bits."""
+    fn, leaves, constants = case(name)
+    loss_of(torch.compile(fn, backend="aot_eager")(*leaves, *constants)).backward()
+    want = [torch.zeros_like(t) if g is None else g for t, g in zip(leaves, plain_grads(name))]      # (a traced graph fills in zeros)
+    assert same([t.grad for t in leaves], want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("name", CALLS)
+def test_saved_tensor_hooks_and_checkpointing(name, dtype):
+    """What the nodes save passes through the hooks (here: to the host and back), and a checkpointed call is run again."""
+    from torch.utils.checkpoint import checkpoint
+    want = plain_grads(name, dtype)
+    fn, leaves, constants = case(name, dtype)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.cpu(), lambda t: t.to(DEV)):
+        out = fn(*leaves, *constants)
+    loss_of(out).backward()
+    assert packed and close(dtype, [t.grad for t in leaves], want)
+    fn, leaves, constants = case(name, dtype)
+    loss_of(checkpoint(fn, *leaves, *constants, use_reentrant=False)).backward()
+    assert close(dtype, [t.grad for t in leaves], want)
+
+
+def close(dtype, got, want):
+    """The same bits, but for the d_q of the 16-bit attention backward, whose sums land in no fixed order (float32 sums rounded to 16 bits)."""
+    if dtype == torch.float32:
+        return same(got, want)
+    return all((a is None and b is None) or torch.allclose(a, b, rtol=2.0 ** -7, atol=2.0 ** -7 * float(b.abs().max())) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_a_graph_kept_for_a_second_backward(name):
+    fn, leaves, constants = case(name)
+    loss = loss_of(fn(*leaves, *constants))
+    loss.backward(retain_graph=True)
+    first = [t.grad.clone() if t.grad is not None else None for t in leaves]
+    loss.backward()
+    assert all((t.grad is None and f is None) or torch.equal(t.grad, 2 * f) for t, f in zip(leaves, first))
+    with pytest.raises(RuntimeError, match="second time"):
+        loss.backward()
