@@ -337,7 +337,7 @@ class AlgebraicTransformerLM(nn.Module):
         depend on later tokens (causal attention, relative bias), so they are kept instead of recomputed.  A step of one
         token per sequence runs as one launch where the fused step covers the model (``_DecodeStep``)."""
         if (cache.seen > 0 and input_ids.dim() == 2 and input_ids.size(1) == 1 and input_ids.dtype == torch.int64 and
-                input_ids.is_cuda and input_ids.device == self.head.weight.device):
+                input_ids.is_cuda and input_ids.device == cache.lengths.device):
             if cache.seen >= cache.capacity:
                 raise RuntimeError(f"key/value cache is full ({cache.capacity} tokens)")
             if cache.step is None or (cache.step is not False and not cache.step.stands(self)):

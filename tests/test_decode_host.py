@@ -39,6 +39,16 @@ def test_ids_of_another_gpu_never_reach_the_launch():
             model.forward_cached(torch.zeros(2, 1, dtype=torch.int64, device="cuda:1"), cache)
 
 
+def test_a_head_without_a_weight_of_its_own_is_asked_for_nothing():
+    """A wrapped head (an adapter, say) makes no fused step; the cached step runs module by module."""
+    with FakeTensorMode():
+        model, cache = model_and_cache()
+        cache.step = None
+        model.head = torch.nn.Sequential(model.head)
+        assert model.forward_cached(torch.zeros(2, 1, dtype=torch.int64, device="cuda:0"), cache).shape == (2, 64)
+        assert cache.step is False and cache.seen == 5
+
+
 @pytest.mark.parametrize("what", ["k", "v", "lengths", "slopes"])
 def test_a_cache_or_slopes_of_another_gpu_make_no_fused_step(what):
     from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
