@@ -406,8 +406,8 @@ class AlgebraicTransformerLM(nn.Module):
                     cache.seen += 1
                 else:
                     logits = self.forward_cached(nxt, cache)
-            if cache.step:
-                _lib.check_waits(idx.device)            # (a step that gave up waiting has NaN logits)
+            if cache.step and not torch.cuda.is_current_stream_capturing():
+                _lib.check_waits(idx.device)            # (a step that gave up waiting has NaN logits; a caller's capture cannot wait for it)
             return idx
         for _ in range(max_new_tokens):
             idx_cond = idx if idx.size(1) <= self.block_size else idx[:, -self.block_size:]

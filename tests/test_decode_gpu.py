@@ -392,6 +392,21 @@ def test_generate_replays_the_faster_way(B, new, fused, monkeypatch):
     assert bool(calls) == fused
 
 
+@pytest.mark.parametrize("new", [3, 12])
+def test_generate_inside_a_callers_capture(new):
+    """A caller may capture the whole call (no capture of its own then): nothing in it waits for the GPU."""
+    model = _half_model()
+    prompt = torch.randint(0, 64, (2, 7), device=DEV)
+    want = model.generate(prompt, new, top_k=1, cuda_graph=False)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = model.generate(prompt, new, top_k=1, cuda_graph=False)
+    for _ in range(2):
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+
+
 def test_workspace_outlives_its_last_launch_on_another_stream():
     """A step dropped while its launch still waits on a side stream: its workspace must not be handed out again yet."""
     model = _half_model()
