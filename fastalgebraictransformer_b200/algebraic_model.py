@@ -169,6 +169,7 @@ class _DecodeStep:
     def __init__(self, parameters, rest, watch, hooks, model, replays_well):
         self.parameters, self.rest, self.watch, self.hooks, self.model, self.replays_well = parameters, rest, watch, hooks, model, replays_well
         self.expected = [d.get(k) for d, k in watch]
+        self.gave_up = rest[0][12:13].view(torch.bool)   # the workspace's mark that a wait ran out in some step (its logits are NaN)
 
     @staticmethod
     def make(model, cache):
@@ -388,6 +389,8 @@ class AlgebraicTransformerLM(nn.Module):
                     cache.step = False
             graph = token = None
             for step in range(max_new_tokens):
+                if cache.step:                              # sampling from a given-up step's NaN would trip a device assert before the
+                    logits.masked_fill_(cache.step.gave_up, 0.0)    # report at the end; the model's own NaN go on as they are
                 nxt = sample(logits)
                 idx = torch.cat((idx, nxt), dim=1)
                 if step + 1 == max_new_tokens:

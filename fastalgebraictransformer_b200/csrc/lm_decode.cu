@@ -57,7 +57,8 @@ struct LmLayerArgs {
 struct LmArgs {
   LmLayerArgs layer[FAT_LM_MAX_LAYERS];
   const int64_t* ids; const void* embed; const void* norm; const void* head; void* logits; int* n_cached; int* status;
-  unsigned* ctl;                                // [0] launches so far, [1] CTAs that have left this one, [2] one of them gave up waiting (both 0 between launches)
+  unsigned* ctl;                                // [0] launches so far, [1] CTAs that have left this one, [2] one of them gave up waiting (both 0 between launches),
+                                                // [3] some step since the workspace was zeroed gave up
   // tagged words, two copies each (even / odd layers): float32 values qkv [B][3C], o [B][C], pend [B][C], part [B*H][n_split]
   // [D + 2] (n_split > 1); pairs of 16-bit values att [B][C/2], act [B][act_words]
   uint2 *qkv, *o, *pend, *att, *act, *part;
@@ -676,6 +677,7 @@ lm_decode_kernel(const __grid_constant__ LmArgs p) {
       for (int64_t i = threadIdx.x; i < int64_t(B) * p.V; i += kLmThreads) static_cast<T*>(p.logits)[i] = Elem<T>::from_c(__int_as_float(0x7fc00000));
     __syncthreads();                             // (everyone has read the mark)
     if (threadIdx.x == 0) {
+      if (bad) p.ctl[3] = 1u;
       p.ctl[2] = 0u;
       p.ctl[1] = 0u;
       p.ctl[0] += 1u;

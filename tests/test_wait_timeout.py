@@ -145,6 +145,7 @@ def test_words_that_never_arrive_end_in_nan_logits_and_a_usable_step():
     assert (status.item() >> 24) & 0xf == 1 and status.item() & 0xffffff == 300, f"status word 0x{status.item():08x}"
     assert torch.isnan(logits).all()
     assert torch.equal(lengths, cache.lengths)
+    assert workspace[12].item() == 1                                           # what generate looks at before it samples
 
     status.zero_()
     assert _lm_step(_lib.lib(), model, cache, ids, workspace, lengths, logits, status) == 0
@@ -186,3 +187,25 @@ def test_generate_reports_a_step_that_gave_up():
     assert model.generate(ids, 4, top_k=1).shape == (2, 5)
     with pytest.raises(RuntimeError, match="without room"):
         fat.check_device_status()
+
+
+@pytest.mark.parametrize("gave_up", [True, False])
+def test_generate_does_not_sample_from_a_step_that_gave_up(gave_up, monkeypatch):
+    """NaN probabilities are a device assert in multinomial, so a given-up step's logits are replaced before it; a model's own
+    NaN are not.  (The step and multinomial are stand-ins here: no NaN reaches the sampler whatever generate does.)"""
+    from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
+    model, _, ids, _ = _lm_case()
+    seen = []
+
+    def step(self, input_ids, cache):
+        self.rest[0][12] = int(gave_up)
+        return torch.full((2, 300), float("nan"), dtype=torch.bfloat16, device="cuda")
+
+    def multinomial(probs, num_samples):
+        seen.append(bool(torch.isfinite(probs).all()))
+        return torch.zeros(2, 1, dtype=torch.int64, device="cuda")
+
+    monkeypatch.setattr(_DecodeStep, "__call__", step)
+    monkeypatch.setattr(torch, "multinomial", multinomial)
+    model.generate(ids, 4, top_k=1)
+    assert seen == [True] + [gave_up] * 3
