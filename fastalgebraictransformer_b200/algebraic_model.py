@@ -224,11 +224,11 @@ class _DecodeStep:
         """Whether a replay of this launch takes less than a replay of the operators' launches (issued one by one those always
         lose).  Every CTA normalises the tokens of the whole step (8 or 16 rows) for itself, and long rows leave its ring fewer
         chunks, so the line is drawn at the size of that tile; for one sequence the operators' contractions are matrix-vector
-        products, which only wide models with aligned rows lose to.  us, fused / operators, 512 cached tokens unless said:
-        768 x 12 blocks, 8 sequences 373 / 455, 16 sequences 566 / 465; 1024 x 24 blocks, 8: 973 / 1197, 16: 1493 / 1229;
-        512 x 8 blocks, 16: 314 / 447; 1280 x 8 blocks, 4: 463 / 463 (1800 tokens 525 / 491); 1536 x 24 blocks, 1: 1243 / 1085, 8: 1423 / 1129;
-        one sequence: 768 x 12 blocks 380 / 460, 1024 x 24 blocks 956 / 986, 512 x 8 blocks 267 / 226, 256 x 4 blocks 109 / 92.
-        Heads of 128 (768 x 12 blocks, 8 sequences): 463 / 461, with 64 cached tokens 399 / 431."""
+        products, which narrow models lose least to.  On this side of the line the launch won at every size measured but the longest
+        contexts of 16 sequences; beyond it either may win.  us, fused / operators, 512 cached tokens unless said: 768 x 12 blocks, 8 sequences
+        201 / 444 (1800 tokens 350 / 496), 1 sequence 202 / 452; 1024 x 24 blocks, 8: 500 / 1196; 512 x 8 blocks, 16: 153 / 448
+        (1800: 259 / 509).  Beyond: 768 x 12 blocks, 16: 321 / 459 (1800: 644 / 615); 1280 x 8 blocks, 16: 799 / 701; 1536 x 24 blocks,
+        8: 1276 / 1110, 1: 923 / 1068; 256 x 4 blocks, 1: 99 / 101."""
         return (8 if B <= 8 else 16) * d_model <= 8192 and (B > 1 or (d_model >= 768 and d_ffn % 2 == 0))
 
     def stands(self, model) -> bool:

@@ -276,6 +276,38 @@ def test_fused_decode_step_of_many_blocks(dtype, d_model, n_head, n_layers, voca
             assert norm_max_err(b, a) < 3e-2
 
 
+# a chunk of the ring: 256 (heads of 64) or 128 (of 128) cached rows, 1024 or 2048 elements of weight rows
+@pytest.mark.parametrize("dtype,d_model,n_head,d_ffn,vocab,B,prompt,strided", [
+    (torch.bfloat16, 768, 12, 1000, 640, 8, 254, False),     # the last rows of a chunk and the first of the next; down rows end inside a block of 32
+    (torch.float16, 768, 6, 2730, 320, 13, 126, True),       # two chunks of down rows off 16-byte boundaries; cached rows apart in memory
+    (torch.bfloat16, 1280, 10, 2048, 200, 2, 17, False),     # a width that is not compiled in, two chunks per row
+    (torch.bfloat16, 320, 5, 2049, 333, 16, 15, True),       # odd rows, two chunks; act rows with a word to spare
+    (torch.float16, 512, 4, 2056, 64, 1, 513, False),        # one chunk and eight elements; shares of the keys
+])
+def test_fused_decode_step_at_the_edges_of_chunks(dtype, d_model, n_head, d_ffn, vocab, B, prompt, strided):
+    """Against the operators, on the same bound as above (two blocks: a rounding that tips moves a few 16-bit steps)."""
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM, check_device_status
+    torch.manual_seed(29)
+    model = AlgebraicTransformerLM(vocab_size=vocab, d_model=d_model, n_head=n_head, n_layers=2, d_ffn=d_ffn, dropout=0.0, block_size=1024)
+    model, ids = model.to(DEV).to(dtype).eval(), torch.randint(0, vocab, (B, prompt + 5), device=DEV)
+    make = model.new_cache
+
+    def new_cache(batch, capacity):
+        cache = make(batch, capacity)
+        if strided:
+            cache.k, cache.v = ([torch.cat([t, t], -1)[..., :t.shape[-1]] for t in side] for side in (cache.k, cache.v))
+        return cache
+    model.new_cache = new_cache
+    caches, logits = _both_ways(model, ids, prompt)
+    check_device_status()
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in zip(*logits):
+        assert norm_max_err(b, a) < 4 * eps
+    for side in ("k", "v"):
+        for a, b in zip(*(getattr(c, side) for c in caches)):
+            assert norm_max_err(b, a) < 4 * eps
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n_head", [1, 2])
 def test_fused_decode_step_rounds_where_the_operators_round(dtype, n_head):
