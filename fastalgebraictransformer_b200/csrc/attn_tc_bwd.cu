@@ -247,7 +247,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ DqMaps maps, const AttnParams p) {
   S& sm = *reinterpret_cast<S*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5;
   int rank, bh;
-  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, kBwdBands, rank, bh)) return;   // padding block of the banded order
+  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.bands, rank, bh)) return;   // padding block of the banded order
   const int b = bh / p.H, h = bh % p.H;
   const int qt = (p.T + BLK - 1) / BLK - 1 - rank;           // long rows first
   const int n = p.causal ? qt + 1 : (p.T + BLK - 1) / BLK;   // key tiles 0..qt (causal) or all of them
@@ -473,7 +473,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ DkvMaps maps, const AttnParams p)
   S& sm = *reinterpret_cast<S*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5;
   int kt, bh;                                                // rank = key tile: early key tiles see the most queries
-  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, kBwdBands, kt, bh)) return;     // padding block of the banded order
+  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.bands, kt, bh)) return;     // padding block of the banded order
   const int b = bh / p.H, h = bh % p.H;
   const int n_q_total = (p.T + BLK - 1) / BLK;
   const int q0 = p.causal ? kt : 0;                          // first query tile that sees this key tile
@@ -708,11 +708,24 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ DkvMaps maps, const AttnParams p)
 // The element-wise warps keep g for 64 score columns in registers between phase A and phase B, which needs
 // about 168 registers per thread; the other warps need far fewer, so the warpgroups trade registers with
 // setmaxnreg (the launch allocates 512 x 128).
-constexpr int kFusedDrainWarp = 8, kFusedTmaWarp = 12, kFusedMmaWarpX = 13, kFusedMmaWarpY = 14, kFusedThreads = 512;
-constexpr int kFusedRegsLaunch = 128, kFusedRegsEw = 168, kFusedRegsDrain = 104, kFusedRegsAux = 64;
-static_assert(256 * kFusedRegsEw + 128 * kFusedRegsDrain + 128 * kFusedRegsAux <= kFusedThreads * kFusedRegsLaunch,
-              "the warpgroups' register shares must fit in what the launch allocates");
+// Heads of 64 leave 128 columns of TMEM and 100 KB of shared memory: there dQ^T has columns of its own, so that dP^T of the next
+// query tile does not wait for dQ^T of this one to be drained, Q has three buffers, dO and dS^T two (with two Q tiles the third
+// came 1000 cycles after S^T wanted it), and 16 warps share the element-wise work. us, with the layout of D = 128 / with this one:
+// 2 x 8 x 8192 x 64 float16 632 / 537, 8 x 16 x 4096 x 64 bfloat16 1254 / 1091, 8 x 12 x 1024 x 64 115 / 101.
+template <int D> struct FusedShape {
+  static constexpr bool kOwnDq = D == 64;
+  static constexpr int kGroups = D == 64 ? 4 : 2;            // element-wise warpgroups; then one that drains dQ^T, and the TMA warp and the issuers
+  static constexpr int kEw = 128 * kGroups, kThreads = kEw + 256;
+  static constexpr int kCols = BLK / kGroups, kCh = kCols / 32;            // score columns of a warpgroup, in chunks of 32
+  static constexpr int kDrainWarp = kEw / 32, kTma = kDrainWarp + 4, kMmaX = kTma + 1, kMmaY = kTma + 2;
+  static constexpr int kQ = kOwnDq ? 3 : 2, kDo = kOwnDq ? 2 : 1, kDs = kOwnDq ? 2 : 1;         // buffers of Q, dO and dS^T
+  static constexpr int kRegsLaunch = D == 64 ? 80 : 128, kRegsEw = D == 64 ? 96 : 168, kRegsDrain = D == 64 ? 56 : 104, kRegsAux = D == 64 ? 40 : 64;
+  static_assert(kEw * kRegsEw + 128 * kRegsDrain + 128 * kRegsAux <= kThreads * kRegsLaunch, "the warpgroups' register shares must fit in what the launch allocates");
+};
 
+// Buffer and barrier parity of the i-th use of a ring of N buffers.
+template <int N> __device__ __forceinline__ uint32_t ring_stage(int i) { return uint32_t(i) % N; }
+template <int N> __device__ __forceinline__ uint32_t ring_parity(int i) { return uint32_t(i) / N & 1u; }
 template <int N> __device__ __forceinline__ void reg_share_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_share_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
@@ -721,13 +734,13 @@ struct FusedSmem {
   static constexpr int kTileBytes = BLK * D * 2;
   alignas(1024) unsigned char k[kTileBytes];
   alignas(1024) unsigned char v[kTileBytes];
-  alignas(1024) unsigned char q[2][kTileBytes];             // q[0] doubles as d_v staging in the epilogue
-  alignas(1024) unsigned char dout[kTileBytes];             // doubles as d_k staging in the epilogue
-  alignas(1024) unsigned char ds[BLK * BLK * 2];            // dS^T, 16-bit [128 keys][128 queries]
-  alignas(1024) float dq_stage[64 * D];                     // d_q staging tile [64 query rows][D]
-  alignas(16) float delta[2][BLK];
-  alignas(16) float inv[2][BLK];
-  uint64_t kv_full, q_full[2], q_empty[2], do_full, do_empty;
+  alignas(1024) unsigned char q[FusedShape<D>::kQ][kTileBytes];           // q[0] doubles as d_v staging in the epilogue
+  alignas(1024) unsigned char dout[FusedShape<D>::kDo][kTileBytes];        // the first doubles as d_k staging in the epilogue
+  alignas(1024) unsigned char ds[FusedShape<D>::kDs][BLK * BLK * 2];       // dS^T, 16-bit [128 keys][128 queries]
+  alignas(1024) float dq_stage[(D == 64 ? 128 : 64) * D];   // d_q staging tiles of [32 query rows][D]
+  alignas(16) float delta[FusedShape<D>::kQ][BLK];
+  alignas(16) float inv[FusedShape<D>::kQ][BLK];
+  uint64_t kv_full, q_full[FusedShape<D>::kQ], q_empty[FusedShape<D>::kQ], do_full[FusedShape<D>::kDo], do_empty[FusedShape<D>::kDo], ds_empty[FusedShape<D>::kDs];
   uint64_t s_full, p_full, dp_full, ds_full, dq_full, dq_free, acc_full;
   uint32_t tmem_base;
   int abort_flag;
@@ -738,15 +751,16 @@ struct FusedMaps { CUtensorMap q, dout, k, v, dk, dv, dq_acc; };    // dq_acc: f
 // MASKED: a padding mask over the keys is in force (p.key_mask is set).  A separate instantiation, so that the kernel of
 // the unmasked case carries none of it.
 template <typename T, int D, bool MASKED>
-__global__ void __launch_bounds__(kFusedThreads, 1)
+__global__ void __launch_bounds__(FusedShape<D>::kThreads, 1)
 attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParams p) {
-  static_assert((D == 128 || D == 64) && kEwGroups == 2, "laid out for D = 64 or 128 and two element-wise warpgroups");
+  static_assert(D == 128 || D == 64, "laid out for D = 64 or 128");
+  using F = FusedShape<D>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   using S = FusedSmem<D>;
   S& sm = *reinterpret_cast<S*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5;
   int kt, bh;                                                // rank = key tile: early key tiles see the most queries
-  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, kBwdBands, kt, bh)) return;     // padding block of the banded order
+  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.bands, kt, bh)) return;     // padding block of the banded order
   const int b = bh / p.H, h = bh % p.H;
   const int n_q_total = (p.T + BLK - 1) / BLK;
   const int q0 = p.causal ? kt : 0;                          // first query tile that sees this key tile
@@ -759,18 +773,20 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
 
   if (tid == 0) {
     sm.abort_flag = 0;
-    mbar_init(&sm.kv_full, 1); mbar_init(&sm.s_full, 1); mbar_init(&sm.p_full, kEwThreads); mbar_init(&sm.dp_full, 1);
-    mbar_init(&sm.ds_full, kEwThreads); mbar_init(&sm.dq_full, 1);
-    mbar_init(&sm.dq_free, 128); mbar_init(&sm.acc_full, 2); mbar_init(&sm.do_full, 1); mbar_init(&sm.do_empty, 2);
-    for (int i = 0; i < 2; ++i) { mbar_init(&sm.q_full[i], 1); mbar_init(&sm.q_empty[i], 1); }
+    mbar_init(&sm.kv_full, 1); mbar_init(&sm.s_full, 1); mbar_init(&sm.p_full, F::kEw); mbar_init(&sm.dp_full, 1);
+    mbar_init(&sm.ds_full, F::kEw); mbar_init(&sm.dq_full, 1);
+    mbar_init(&sm.dq_free, 128); mbar_init(&sm.acc_full, 2);
+    for (int i = 0; i < F::kDo; ++i) { mbar_init(&sm.do_full[i], 1); mbar_init(&sm.do_empty[i], 2); }
+    for (int i = 0; i < F::kDs; ++i) mbar_init(&sm.ds_empty[i], 1);
+    for (int i = 0; i < F::kQ; ++i) { mbar_init(&sm.q_full[i], 1); mbar_init(&sm.q_empty[i], 1); }
     mbar_fence_init();
   }
-  if (warp == kFusedTmaWarp) { tmem_alloc(&sm.tmem_base, kTmemCols); tmem_relinquish(); }
+  if (warp == F::kTma) { tmem_alloc(&sm.tmem_base, kTmemCols); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
-  const uint32_t tS = tmem, tP = tmem + BLK, tV = tmem + 2 * BLK, tK = tV + D;
+  const uint32_t tS = tmem, tP = tmem + BLK, tV = tmem + 2 * BLK, tK = tV + D, tQ = F::kOwnDq ? tmem + 3 * BLK : tP;
   float dscale, dscale_inv;                                  // c and 1/c of this (batch, head), see the top of the file
   dout_scale(dmax_of(p)[bh], dscale, dscale_inv);
 
@@ -781,25 +797,25 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
   const float* delta_bh = p.delta + (int64_t(b) * p.H + h) * pad_rows(p.T);
   const float* inv_bh = delta_bh + int64_t(p.B) * p.H * pad_rows(p.T);
   auto load_q = [&](int i) {                                  // Q tile, Delta and kOpScale/(L+eps) of query tile q0 + i
-    const int st = i & 1, qi = q0 + i;
+    const int st = ring_stage<F::kQ>(i), qi = q0 + i;
     mbar_expect_tx(&sm.q_full[st], S::kTileBytes + 2 * BLK * 4);
     load_tile_tma_noexpect<D>(sm.q[st], &maps.q, &sm.q_full[st], qi * BLK, h, b);
     bulk_load(sm.delta[st], delta_bh + qi * BLK, BLK * 4, &sm.q_full[st]);
     bulk_load(sm.inv[st], inv_bh + qi * BLK, BLK * 4, &sm.q_full[st]);
   };
-  if (warp == kFusedTmaWarp && elect_one()) {
+  if (warp == F::kTma && elect_one()) {
     mbar_expect_tx(&sm.kv_full, 2 * S::kTileBytes);
     load_tile_tma_noexpect<D>(sm.k, &maps.k, &sm.kv_full, kt * BLK, h, b);
     load_tile_tma_noexpect<D>(sm.v, &maps.v, &sm.kv_full, kt * BLK, h, b);
     load_q(0);
-    load_tile_tma<D>(sm.dout, &maps.dout, &sm.do_full, q0 * BLK, h, b);
-    if (n > 1) load_q(1);
+    load_tile_tma<D>(sm.dout[0], &maps.dout, &sm.do_full[0], q0 * BLK, h, b);
+    for (int i = 1; i < F::kQ && i < n; ++i) load_q(i);
   }
   if constexpr (!std::is_same<T, __half>::value) {
     if (g.wait(&sm.kv_full, 0, 139)) {
       uint32_t out_of_range = 0;
 #pragma unroll
-      for (int off = tid * 16; off < S::kTileBytes; off += kFusedThreads * 16)
+      for (int off = tid * 16; off < S::kTileBytes; off += F::kThreads * 16)
         *reinterpret_cast<uint4*>(sm.k + off) = bf16x8_to_f16x8(*reinterpret_cast<const uint4*>(sm.k + off), out_of_range);
       if (out_of_range && p.status) atomicOr(p.status, kStatusF16Range);
       fence_async_smem();
@@ -807,100 +823,108 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
     __syncthreads();
   }
 
-  if (warp >= kFusedTmaWarp) {
-    reg_share_dec<kFusedRegsAux>();                             // warps 12..15 (15 only takes part in this)
-    if (warp == kFusedTmaWarp) {
+  if (warp >= F::kTma) {
+    reg_share_dec<F::kRegsAux>();                             // warps 12..15 (15 only takes part in this)
+    if (warp == F::kTma) {
       // ---------------------------------------------------------------- TMA producer
       if (elect_one()) {
-        for (int i = 1; i < n; ++i) {                                          // (Q(0), Q(1) and dO(0) are on their way)
-          if (i >= 2) {
-            if (!g.wait(&sm.q_empty[i & 1], ((i >> 1) & 1) ^ 1, 140)) break;
+        for (int i = 1; i < n; ++i) {                                          // (the first Q tiles and dO(0) are on their way)
+          if (i >= F::kQ) {
+            if (!g.wait(&sm.q_empty[ring_stage<F::kQ>(i)], ring_parity<F::kQ>(i) ^ 1, 140)) break;
             load_q(i);
           }
-          if (!g.wait(&sm.do_empty, (i & 1) ^ 1, 141)) break;                  // dV(i-1) and dP^T(i-1) have read dO(i-1)
-          load_tile_tma<D>(sm.dout, &maps.dout, &sm.do_full, (q0 + i) * BLK, h, b);
+          const int ds = ring_stage<F::kDo>(i);
+          if (!g.wait(&sm.do_empty[ds], ring_parity<F::kDo>(i) ^ 1, 141)) break;   // dV and dP^T have read what the buffer held
+          load_tile_tma<D>(sm.dout[ds], &maps.dout, &sm.do_full[ds], (q0 + i) * BLK, h, b);
         }
       }
-    } else if (warp == kFusedMmaWarpX || warp == kFusedMmaWarpY) {
+    } else if (warp == F::kMmaX || warp == F::kMmaY) {
       // ---------------------------------------------------------------- tensor-core issuers
       if (elect_one()) {
-        constexpr int F = Pack16<T>::kFmt, H16 = Pack16<__half>::kFmt;
+        constexpr int FT = Pack16<T>::kFmt, H16 = Pack16<__half>::kFmt;
         constexpr uint32_t idesc_s = idesc_f16(BLK, BLK, H16, 0, 0);        // S^T = K Q^T: both operands K-major, float16 (q and k tiles are float16)
-        constexpr uint32_t idesc_dp = idesc_f16(BLK, BLK, F, 0, 0);         // dP^T = V dO^T: tensor dtype
-        constexpr uint32_t idesc_dv = idesc_f16(BLK, D, F, 0, 1);           // dV += P^T dO: B (dO) MN-major, tensor dtype
+        constexpr uint32_t idesc_dp = idesc_f16(BLK, BLK, FT, 0, 0);         // dP^T = V dO^T: tensor dtype
+        constexpr uint32_t idesc_dv = idesc_f16(BLK, D, FT, 0, 1);           // dV += P^T dO: B (dO) MN-major, tensor dtype
         constexpr uint32_t idesc_dk = idesc_f16(BLK, D, H16, 0, 1);         // dK += dS^T Q: B (Q) MN-major, float16
         constexpr uint32_t idesc_dq = idesc_f16(BLK, BLK, H16, 1, 1);       // dQ^T: A = K (MN-major), B = dS^T (MN-major), float16
         bool ok = g.wait(&sm.kv_full, 0, 150);
-        if (warp == kFusedMmaWarpX) {
+        if (warp == F::kMmaX) {
           // ---- issuer X: dV as soon as P^T is written, then the next S^T into the same columns
           const uint64_t kd = desc_kmajor(sm.k);
-          const uint64_t qd[2] = {desc_kmajor(sm.q[0]), desc_kmajor(sm.q[1])};
-          const uint64_t dod_mn = desc_mnmajor(sm.dout);
+          constexpr uint32_t kNext = S::kTileBytes >> 4;       // from a buffer's descriptor to the next buffer's
+          const uint64_t qd = desc_kmajor(sm.q[0]), qd1 = desc_kmajor(sm.q[1]), dod_mn = desc_mnmajor(sm.dout[0]);
           if (ok && (ok = g.wait(&sm.q_full[0], 0, 151))) {
             tc_fence_after();
-            issue_gemm_nt<D>(tS, kd, qd[0], idesc_s);
+            issue_gemm_nt<D>(tS, kd, qd, idesc_s);
             mma_commit(&sm.s_full);
           }
           for (int i = 0; i < n && ok; ++i) {
-            const int st = i & 1, st1 = st ^ 1;
+            const int st1 = ring_stage<F::kQ>(i + 1);
             // dO(i) and Q(i+1) were requested long ago: their barriers are settled before P^T, so that nothing but the issue
             // of the MMAs stands between the end of phase A and the next S^T (a satisfied wait still costs 150-250 cycles)
-            if (!(ok = g.wait_polling(&sm.do_full, i & 1, 153))) break;
-            if (i + 1 < n && !(ok = g.wait_polling(&sm.q_full[st1], ((i + 1) >> 1) & 1, 154))) break;
+            const int ds = ring_stage<F::kDo>(i);
+            if (!(ok = g.wait_polling(&sm.do_full[ds], ring_parity<F::kDo>(i), 153))) break;
+            if (i + 1 < n && !(ok = g.wait_polling(&sm.q_full[st1], ring_parity<F::kQ>(i + 1), 154))) break;
             if (!(ok = g.wait_polling(&sm.p_full, i & 1, 152))) break;
             tc_fence_after();
-            if constexpr (MASKED && kMaskedHiLo<T>) issue_gemm_tn_hilo(tV, tS, dod_mn, idesc_dv, i > 0);
-            else issue_gemm_tn<kColsPerGroup>(tV, tS, dod_mn, idesc_dv, i > 0);               // dV += P^T dO
-            mma_commit(&sm.do_empty);                                                // X's share of releasing dO(i)
+            if constexpr (MASKED && kMaskedHiLo<T>) issue_gemm_tn_hilo(tV, tS, dod_mn + ds * kNext, idesc_dv, i > 0);
+            else issue_gemm_tn<F::kCols>(tV, tS, dod_mn + ds * kNext, idesc_dv, i > 0);               // dV += P^T dO
+            mma_commit(&sm.do_empty[ds]);                                                // X's share of releasing dO(i)
             if (i + 1 < n) {
-              issue_gemm_nt<D>(tS, kd, qd[st1], idesc_s);                                // S^T of the next query tile
+              issue_gemm_nt<D>(tS, kd, F::kQ == 2 ? (st1 ? qd1 : qd) : qd + st1 * kNext, idesc_s);                                // S^T of the next query tile
               mma_commit(&sm.s_full);
             }
           }
         } else {
-          // ---- issuer Y: dQ^T and dK from the shared-memory dS^T tile, then the next dP^T once dQ^T has been drained
+          // ---- issuer Y: dQ^T and dK from the shared-memory dS^T tile; the next dP^T once dQ^T has been drained, or, where dQ^T has
+          // columns of its own, before it
           const uint64_t vd = desc_kmajor(sm.v), kd_mn = desc_mnmajor(sm.k);
-          const uint64_t dsd_k = desc_kmajor(sm.ds), dsd_mn = desc_mnmajor(sm.ds);
-          const uint64_t qd_mn[2] = {desc_mnmajor(sm.q[0]), desc_mnmajor(sm.q[1])};
-          const uint64_t dod = desc_kmajor(sm.dout);
-          if (ok && (ok = g.wait(&sm.do_full, 0, 155))) {
+          const uint64_t dsd_k0 = desc_kmajor(sm.ds[0]), dsd_mn0 = desc_mnmajor(sm.ds[0]), qd_mn0 = desc_mnmajor(sm.q[0]), qd_mn1 = desc_mnmajor(sm.q[1]), dod = desc_kmajor(sm.dout[0]);
+          constexpr uint32_t kNext = S::kTileBytes >> 4, kNextDs = (BLK * BLK * 2) >> 4;
+          auto issue_dp = [&](int i) {
             tc_fence_after();
-            issue_gemm_nt<D>(tP, vd, dod, idesc_dp);
+            issue_gemm_nt<D>(tP, vd, dod + ring_stage<F::kDo>(i) * kNext, idesc_dp);
             mma_commit(&sm.dp_full);
-            mma_commit(&sm.do_empty);
-          }
+            mma_commit(&sm.do_empty[ring_stage<F::kDo>(i)]);                                        // Y's share of releasing dO(i)
+          };
+          if (ok && (ok = g.wait(&sm.do_full[0], 0, 155))) issue_dp(0);
           for (int i = 0; i < n && ok; ++i) {
-            const int st = i & 1;
+            const int st = ring_stage<F::kQ>(i), sd = ring_stage<F::kDs>(i);
+            const uint64_t dsd_k = dsd_k0 + sd * kNextDs, dsd_mn = dsd_mn0 + sd * kNextDs, qd_mn = F::kQ == 2 ? (st ? qd_mn1 : qd_mn0) : qd_mn0 + st * kNext;
+            if (F::kOwnDq && i + 1 < n && !(ok = g.wait_polling(&sm.do_full[ring_stage<F::kDo>(i + 1)], ring_parity<F::kDo>(i + 1), 158))) break;
             if (!(ok = g.wait_polling(&sm.ds_full, i & 1, 156))) break;                  // phase B done: dS^T in smem, dP^T read
+            if constexpr (F::kOwnDq) {
+              if (i + 1 < n) issue_dp(i + 1);
+              if (i > 0 && !(ok = g.wait_polling(&sm.dq_free, (i - 1) & 1, 157))) break;   // dQ^T(i-1) has left TMEM
+            }
             tc_fence_after();
             // dQ^T = K^T dS^T over the keys.  The MMA is always 128 rows tall: with D = 64 the second 64-row chunk of the
             // MN-major A operand is the tile that follows K in shared memory (V), so TMEM lanes 64..127 receive numbers
             // nobody reads; the tensor pipe has the time, and M = 64 would use another accumulator layout.
 #pragma unroll
             for (int s = 0; s < BLK / 16; ++s)
-              mma_ss(tP, kd_mn + ((s * 2048) >> 4), dsd_mn + ((s * 2048) >> 4), idesc_dq, s > 0);
+              mma_ss(tQ, kd_mn + ((s * 2048) >> 4), dsd_mn + ((s * 2048) >> 4), idesc_dq, s > 0);
             mma_commit(&sm.dq_full);
 #pragma unroll
             for (int s = 0; s < BLK / 16; ++s)                                           // dK += dS^T Q over the queries
-              mma_ss(tK, dsd_k + ((((s / 4) * (BLK * 128) + (s % 4) * 32)) >> 4), qd_mn[st] + ((s * 2048) >> 4), idesc_dk, i > 0 || s > 0);
+              mma_ss(tK, dsd_k + ((((s / 4) * (BLK * 128) + (s % 4) * 32)) >> 4), qd_mn + ((s * 2048) >> 4), idesc_dk, i > 0 || s > 0);
             mma_commit(&sm.q_empty[st]);
-            if (i + 1 < n) {
-              if (!(ok = g.wait_polling(&sm.do_full, (i + 1) & 1, 158))) break;         // (settled long before dQ^T is out)
+            if constexpr (F::kOwnDq) {
+              mma_commit(&sm.ds_empty[sd]);
+            } else if (i + 1 < n) {
+              if (!(ok = g.wait_polling(&sm.do_full[0], (i + 1) & 1, 158))) break;      // (settled long before dQ^T is out)
               if (!(ok = g.wait_polling(&sm.dq_free, i & 1, 157))) break;                // dQ^T(i) has left TMEM
-              tc_fence_after();
-              issue_gemm_nt<D>(tP, vd, dod, idesc_dp);                                   // dP^T of the next query tile
-              mma_commit(&sm.dp_full);
-              mma_commit(&sm.do_empty);                                             // Y's share of releasing dO(i+1)
+              issue_dp(i + 1);                                                           // dP^T of the next query tile
             }
           }
         }
         if (ok) mma_commit(&sm.acc_full);
       }
     }
-  } else if (warp >= kFusedDrainWarp) {
+  } else if (warp >= F::kDrainWarp) {
     // ------------------------------------------------------------------ dQ^T drain: TMEM -> smem (transposed) -> reduce-add
-    reg_share_dec<kFusedRegsDrain>();
-    const int dl = tid - kFusedDrainWarp * 32;                   // head-dimension index == TMEM lane
+    reg_share_dec<F::kRegsDrain>();
+    const int dl = tid - F::kDrainWarp * 32;                   // head-dimension index == TMEM lane
     const uint32_t lane_base = uint32_t(warp & 3) * 32;
     float* stage0 = sm.dq_stage;                              // two staging tiles of [32 query rows][D] float32
     float* stage1 = sm.dq_stage + 32 * D;
@@ -924,6 +948,34 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
         tma_store_commit();                                   // also when nothing was issued (rows beyond T): the waits above count groups
       }
     };
+    if constexpr (F::kOwnDq) {
+      // a quarter at a time through four staging tiles: up to three groups may still be reading
+      for (int i = 0; i < n && ok; ++i) {
+        if (!(ok = g.wait(&sm.dq_full, i & 1, 160))) break;
+        tc_fence_after();
+#pragma unroll
+        for (int part = 0; part < 4; ++part) {
+          uint32_t a[32];
+          tmem_ld32(tmem_addr(tQ, lane_base, 32 * part), a);
+          tmem_wait_ld_regs(a);
+          if (part == 3) { tc_fence_before(); mbar_arrive(&sm.dq_free); }                 // the next dQ^T may be issued
+          if (dl == 0) tma_store_wait_read3();
+          named_barrier(3, 128);
+          float* stage = sm.dq_stage + part * (32 * D);
+          if (dl < D) {                                       // lanes beyond the head dimension hold nothing
+#pragma unroll
+            for (int qi = 0; qi < 32; ++qi) stage[qi * D + dl] = __uint_as_float(a[qi]);
+          }
+          fence_async_smem();
+          named_barrier(3, 128);
+          const int row = (q0 + i) * BLK + 32 * part;
+          if (dl == 0) {
+            if (row < p.T) tma_reduce_add_4d(&maps.dq_acc, stage, 0, row, h, b);
+            tma_store_commit();                               // also when nothing was issued (rows beyond T): the waits count groups
+          }
+        }
+      }
+    } else {
     for (int i = 0; i < n; ++i) {
       const int row0 = (q0 + i) * BLK;
       if (!(ok = g.wait(&sm.dq_full, i & 1, 160))) break;
@@ -959,11 +1011,12 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
       flush(a, stage0, row0 + 64, true);                      // waits until only the stage1 group is still reading
       flush(c, stage1, row0 + 96, true);
     }
+    }
     if (dl == 0) tma_store_wait_all();
   } else {
     // ------------------------------------------------------------------ element-wise warpgroups
-    reg_share_inc<kFusedRegsEw>();
-    const int w = warp >> 2;                                 // query columns [64w, 64w+64) of each step
+    reg_share_inc<F::kRegsEw>();
+    const int w = warp >> 2;                                 // query columns [kCols w, kCols w + kCols) of each step
     const int r = tid & (BLK - 1);                           // key row inside the tile == TMEM lane
     const int key = kt * BLK + r;
     const bool kept = !MASKED || key >= p.T || key_kept(p, b, key);     // a key the padding mask takes out gets a bias that zeroes it
@@ -975,11 +1028,11 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
     const f32x2 cs2 = pk2(cs, cs);
     bool ok = true;
     for (int i = 0; i < n; ++i) {
-      const int st = i & 1, qi = q0 + i;
+      const int st = ring_stage<F::kQ>(i), qi = q0 + i;
       const bool diag = (qi == kt);
-      f32x2 gq[kColsPerGroup / 2];
+      f32x2 gq[F::kCols / 2];
       // ---- phase A: p = sigma^4 / (L+eps) -> packed P^T over S^T; g / (L+eps) kept in registers
-      if (!(ok = g.wait(&sm.q_full[st], (i >> 1) & 1, 170))) break;        // Delta / inv arrived with the Q tile
+      if (!(ok = g.wait(&sm.q_full[st], ring_parity<F::kQ>(i), 170))) break;        // Delta / inv arrived with the Q tile
       if (!(ok = g.wait(&sm.s_full, i & 1, 171))) break;
       tc_fence_after();
       // bias of query column c: -slope |key - (qi BLK + c)| = -sl * c + base with sl = slope for queries from the key on,
@@ -993,11 +1046,11 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
         constexpr int kMode = decltype(MODE)::value;
         constexpr bool kHiLo = decltype(HL)::value && std::is_same<T, __nv_bfloat16>::value;
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
+        for (int c = 0; c < F::kCh; ++c) {
           uint32_t sreg[32], preg[16], lreg[kHiLo ? 16 : 1];
-          tmem_ld32(tmem_addr(tS, lane_base, kColsPerGroup * w + 32 * c), sreg);
+          tmem_ld32(tmem_addr(tS, lane_base, F::kCols * w + 32 * c), sreg);
           tmem_wait_ld_regs(sreg);
-          const int col0 = kColsPerGroup * w + 32 * c;
+          const int col0 = F::kCols * w + 32 * c;
           f32x2 bias2 = pk2(fmaf(-sl, float(col0), base), fmaf(-sl, float(col0 + 1), base));
           float4 ivq = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -1033,7 +1086,7 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
             tmem_st16(tmem_addr(tS, lane_base, col0), preg);
             tmem_st16(tmem_addr(tS, lane_base, col0 + 16), lreg);
           } else {
-            tmem_st16(tmem_addr(tS, lane_base, packed_col(w, c)), preg);
+            tmem_st16(tmem_addr(tS, lane_base, uint32_t(F::kCols * w + 16 * c)), preg);
           }
         }
       };
@@ -1047,12 +1100,14 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
       // dP^T(i) was committed by the issuer of dQ^T(i-1) and dK(i-1), after them: its barrier also says that those
       // have finished reading the dS^T tile
       if (!(ok = g.wait(&sm.dp_full, i & 1, 172))) break;
+      if (F::kOwnDq && !(ok = g.wait(&sm.ds_empty[ring_stage<F::kDs>(i)], ring_parity<F::kDs>(i) ^ 1, 173))) break;       // (there dP^T is issued before them)
       tc_fence_after();
+      unsigned char* ds_tile = sm.ds[ring_stage<F::kDs>(i)];
       const float* dl = sm.delta[st];
 #pragma unroll
-      for (int c = 0; c < kChunks; ++c) {
+      for (int c = 0; c < F::kCh; ++c) {
         uint32_t dreg[32], preg[16];
-        const int col0 = kColsPerGroup * w + 32 * c;
+        const int col0 = F::kCols * w + 32 * c;
         tmem_ld32(tmem_addr(tP, lane_base, col0), dreg);
         tmem_wait_ld_regs(dreg);
         float4 dq4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1066,8 +1121,8 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
           preg[e] = pack_ds(d0, d1);
         }
 #pragma unroll
-        for (int sgm = 0; sgm < 4; ++sgm)        // 64-query chunk w of the tile, 16-byte segments 4c..4c+3 of this key's row
-          *reinterpret_cast<uint4*>(sm.ds + w * (BLK * 128) + sw128_offset(r, 4 * c + sgm)) =
+        for (int sgm = 0; sgm < 4; ++sgm)        // 64-query chunk of the tile, four 16-byte segments of this key's row
+          *reinterpret_cast<uint4*>(ds_tile + (F::kCols == 64 ? w : w >> 1) * (BLK * 128) + sw128_offset(r, (F::kCols == 64 ? 4 * c : 4 * (w & 1)) + sgm)) =
               make_uint4(preg[4 * sgm], preg[4 * sgm + 1], preg[4 * sgm + 2], preg[4 * sgm + 3]);
       }
       fence_async_smem();
@@ -1075,25 +1130,25 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
       mbar_arrive(&sm.ds_full);
     }
     if (ok) ok = g.wait(&sm.acc_full, 0, 174);
-    named_barrier(1, kEwThreads);
+    named_barrier(1, F::kEw);
     if (!g.aborted()) {
       // d_v (staged in q[0]) and d_k (staged in dout[0]); the multipliers undo the 16x (F16) and 8x (g8) units
       tc_fence_after();
-      for (int ch = w; ch < 2 * D / 32; ch += kEwGroups) {
+      for (int ch = w; ch < 2 * D / 32; ch += F::kGroups) {
         const bool is_dk = ch >= D / 32;
         const int c0 = (is_dk ? ch - D / 32 : ch) * 32;
         uint32_t oreg[32];
         tmem_ld32(tmem_addr(is_dk ? tK : tV, lane_base, c0), oreg);
         tmem_wait_ld_regs(oreg);
-        stage_row32<T>(is_dk ? sm.dout : sm.q[0], r, c0, oreg, is_dk ? 0.25f * scale * dscale_inv / kDsScale : 0.0625f / kOpScale);
+        stage_row32<T>(is_dk ? sm.dout[0] : sm.q[0], r, c0, oreg, is_dk ? 0.25f * scale * dscale_inv / kDsScale : 0.0625f / kOpScale);
       }
       fence_async_smem();
-      named_barrier(1, kEwThreads);
+      named_barrier(1, F::kEw);
       if (tid == 0) {
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
           tma_store_4d(&maps.dv, sm.q[0] + c * (BLK * 128), c * 64, kt * BLK, h, b);
-          tma_store_4d(&maps.dk, sm.dout + c * (BLK * 128), c * 64, kt * BLK, h, b);
+          tma_store_4d(&maps.dk, sm.dout[0] + c * (BLK * 128), c * 64, kt * BLK, h, b);
         }
         tma_store_commit();
         tma_store_wait_all();
@@ -1102,7 +1157,7 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == kFusedTmaWarp) tmem_dealloc(tmem, kTmemCols);
+  if (warp == F::kTma) tmem_dealloc(tmem, kTmemCols);
 }
 
 // d_q = round(dq_acc * scale / (4 kDsScale c)): float32 accumulator (dense [B,H,T,D]) -> tensor dtype with the caller's strides.
@@ -1179,7 +1234,7 @@ bool make_qk_maps(const AttnParams& p, CUtensorMap* mq, CUtensorMap* mk, bool k_
 template <typename Kern, typename Maps>
 int launch_main(Kern kern, const Maps& maps, const AttnParams& p, size_t smem, int threads, cudaStream_t st, const char* what) {
   if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, what)) return rc;
-  const dim3 grid(banded_grid((p.T + BLK - 1) / BLK, p.B * p.H, kBwdBands));
+  const dim3 grid(banded_grid((p.T + BLK - 1) / BLK, p.B * p.H, p.bands));
   kern<<<grid, threads, smem, st>>>(maps, p);
   return check_launch(what);
 }
@@ -1210,9 +1265,10 @@ int launch_bwd_fused(const AttnParams& p, cudaStream_t st) {
   auto kern = p.key_mask ? attn_bwd_fused_tc_kernel<T, D, true> : attn_bwd_fused_tc_kernel<T, D, false>;
   int regs = 0;
   if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), sizeof(FusedSmem<D>), "attn_bwd_fused_tc", &regs)) return rc;
-  if (regs * kFusedThreads < 256 * kFusedRegsEw + 128 * kFusedRegsDrain + 128 * kFusedRegsAux) {
+  using F = FusedShape<D>;
+  if (regs < F::kRegsLaunch) {
     // the warpgroups could never collect their register shares: refuse instead of letting setmaxnreg.inc wait
-    set_error("attn_bwd_fused: built with %d registers per thread, the register hand-over needs %d", regs, kFusedRegsLaunch);
+    set_error("attn_bwd_fused: built with %d registers per thread, the register hand-over needs %d", regs, F::kRegsLaunch);
     return FAT_ERR_LAUNCH;
   }
   FusedMaps m;
@@ -1224,7 +1280,7 @@ int launch_bwd_fused(const AttnParams& p, cudaStream_t st) {
       !make_tmap_bhtd_f32(&m.dq_acc, dq_acc, p.B, p.H, p.T, D, D, 32))
     return FAT_ERR_LAUNCH;
   if (int rc = launch_prepare<T, D>(p, st, dq_acc, false)) return rc;
-  if (int rc = launch_main(kern, m, p, sizeof(FusedSmem<D>), kFusedThreads, st, "attn_bwd_fused_tc")) return rc;
+  if (int rc = launch_main(kern, m, p, sizeof(FusedSmem<D>), F::kThreads, st, "attn_bwd_fused_tc")) return rc;
   const unsigned blocks = unsigned(p.B) * p.H * unsigned((p.T + kConvRows - 1) / kConvRows);
   attn_bwd_dq_convert_kernel<T, D><<<blocks, 256, 0, st>>>(p, dq_acc);
   return check_launch("attn_bwd_dq_convert");
@@ -1244,7 +1300,9 @@ size_t attn_bwd_tc_workspace_bytes(int B, int H, int T, int D, int dtype) {
   return stats_bytes(B, H, T) + dq_acc_bytes(B, H, T, D) + (dtype == FAT_BF16 ? 2 * f16_copy_bytes(B, H, T, D) : 0);
 }
 
-int attn_bwd_tc(const AttnParams& p, int dtype, cudaStream_t st) {
+int attn_bwd_tc(const AttnParams& args, int dtype, cudaStream_t st) {
+  AttnParams p = args;
+  p.bands = work_bands(p, 1, (p.T + BLK - 1) / BLK);
   if (dtype == FAT_BF16) return launch_bwd<__nv_bfloat16>(p, st);
   if (dtype == FAT_F16) return launch_bwd<__half>(p, st);
   set_error("attn_bwd_tc: unsupported dtype tag %d", dtype);

@@ -69,14 +69,19 @@ __device__ __forceinline__ void load_tile_tma(unsigned char* dst, const CUtensor
 // starts its longest CTA when almost nothing else is left and the GPU idles behind it.  The 1-D grid can therefore be
 // ordered in bands of ranks: band 0 holds the longest ranks of every (batch, head), the last band the shortest; inside
 // a band the ranks of one (batch, head) stay adjacent so that CTAs running together still share its tiles in L2.
-// More bands shorten the tail but spread each (batch, head) over more of the launch; measured at B*H = 128, S = 4096:
-// two bands are best for the forward (-2 %), four and more lose to L2 misses, and the backward kernels are best
-// with one band (all ranks of a (batch, head) adjacent, long ranks first).
-#ifndef FAT_FWD_BANDS
-#define FAT_FWD_BANDS 2
-#define FAT_BWD_BANDS 1
-#endif
-constexpr int kFwdBands = FAT_FWD_BANDS, kBwdBands = FAT_BWD_BANDS;
+// More bands shorten the tail, because long CTAs come first over the whole launch, but spread each (batch, head) over more of it,
+// and tiles are read again from HBM once the (batch, head)s under way no longer fit in L2 (126 MB).  The line is drawn at the bytes of one
+// [B,H,T,D] tensor of 16-bit elements: up to 40 MB every rank is a band of its own, up to 100 MB there are up to four, beyond that two in the forward
+// and one in the backward.  us, forward / fused backward, with 2 / 1 bands, 4 / 4, one per rank: 1 x 16 x 2000 x 128 (8 MB) - / 92.7, 73.2,
+// 65.8; 2 x 8 x 4096 x 64 (8 MB) 92.5 / 179, 82.6 / 156, 72.8 / 149; 4 x 16 x 2048 x 128 (34 MB) 131 / 292, 122 / 264, 115 / 241;
+// 1 x 16 x 8192 x 128 (34 MB) 319 / 722, 298 / 676, 282 / 660; 4 x 16 x 4096 x 128 (67 MB) 334 / 761, 325 / 745, 324 / 786;
+// 8 x 16 x 4096 x 64 (67 MB) 566 / 1097, 552 / 1076, 544 / 1138; 8 x 16 x 4096 x 128 (134 MB) 633 / 1458, 631 / 1476, 720 / 1947.
+inline int work_bands(const AttnParams& p, int large, int n_tiles) {
+  const int64_t bytes = int64_t(p.B) * p.H * p.T * p.D * 2;
+  if (bytes <= 40 << 20) return n_tiles;
+  const int some = n_tiles / 4 < 4 ? n_tiles / 4 : 4;
+  return bytes <= 100 << 20 && some > large ? some : large;
+}
 __host__ __device__ inline int band_size(int n_tiles, int bands) { return (n_tiles + bands - 1) / bands; }
 inline unsigned banded_grid(int n_tiles, int n_bh, int bands) {
   const int bs = band_size(n_tiles, bands);
