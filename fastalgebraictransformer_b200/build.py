@@ -77,6 +77,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("link of libfat_b200.so failed")
     build_ops(force, verbose)
     build_wait_test(force, verbose)
+    build_fill_shared(force)
     return LIB
 
 
@@ -118,6 +119,21 @@ def build_wait_test(force: bool = False, verbose: bool = False) -> str:
         if r.returncode:
             raise RuntimeError("build of the wait-timeout test library failed")
     return WAIT_TEST_LIB
+
+
+FILL_SHARED_LIB = os.path.join(PKG, "..", "tests", "_build", "libfill_shared.so")
+
+
+def build_fill_shared(force: bool = False) -> str:
+    """The tests' kernel that fills shared memory (tests/fill_shared.cu -> tests/_build/, never loaded by the package)."""
+    src = os.path.join(PKG, "..", "tests", "fill_shared.cu")
+    if os.path.exists(src) and (force or _stale(FILL_SHARED_LIB, [src])):
+        os.makedirs(os.path.dirname(FILL_SHARED_LIB), exist_ok=True)
+        r = subprocess.run([_nvcc(), *NVCC_FLAGS, "-shared", src, "-o", FILL_SHARED_LIB], capture_output=True, text=True)
+        if r.returncode:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("build of the tests' libfill_shared.so failed")
+    return FILL_SHARED_LIB
 
 
 def build_ops(force: bool = False, verbose: bool = False) -> str:

@@ -814,8 +814,9 @@ lm_decode_kernel(const __grid_constant__ LmArgs p, int stages) {
         c.run(a_lane, as, red, B, [&](int tok, int n, float2 v0, float2 v1) {
           const float2 gate = Pair16<T>::get(Pair16<T>::put(v0.x, v0.y)), value = Pair16<T>::get(Pair16<T>::put(v1.x, v1.y));
           if (n + 2 >= p.F && p.act_words > n / 2 + 1) st_word(act + tok * p.act_words + n / 2 + 1, 0u, tag + 3);          // (rows have an even number of words)
-          st_word(act + tok * p.act_words + n / 2,
-                  Pair16<T>::put(gate.x * rsigmoid(gate.x, rcp1p_abs(gate.x)) * value.x, gate.y * rsigmoid(gate.y, rcp1p_abs(gate.y)) * value.y), tag + 3);
+          // (column F of an odd width comes from a ring row that nothing was copied to: its weight in P5 is zero, which a NaN does not mind)
+          const float second = n + 1 < p.F ? gate.y * rsigmoid(gate.y, rcp1p_abs(gate.y)) * value.y : 0.f;
+          st_word(act + tok * p.act_words + n / 2, Pair16<T>::put(gate.x * rsigmoid(gate.x, rcp1p_abs(gate.x)) * value.x, second), tag + 3);
         });
         sync_computing();
       }

@@ -6,6 +6,7 @@ n must equal row n of the oracle's causal attention over the n+1 tokens, and the
 full forward gives at the same position.
 """
 import ctypes
+import os
 
 import pytest
 import torch
@@ -306,6 +307,57 @@ def test_fused_decode_step_at_the_edges_of_chunks(dtype, d_model, n_head, d_ffn,
     for side in ("k", "v"):
         for a, b in zip(*(getattr(c, side) for c in caches)):
             assert norm_max_err(b, a) < 4 * eps
+
+
+def _fill_shared(value):
+    """Every 32-bit word of every SM's shared memory."""
+    from fastalgebraictransformer_b200.build import FILL_SHARED_LIB
+    if not os.path.exists(FILL_SHARED_LIB):
+        pytest.skip("tests/_build/libfill_shared.so has not been built")
+    fill = ctypes.CDLL(FILL_SHARED_LIB).test_fill_shared
+    assert fill(ctypes.c_uint32(value), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+
+
+# what the ring's stages hold where nothing is copied to: rows of the matrix beyond its last one, the ends of rows, cached rows beyond the
+# last.  Odd feed-forward widths, whose last unit is in the second half of a chunk (1365) or in the first (3413), and an even one
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d_model,n_head,d_ffn", [(512, 8, 1365), (512, 4, 1365), (1280, 20, 3413), (1280, 10, 3413), (768, 12, 1042)])
+@pytest.mark.parametrize("B", [1, 8, 16])
+def test_fused_decode_step_uses_nothing_that_it_has_not_written(dtype, d_model, n_head, d_ffn, B):
+    """Shared memory full of NaN before every step, and one sequence whose cached rows are NaN: what the others get is to the bit what
+    they get from finite leftovers, and stays as close to the operators as in the tests above."""
+    from fastalgebraictransformer_b200 import AlgebraicTransformerLM, check_device_status
+    torch.manual_seed(31)
+    model = AlgebraicTransformerLM(vocab_size=203, d_model=d_model, n_head=n_head, n_layers=2, d_ffn=d_ffn, dropout=0.0, block_size=512)
+    model = model.to(DEV).to(dtype).eval()
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for prompt in (3, 300):
+        n = prompt + 3
+        ids = torch.randint(0, 203, (B, n), device=DEV)
+        start = model.new_cache(B, n)
+        model.forward_cached(ids[:, :prompt], start)
+        out = {}
+        for how in ("operators", "zeros", "nan", "nan rows"):
+            cache = model.new_cache(B, n)
+            for mine, its in zip(cache.k + cache.v, start.k + start.v):
+                mine.copy_(its)
+                if how == "nan rows":
+                    mine[0, :, :prompt] = float("nan")
+            cache.lengths.copy_(start.lengths)
+            cache.seen = start.seen
+            if how == "operators":
+                cache.step = False
+            steps = []
+            for t in range(prompt, n):
+                _fill_shared(0xffffffff if how == "nan" else 0)
+                steps.append(model.forward_cached(ids[:, t:t + 1], cache))
+            assert (how == "operators") != bool(cache.step)
+            out[how] = steps + [c[:, :, prompt:n] for c in cache.k + cache.v]
+        check_device_status()
+        for want, zeros, nan, rows in zip(*out.values()):
+            assert norm_max_err(zeros, want) < 4 * eps
+            assert torch.equal(nan, zeros)
+            assert torch.equal(rows[1:], zeros[1:])
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
