@@ -82,7 +82,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 WAIT_TEST_LIB = os.path.join(PKG, "..", "tests", "_build", "libfat_b200_waittest.so")
-WAIT_TEST_FLAGS = ["-DFAT_TEST_WITHHOLD_V_TILE=0", "-DFAT_TEST_CE_WITHHOLD_ROW=4", "-DFAT_TEST_LM_WITHHOLD_UNIT=0", "-DFAT_WAIT_HINT_NS=100000",
+WAIT_TEST_FLAGS = ["-DFAT_TEST_WITHHOLD_V_TILE=0", "-DFAT_TEST_CE_WITHHOLD_ROW=4", "-DFAT_TEST_LM_WITHHOLD_UNIT=0", "-DFAT_TEST_LM_NO_RING_WAIT=301",
+                   "-DFAT_WAIT_HINT_NS=100000",
                    "-DFAT_WAIT_SPINS=30", "-DFAT_LM_POLL_LIMIT=4096"]
 WAIT_TEST_SOURCES = ("attn_tc_fwd.cu", "loss.cu", "lm_decode.cu")
 
@@ -90,8 +91,8 @@ WAIT_TEST_SOURCES = ("attn_tc_fwd.cu", "loss.cu", "lm_decode.cu")
 def build_wait_test(force: bool = False, verbose: bool = False) -> str:
     """A TEST-ONLY variant of the library (tests/_build/, never loaded by the package): the attention forward is compiled
     so that its producer leaves out one V tile, the staged loss kernel so that its first block never requests the copy of
-    one row, the language model's decode step so that one unit of its first projection is never handed on, and every bounded
-    wait gives up after ~3 ms.  tests/test_wait_timeout.py uses it to run the give-up paths once (status word, NaN losses or
+    one row, the language model's decode step so that one unit of its first projection is never handed on and, with a vocabulary of 301, no
+    warp waits for its weights, and every bounded wait gives up after ~3 ms.  tests/test_wait_timeout.py uses it to run the give-up paths once (status word, NaN losses or
     logits, teardown, TMEM release).  Only those sources are recompiled; the other objects are the shipped ones."""
     srcs = [os.path.join(CSRC, n) for n in WAIT_TEST_SOURCES]
     headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + sorted(glob.glob(os.path.join(PKG, "..", "include", "*.h")))

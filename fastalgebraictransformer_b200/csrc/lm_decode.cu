@@ -301,8 +301,18 @@ struct RingBars { uint64_t full[kMaxStages], empty[kMaxStages], norm_full[2], no
 // Bounded like the polls: gives up after kWaitSpins tries (then the wait counts as run out).
 struct RingWait {
   volatile int *ring_failed, *failed;            // shared memory: a wait for the ring has run out in this CTA (later ones return at once)
+#ifdef FAT_TEST_LM_NO_RING_WAIT
+  bool gives_up;                                 // test builds only: with that many words in the vocabulary the computing warps' first wait runs out
+#endif
   __device__ __forceinline__ bool operator()(uint64_t* bar, uint32_t parity) const {
     bool ok = false;
+#ifdef FAT_TEST_LM_NO_RING_WAIT
+    if (gives_up && int(threadIdx.x) < kLmThreads) {
+      *ring_failed = 1;
+      *failed = 1;
+      return false;
+    }
+#endif
 #pragma unroll 1
     for (uint32_t i = 0; i < tc::kWaitSpins; ++i) {
       ok = tc::mbar_try_wait(bar, parity);
@@ -369,7 +379,7 @@ template <typename T, int D>
 __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, unsigned char* norm_w, const int* lens, RingBars& bars, const RingWait& wait, int stages) {
   using R = Rows<D>;
   const int lane = threadIdx.x & 31;
-  int stage = 0, sent = 0;
+  int stage = 0, sent = 0, norm1_sent = 0, norm2_sent = 0;
   uint32_t parity = 1;
   bool ok = true;
   auto copy = [&](uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -394,6 +404,7 @@ __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, u
       const int buf = ph >> 1;
       ok = wait(&bars.norm_empty[buf], (li & 1) ^ 1);
       if (ok && lane == 0) {
+        ++(buf ? norm2_sent : norm1_sent);
         tc::mbar_expect_tx(&bars.norm_full[buf], uint32_t(p.C) * 2u);
         copy(tc::smem_u32(norm_w) + uint32_t(buf * p.C) * 2u, li == p.L ? p.norm : ph ? p.layer[li].norm2 : p.layer[li].norm1, uint32_t(p.C) * 2u, &bars.norm_full[buf]);
       }
@@ -434,12 +445,19 @@ __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, u
         asked();
       }
   }
-  if (!ok)                                       // (something has run out: what is under way still has to land, within the same limits)
-    for (int i = 0; i < min(sent, stages); ++i) {
-      stage = (stage == 0 ? stages : stage) - 1;
-      if (stage == stages - 1) parity ^= 1u;
-      for (uint32_t n = 0; n < tc::kWaitSpins && !tc::mbar_try_wait(&bars.full[stage], parity ^ 1u); ++n) {}
-    }
+  // Nothing may be on its way into shared memory when the CTA leaves: the computing warps have waited for all of it unless something
+  // ran out, on either side.  One limit for all of these waits.
+  uint32_t left = tc::kWaitSpins;
+  auto landed = [&](uint64_t* bar, uint32_t phase) {
+    while (left != 0u && !tc::mbar_try_wait(bar, phase)) --left;
+  };
+  for (int i = 0; i < min(sent, stages); ++i) {
+    stage = (stage == 0 ? stages : stage) - 1;
+    if (stage == stages - 1) parity ^= 1u;
+    landed(&bars.full[stage], parity ^ 1u);
+  }
+  if (norm1_sent > 0) landed(&bars.norm_full[0], (norm1_sent - 1) & 1);
+  if (norm2_sent > 0) landed(&bars.norm_full[1], (norm2_sent - 1) & 1);
 }
 
 // Attention of one item: scores (keys from the ring as the A operand, the query in every column of B, so that a lane finds the scores
@@ -730,7 +748,11 @@ lm_decode_kernel(const __grid_constant__ LmArgs p, int stages) {
   unsigned char* norm_w = reinterpret_cast<unsigned char*>(h) + MR * 8 * p.C * 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Poller poll{&failed};
+#ifdef FAT_TEST_LM_NO_RING_WAIT
+  const RingWait ring_wait{&ring_failed, &failed, p.V == FAT_TEST_LM_NO_RING_WAIT};
+#else
   const RingWait ring_wait{&ring_failed, &failed};
+#endif
   const int B = p.B, C = NC ? NC * 256 : p.C, items = B * p.H * p.n_split;
   if (threadIdx.x == 0) {
     failed = ring_failed = 0;
