@@ -372,8 +372,8 @@ __device__ __forceinline__ int chunks_per_set(const Contraction& c) {
 }
 __device__ __forceinline__ int units_per_round(int wpu_log2) { return int(gridDim.x) * (kLmWarps >> wpu_log2); }
 
-// The loading warp: every chunk of the launch in the order in which the computing warps use them, as bulk copies (whole rows, one or a
-// few per lane).  What is copied starts and ends on 16-byte boundaries: around a row of the down projection that does not, up to 14 bytes
+// The loading warp: every chunk of the launch in the order in which the computing warps use them, as bulk copies (whole rows, one per
+// lane, or all of a chunk's cached rows at once).  What is copied starts and ends on 16-byte boundaries: around a row of the down projection that does not, up to 14 bytes
 // of its neighbours come along (the matrix itself starts and ends on one).
 template <typename T, int D>
 __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, unsigned char* norm_w, const int* lens, RingBars& bars, const RingWait& wait, int stages) {
@@ -415,12 +415,15 @@ __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, u
         const Item it = item_at(p, lens, item);
 #pragma unroll 1
         for (int sub = 0; it.lo + (sub >> 1) * R::kStep < it.hi && ok; ++sub) {
-          const int j = it.lo + (sub >> 1) * R::kStep + lane * (R::kStep / 32), n = max(0, min(R::kStep / 32, it.hi - j));
+          // Rows that lie next to each other are one copy of up to 32 KB: what bounds a long context is how many copies there are.  us per step,
+          // 4 blocks of 768, 8 sequences, 8000 cached tokens: 32 copies of 1 KB per chunk 383 (24 GB/s per SM), 8 of 4 KB 217, one 189 (65 GB/s).
+          const bool dense = p.cs_t == D;
+          const int per = dense ? R::kStep : R::kStep / 32, j = it.lo + (sub >> 1) * R::kStep + lane * per, n = dense && lane > 0 ? 0 : max(0, min(per, it.hi - j));
           const T* src = static_cast<const T*>((sub & 1) ? p.layer[li].v_cache : p.layer[li].k_cache) + it.rows + j * p.cs_t;
           uint64_t* bar = &bars.full[stage];
           const uint32_t dst = next(uint32_t(n) * (D * 2)) + uint32_t(lane) * (R::kStep / 32 * D * 2);
           if (ok && n > 0) {
-            if (p.cs_t == D) copy(dst, src, uint32_t(n) * (D * 2), bar);
+            if (dense) copy(dst, src, uint32_t(n) * (D * 2), bar);
             else
 #pragma unroll 1
               for (int i = 0; i < n; ++i) copy(dst + i * (D * 2), src + i * p.cs_t, D * 2, bar);

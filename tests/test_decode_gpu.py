@@ -284,12 +284,13 @@ def test_fused_decode_step_of_many_blocks(dtype, d_model, n_head, n_layers, voca
     (torch.bfloat16, 1280, 10, 2048, 200, 2, 17, False),     # a width that is not compiled in, two chunks per row
     (torch.bfloat16, 320, 5, 2049, 333, 16, 15, True),       # odd rows, two chunks; act rows with a word to spare
     (torch.float16, 512, 4, 2056, 64, 1, 513, False),        # one chunk and eight elements; shares of the keys
+    (torch.bfloat16, 512, 8, 1000, 64, 8, 1789, False),      # cached rows go round the ring; the last chunk has one row, then more
 ])
 def test_fused_decode_step_at_the_edges_of_chunks(dtype, d_model, n_head, d_ffn, vocab, B, prompt, strided):
     """Against the operators, on the same bound as above (two blocks: a rounding that tips moves a few 16-bit steps)."""
     from fastalgebraictransformer_b200 import AlgebraicTransformerLM, check_device_status
     torch.manual_seed(29)
-    model = AlgebraicTransformerLM(vocab_size=vocab, d_model=d_model, n_head=n_head, n_layers=2, d_ffn=d_ffn, dropout=0.0, block_size=1024)
+    model = AlgebraicTransformerLM(vocab_size=vocab, d_model=d_model, n_head=n_head, n_layers=2, d_ffn=d_ffn, dropout=0.0, block_size=2048)
     model, ids = model.to(DEV).to(dtype).eval(), torch.randint(0, vocab, (B, prompt + 5), device=DEV)
     make = model.new_cache
 
