@@ -47,7 +47,7 @@ namespace fat {
 namespace {
 
 constexpr int kLmThreads = 512, kLmWarps = kLmThreads / 32;     // the warps that compute
-constexpr int kLmBlock = kLmThreads + 128;     // and a warpgroup of which one warp loads
+constexpr int kLmBlock = kLmThreads + 128;     // and a warpgroup of which one warp loads (all four where cached rows are apart in memory)
 constexpr int kLaunchRegs = 96, kComputeRegs = 104, kLoadRegs = 56;       // registers per thread: at launch (65536 / 640 threads), after the two groups have shared them out
 static_assert(kLmThreads * kComputeRegs + 128 * kLoadRegs <= kLmBlock * kLaunchRegs, "the register shares must fit in what the launch allocates");
 constexpr int kPieces = 4;                      // 16-byte pieces that a computing thread takes from a chunk
@@ -372,11 +372,31 @@ __device__ __forceinline__ int chunks_per_set(const Contraction& c) {
 }
 __device__ __forceinline__ int units_per_round(int wpu_log2) { return int(gridDim.x) * (kLmWarps >> wpu_log2); }
 
-// The loading warp: every chunk of the launch in the order in which the computing warps use them, as bulk copies (whole rows, one per
-// lane, or all of a chunk's cached rows at once).  What is copied starts and ends on 16-byte boundaries: around a row of the down projection that does not, up to 14 bytes
-// of its neighbours come along (the matrix itself starts and ends on one).
+// kFetchers warps (this one is number `part`): n rows of D elements, cs_t elements apart, in 16-byte pieces that do not wait; `bar` gets
+// an arrival of every lane when its pieces are there.  (A lane's pieces have the same place in every so many rows.)
+constexpr int kFetchers = 4;
 template <typename T, int D>
-__device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, unsigned char* norm_w, const int* lens, RingBars& bars, const RingWait& wait, int stages) {
+__device__ __forceinline__ void fetch_rows(uint32_t dst, const T* src, int64_t cs_t, int n, uint64_t* bar, int part) {
+  using R = Rows<D>;
+  const int at = part * 32 + int(threadIdx.x & 31), row0 = at / R::kLanes;
+  src += row0 * cs_t + at % R::kLanes * 8;
+  dst += uint32_t(at) * 16u;
+#pragma unroll 8
+  for (int row = row0; row < n; row += kFetchers * R::kRowsPerPiece) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    src += kFetchers * R::kRowsPerPiece * cs_t;
+    dst += kFetchers * 512u;
+  }
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+
+// The loading warp: every chunk of the launch in the order in which the computing warps use them, as bulk copies (whole rows, one per
+// lane, or all of a chunk's cached rows at once).  What is copied starts and ends on 16-byte boundaries: around a row of the down
+// projection that does not, up to 14 bytes of its neighbours come along (the matrix itself starts and ends on one).
+// Cached rows that are apart in memory are too small for bulk copies: then all warps of the group run this, and fetch those together;
+// part 0 does the rest, the others say on every chunk's barrier that they have nothing to add.
+template <typename T, int D>
+__device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, unsigned char* norm_w, const int* lens, RingBars& bars, const RingWait& wait, int stages, int part) {
   using R = Rows<D>;
   const int lane = threadIdx.x & 31;
   int stage = 0, sent = 0, norm1_sent = 0, norm2_sent = 0;
@@ -389,6 +409,7 @@ __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, u
   // the next stage, free; every lane says how many bytes it will ask for
   auto next = [&](uint32_t bytes) {
     ok = ok && wait(&bars.empty[stage], parity);
+    if (p.cs_t != D) tc::fence_async_smem();     // (ordinary copies may have written to the stage)
     if (ok) tc::mbar_expect_tx(&bars.full[stage], bytes);
     return tc::smem_u32(smem) + uint32_t(stage) * kChunkBytes;
   };
@@ -400,7 +421,7 @@ __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, u
 #pragma unroll 1
   for (int step = 0; step <= 4 * p.L && ok; ++step) {
     const int li = step >> 2, ph = opaque(step & 3);
-    if (!(ph & 1)) {
+    if (!(ph & 1) && part == 0) {
       const int buf = ph >> 1;
       ok = wait(&bars.norm_empty[buf], (li & 1) ^ 1);
       if (ok && lane == 0) {
@@ -417,16 +438,16 @@ __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, u
         for (int sub = 0; it.lo + (sub >> 1) * R::kStep < it.hi && ok; ++sub) {
           // Rows that lie next to each other are one copy of up to 32 KB: what bounds a long context is how many copies there are.  us per step,
           // 4 blocks of 768, 8 sequences, 8000 cached tokens: 32 copies of 1 KB per chunk 383 (24 GB/s per SM), 8 of 4 KB 217, one 189 (65 GB/s).
-          const bool dense = p.cs_t == D;
-          const int per = dense ? R::kStep : R::kStep / 32, j = it.lo + (sub >> 1) * R::kStep + lane * per, n = dense && lane > 0 ? 0 : max(0, min(per, it.hi - j));
+          // Rows apart: a bulk copy for each of 128 bytes 2008, one warp fetching 16-byte pieces 314, four 216.
+          const int j = it.lo + (sub >> 1) * R::kStep, n = min(R::kStep, it.hi - j);
           const T* src = static_cast<const T*>((sub & 1) ? p.layer[li].v_cache : p.layer[li].k_cache) + it.rows + j * p.cs_t;
           uint64_t* bar = &bars.full[stage];
-          const uint32_t dst = next(uint32_t(n) * (D * 2)) + uint32_t(lane) * (R::kStep / 32 * D * 2);
-          if (ok && n > 0) {
-            if (dense) copy(dst, src, uint32_t(n) * (D * 2), bar);
-            else
-#pragma unroll 1
-              for (int i = 0; i < n; ++i) copy(dst + i * (D * 2), src + i * p.cs_t, D * 2, bar);
+          if (p.cs_t == D) {
+            const uint32_t bytes = lane == 0 ? uint32_t(n) * (D * 2) : 0u, dst = next(bytes);
+            if (ok && bytes) copy(dst, src, bytes, bar);
+          } else {
+            ok = ok && wait(&bars.empty[stage], parity);
+            if (ok) fetch_rows<T, D>(tc::smem_u32(smem) + uint32_t(stage) * kChunkBytes, src, p.cs_t, n, bar, part);
           }
           asked();
         }
@@ -441,7 +462,7 @@ __device__ __forceinline__ void load_all(const LmArgs& p, unsigned char* smem, u
         const int set = sub >= per_set, n = (unit0 + (lane >> 3) * int(gridDim.x)) * 8 + (lane & 7), k = (sub - set * per_set) * cols;
         const int64_t row = (int64_t(set) * c.N + n) * c.K;
         const uint64_t lo = uint64_t(row + k) * 2 & ~uint64_t(15), hi = (uint64_t(row + min(k + cols, c.K)) * 2 + 15) & ~uint64_t(15);
-        const uint32_t bytes = lane < 8 * slots && n < c.N ? uint32_t(hi - lo) : 0u;
+        const uint32_t bytes = part == 0 && lane < 8 * slots && n < c.N ? uint32_t(hi - lo) : 0u;
         uint64_t* bar = &bars.full[stage];
         const uint32_t dst = next(bytes) + uint32_t(lane) * uint32_t((cols + 32) * 2);
         if (ok && bytes) copy(dst, static_cast<const unsigned char*>(c.W) + lo, bytes, bar);
@@ -756,10 +777,10 @@ lm_decode_kernel(const __grid_constant__ LmArgs p, int stages) {
 #else
   const RingWait ring_wait{&ring_failed, &failed};
 #endif
-  const int B = p.B, C = NC ? NC * 256 : p.C, items = B * p.H * p.n_split;
+  const int B = p.B, C = NC ? NC * 256 : p.C, items = B * p.H * p.n_split, loaders = p.cs_t == D ? 1 : kFetchers;
   if (threadIdx.x == 0) {
     failed = ring_failed = 0;
-    for (int i = 0; i < kMaxStages; ++i) { tc::mbar_init(&bars.full[i], 32); tc::mbar_init(&bars.empty[i], kLmWarps); }
+    for (int i = 0; i < kMaxStages; ++i) { tc::mbar_init(&bars.full[i], 32 * loaders); tc::mbar_init(&bars.empty[i], kLmWarps); }
     for (int i = 0; i < 2; ++i) { tc::mbar_init(&bars.norm_full[i], 1); tc::mbar_init(&bars.norm_empty[i], kLmWarps); }
     tc::mbar_fence_init();
   }
@@ -771,7 +792,7 @@ lm_decode_kernel(const __grid_constant__ LmArgs p, int stages) {
   __syncthreads();
   if (warp >= kLmWarps) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLoadRegs));
-    if (warp == kLmWarps) load_all<T, D>(p, lm_smem, norm_w, lens, bars, ring_wait, stages);
+    if (warp - kLmWarps < loaders) load_all<T, D>(p, lm_smem, norm_w, lens, bars, ring_wait, stages, warp - kLmWarps);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kComputeRegs));
     Ring st{bars, ring_wait, tc::smem_u32(lm_smem), 0, stages, 0u};

@@ -284,7 +284,9 @@ def test_fused_decode_step_of_many_blocks(dtype, d_model, n_head, n_layers, voca
     (torch.bfloat16, 1280, 10, 2048, 200, 2, 17, False),     # a width that is not compiled in, two chunks per row
     (torch.bfloat16, 320, 5, 2049, 333, 16, 15, True),       # odd rows, two chunks; act rows with a word to spare
     (torch.float16, 512, 4, 2056, 64, 1, 513, False),        # one chunk and eight elements; shares of the keys
-    (torch.bfloat16, 512, 8, 1000, 64, 8, 1789, False),      # cached rows go round the ring; the last chunk has one row, then more
+    (torch.bfloat16, 512, 8, 1000, 64, 8, 1789, False),      # cached rows go round the ring; the last chunk is not whole
+    (torch.bfloat16, 512, 8, 1000, 64, 8, 1789, True),       # and fetched row by row
+    (torch.float16, 768, 6, 1000, 64, 2, 1789, True),
 ])
 def test_fused_decode_step_at_the_edges_of_chunks(dtype, d_model, n_head, d_ffn, vocab, B, prompt, strided):
     """Against the operators, on the same bound as above (two blocks: a rounding that tips moves a few 16-bit steps)."""
