@@ -58,6 +58,7 @@ constexpr int kChunkBytes = 16 * row_pitch(3);
 static_assert(kChunkBytes >= 8 * row_pitch(4) && kChunkBytes >= kPieces * kLmThreads * 16, "a chunk holds 2 x 8 rows, 8 long rows, or cached rows");
 constexpr int kMaxStages = 5;
 constexpr size_t kLmSmemLimit = 226 * 1024;
+constexpr size_t kTileLimit = 188 * 1024;      // of that, what the tokens' rows may take (see plan_step)
 #ifdef FAT_LM_POLL_LIMIT                        // (test builds only)
 constexpr int kPollLimit = FAT_LM_POLL_LIMIT;
 #else
@@ -934,6 +935,10 @@ bool plan_step(int B, int C, int H, int D, int F, int V, int L, int capacity, Pl
   if (B < 1 || B > 16 || L < 1 || L > FAT_LM_MAX_LAYERS || (D != 64 && D != 128) || C != H * D || F < 1 || V < 1 || capacity < 1) return false;
   const int rows = B <= 8 ? 8 : 16, wide = F > C ? F : C;
   out->rows = rows;
+  // The tokens' activations, stream and partial sums.  Beyond this line one chunk or two are left for the ring, so that little streams
+  // ahead, and the operators, issued one by one, win at long contexts: us per step, fused / operators, 16 sequences, 8 blocks of 1280 with
+  // heads of 128: 64 cached tokens 630 / 1186, 1800 tokens 1209 / 1117, 4000 tokens 1825 / 1182.
+  if (size_t(rows) * (row_bytes((wide + 31) / 32 * 32) + size_t(C) * 4 + 2048) > kTileLimit) return false;
   const size_t red = size_t(kLmWarps) * (2 * (rows * 8 + 8) > D + 4 ? 2 * (rows * 8 + 8) : D + 4) * sizeof(float);
   out->smem = size_t(rows) * (row_bytes((wide + 31) / 32 * 32) + size_t(C) * 2) + red + size_t(2 * C) * 2;
   if (out->smem + kChunkBytes > kLmSmemLimit) return false;

@@ -322,10 +322,10 @@ def _fill_shared(value):
 
 
 # what the ring's stages hold where nothing is copied to: rows of the matrix beyond its last one, the ends of rows, cached rows beyond the
-# last.  Odd feed-forward widths, whose last unit is in the second half of a chunk (1365) or in the first (3413), and an even one
+# last.  Odd feed-forward widths, whose last unit is in the second half of a chunk (1365) or in the first (3413, 2389), and an even one
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("d_model,n_head,d_ffn", [(512, 8, 1365), (512, 4, 1365), (1280, 20, 3413), (1280, 10, 3413), (768, 12, 1042)])
-@pytest.mark.parametrize("B", [1, 8, 16])
+@pytest.mark.parametrize("d_model,n_head,d_ffn,B", [(*m, B) for m in ((512, 8, 1365), (512, 4, 1365), (768, 12, 1042)) for B in (1, 8, 16)] +
+                         [(*m, B) for m in ((1280, 20, 3413), (1280, 10, 3413)) for B in (1, 8)] + [(896, 14, 2389, 16), (896, 7, 2389, 16)])
 def test_fused_decode_step_uses_nothing_that_it_has_not_written(dtype, d_model, n_head, d_ffn, B):
     """Shared memory full of NaN before every step, and one sequence whose cached rows are NaN: what the others get is to the bit what
     they get from finite leftovers, and stays as close to the operators as in the tests above."""

@@ -186,3 +186,16 @@ def test_copies_of_a_cache_leave_the_step_behind():
     for other in (copy.copy(cache), copy.deepcopy(cache), pickle.loads(pickle.dumps(cache))):
         assert other.step is None and other.seen == 3 and torch.equal(other.lengths, cache.lengths)
     assert isinstance(cache.step, Step)
+
+
+@pytest.mark.parametrize("C,D,widest", [(1280, 64, {8: 8384, 16: 2368}), (1024, 128, {8: 8896, 16: 2880}), (768, 64, {8: 9408, 16: 3392}), (2048, 128, {8: 6848, 16: 0})])
+def test_the_widest_feed_forward_row_that_the_step_takes(C, D, widest):
+    """What the launch refuses goes module by module: the line at which the tokens' rows are too large for it (1280 wide with 16 sequences and the
+    default d_ffn of 3413 is beyond it), on both of its sides."""
+    from fastalgebraictransformer_b200 import _lib
+    need = _lib.lib().fat_lm_decode_workspace_bytes
+    need.restype, need.argtypes = _lib.PROTOTYPES["fat_lm_decode_workspace_bytes"]
+    for rows, F in widest.items():
+        for B in (rows, rows - 7):
+            assert F == 0 or need(B, C, C // D, D, F, 100, 2, 64, _lib.BF16) > 0
+            assert need(B, C, C // D, D, max(F, C) + 1, 100, 2, 64, _lib.BF16) == 0
