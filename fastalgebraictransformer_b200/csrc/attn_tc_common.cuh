@@ -63,8 +63,8 @@ __device__ __forceinline__ void load_tile_tma(unsigned char* dst, const CUtensor
   for (int c = 0; c < D / 64; ++c) tma_load_4d(dst + c * (BLK * 128), m, bar, c * 64, row0, h, b);
 }
 
-// ------------------------------------------------------------------ CTA work order of the causal kernels
-// Per (batch, head) there are n_tiles CTAs whose cost falls with their rank (rank 0 sees the most tiles of the other
+// ------------------------------------------------------------------ CTA work order
+// Per (batch, head) there are n_tiles CTAs; causal ones cost less the higher their rank (rank 0 sees the most tiles of the other
 // side).  Blocks are dispatched in index order; with all ranks of one (batch, head) adjacent, the last (batch, head)
 // starts its longest CTA when almost nothing else is left and the GPU idles behind it.  The 1-D grid can therefore be
 // ordered in bands of ranks: band 0 holds the longest ranks of every (batch, head), the last band the shortest; inside
@@ -72,12 +72,20 @@ __device__ __forceinline__ void load_tile_tma(unsigned char* dst, const CUtensor
 // More bands shorten the tail, because long CTAs come first over the whole launch, but spread each (batch, head) over more of it,
 // and tiles are read again from HBM once the (batch, head)s under way no longer fit in L2 (126 MB).  The line is drawn at the bytes of one
 // [B,H,T,D] tensor of 16-bit elements: up to 40 MB every rank is a band of its own, up to 100 MB there are up to four, beyond that two in the forward
-// and one in the backward.  us, forward / fused backward, with 2 / 1 bands, 4 / 4, one per rank: 1 x 16 x 2000 x 128 (8 MB) - / 92.7, 73.2,
-// 65.8; 2 x 8 x 4096 x 64 (8 MB) 92.5 / 179, 82.6 / 156, 72.8 / 149; 4 x 16 x 2048 x 128 (34 MB) 131 / 292, 122 / 264, 115 / 241;
-// 1 x 16 x 8192 x 128 (34 MB) 319 / 722, 298 / 676, 282 / 660; 4 x 16 x 4096 x 128 (67 MB) 334 / 761, 325 / 745, 324 / 786;
-// 8 x 16 x 4096 x 64 (67 MB) 566 / 1097, 552 / 1076, 544 / 1138; 8 x 16 x 4096 x 128 (134 MB) 633 / 1458, 631 / 1476, 720 / 1947.
+// and one in the backward.  us, forward / fused backward / deterministic dQ / dK and dV, with 2 forward and 1 backward bands, 4, one per rank:
+//    8 MB   2 x 8 x 4096 x 64      91.6 / 180 / 126 / 170,  83.3 / 157 / 109 / 146,  72.1 / 148 / 102 / 138
+//    8 MB   1 x 16 x 2000 x 128       - / 92.4 / 54.0 / 71.5,  - / 73.5 / 42.8 / 55.7,  - / 66.6 / 39.2 / 50.3
+//    34 MB  4 x 16 x 2048 x 128     116 / 259 / 152 / 201,  110 / 241 / 142 / 186,  110 / 235 / 144 / 184
+//    34 MB  1 x 16 x 8192 x 128     324 / 733 / 436 / 588,  302 / 683 / 405 / 544,  283 / 662 / 394 / 528
+//    67 MB  8 x 16 x 4096 x 64      561 / 1096 / 782 / 1046,  551 / 1069 / 767 / 1026,  545 / 1140 / 772 / 1025
+//    67 MB  4 x 16 x 4096 x 128     334 / 761 / 464 / 622,  326 / 745 / 445 / 595,  320 / 786 / 457 / 595
+//    134 MB 8 x 16 x 4096 x 128     633 / 1458,  631 / 1476,  720 / 1947
+// Where nothing is causal all ranks cost the same: there is no tail to shorten and the bands are those of large tensors at every size.  us, fused
+// backward with 1 band, 4, one per rank: 4 x 16 x 2048 x 128 358, 361, 378; 4 x 16 x 4096 x 64 948, 945, 977; 16 x 24 x 1024 x 128 595, 647, 803;
+// 1 x 16 x 8192 x 128 1212, 1229, 1260; the other kernels, and smaller tensors, do not care.
 inline int work_bands(const AttnParams& p, int large, int n_tiles) {
   const int64_t bytes = int64_t(p.B) * p.H * p.T * p.D * 2;
+  if (!p.causal) return large;
   if (bytes <= 40 << 20) return n_tiles;
   const int some = n_tiles / 4 < 4 ? n_tiles / 4 : 4;
   return bytes <= 100 << 20 && some > large ? some : large;
