@@ -24,7 +24,7 @@ struct AttnParams {
   // element b takes part; mask_words = 4 * ceil(T / 128), bits from T on are clear.  Null: every key takes part.
   const uint32_t* key_mask;
   int mask_words;
-  int bands;                                  // tensor path: bands of the CTAs' work order
+  int band;                                   // tensor path: ranks per band of the CTAs' work order
 };
 
 // Whether key `col` (< T) of batch element b takes part.

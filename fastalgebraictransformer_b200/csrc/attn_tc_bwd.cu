@@ -247,7 +247,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ DqMaps maps, const AttnParams p) {
   S& sm = *reinterpret_cast<S*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5;
   int rank, bh;
-  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.bands, rank, bh)) return;   // padding block of the banded order
+  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.band, rank, bh)) return;   // padding block of the banded order
   const int b = bh / p.H, h = bh % p.H;
   const int qt = (p.T + BLK - 1) / BLK - 1 - rank;           // long rows first
   const int n = p.causal ? qt + 1 : (p.T + BLK - 1) / BLK;   // key tiles 0..qt (causal) or all of them
@@ -473,7 +473,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ DkvMaps maps, const AttnParams p)
   S& sm = *reinterpret_cast<S*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5;
   int kt, bh;                                                // rank = key tile: early key tiles see the most queries
-  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.bands, kt, bh)) return;     // padding block of the banded order
+  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.band, kt, bh)) return;     // padding block of the banded order
   const int b = bh / p.H, h = bh % p.H;
   const int n_q_total = (p.T + BLK - 1) / BLK;
   const int q0 = p.causal ? kt : 0;                          // first query tile that sees this key tile
@@ -760,7 +760,7 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
   S& sm = *reinterpret_cast<S*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5;
   int kt, bh;                                                // rank = key tile: early key tiles see the most queries
-  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.bands, kt, bh)) return;     // padding block of the banded order
+  if (!banded_tile((p.T + BLK - 1) / BLK, p.B * p.H, p.band, kt, bh)) return;     // padding block of the banded order
   const int b = bh / p.H, h = bh % p.H;
   const int n_q_total = (p.T + BLK - 1) / BLK;
   const int q0 = p.causal ? kt : 0;                          // first query tile that sees this key tile
@@ -1234,7 +1234,7 @@ bool make_qk_maps(const AttnParams& p, CUtensorMap* mq, CUtensorMap* mk, bool k_
 template <typename Kern, typename Maps>
 int launch_main(Kern kern, const Maps& maps, const AttnParams& p, size_t smem, int threads, cudaStream_t st, const char* what) {
   if (int rc = ready_kernel(reinterpret_cast<const void*>(kern), smem, what)) return rc;
-  const dim3 grid(banded_grid((p.T + BLK - 1) / BLK, p.B * p.H, p.bands));
+  const dim3 grid(banded_grid((p.T + BLK - 1) / BLK, p.B * p.H, p.band));
   kern<<<grid, threads, smem, st>>>(maps, p);
   return check_launch(what);
 }
@@ -1302,7 +1302,7 @@ size_t attn_bwd_tc_workspace_bytes(int B, int H, int T, int D, int dtype) {
 
 int attn_bwd_tc(const AttnParams& args, int dtype, cudaStream_t st) {
   AttnParams p = args;
-  p.bands = work_bands(p, 1, (p.T + BLK - 1) / BLK);
+  p.band = band_of(p, 1, (p.T + BLK - 1) / BLK);
   if (dtype == FAT_BF16) return launch_bwd<__nv_bfloat16>(p, st);
   if (dtype == FAT_F16) return launch_bwd<__half>(p, st);
   set_error("attn_bwd_tc: unsupported dtype tag %d", dtype);

@@ -199,7 +199,7 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p, int
     rank = unit / n_bh + (shared ? 0 : n_shared);
     bh = unit % n_bh;
     if (rank >= n_qb) return;                                // (the last whole block may lack a neighbour)
-  } else if (!banded_tile(n_qb, p.B * p.H, p.bands, rank, bh)) {
+  } else if (!banded_tile(n_qb, p.B * p.H, p.band, rank, bh)) {
     return;                                                  // padding block of the banded order
   }
   const int b = bh / p.H, h = bh % p.H;
@@ -525,7 +525,7 @@ int launch_fwd_grid(const FwdMaps& maps, const AttnParams& p, int n_shared, cuda
   cluster.val.clusterDim.x = 2;
   cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(PAIRS ? 2 * unsigned(n_shared * n_bh + ((n_qb - n_shared) * n_bh + 1) / 2) : banded_grid(n_qb, n_bh, p.bands));
+  cfg.gridDim = dim3(PAIRS ? 2 * unsigned(n_shared * n_bh + ((n_qb - n_shared) * n_bh + 1) / 2) : banded_grid(n_qb, n_bh, p.band));
   cfg.blockDim = dim3(kFwdThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -556,7 +556,7 @@ int launch_fwd(const AttnParams& p, cudaStream_t st) {
 
 int attn_fwd_tc(const AttnParams& args, int dtype, cudaStream_t st) {
   AttnParams p = args;
-  p.bands = work_bands(p, 2, (p.T + 2 * BLK - 1) / (2 * BLK));
+  p.band = band_of(p, 2, (p.T + 2 * BLK - 1) / (2 * BLK));
   if (dtype == FAT_BF16) return p.D == 128 ? launch_fwd<__nv_bfloat16, 128>(p, st) : launch_fwd<__nv_bfloat16, 64>(p, st);
   if (dtype == FAT_F16) return p.D == 128 ? launch_fwd<__half, 128>(p, st) : launch_fwd<__half, 64>(p, st);
   set_error("attn_fwd_tc: unsupported dtype tag %d", dtype);
