@@ -222,13 +222,16 @@ class _DecodeStep:
     @staticmethod
     def beats_replayed_operators(B: int, d_ffn: int, d_model: int) -> bool:
         """Whether a replay of this launch takes less than a replay of the operators' launches (issued one by one those always
-        lose).  Every CTA normalises the tokens of the whole step (8 or 16 rows) for itself, and long rows leave its ring fewer
-        chunks, so the line is drawn at the size of that tile; for one sequence the operators' contractions are matrix-vector
-        products, which narrow models lose least to.  On this side of the line the launch won at every size measured but the longest
-        contexts of 16 sequences; beyond it either may win.  us, fused / operators, 512 cached tokens unless said: 768 x 12 blocks, 8 sequences
-        201 / 444 (1800 tokens 350 / 496), 1 sequence 202 / 452; 1024 x 24 blocks, 8: 500 / 1196; 512 x 8 blocks, 16: 153 / 448
-        (1800: 259 / 509).  Beyond: 768 x 12 blocks, 16: 321 / 459 (1800: 644 / 615); 1280 x 8 blocks, 16: 799 / 701; 1536 x 24 blocks,
-        8: 1276 / 1110, 1: 923 / 1068; 256 x 4 blocks, 1: 99 / 101."""
+        lose up to some thousand cached tokens).  Every CTA normalises the tokens of the whole step (8 or 16 rows) for itself, and long rows
+        leave its ring fewer chunks, so the line is drawn at the size of that tile; for one sequence the operators' contractions are
+        matrix-vector products, which narrow models lose least to.  The line is the one that was measured when weights came by every thread's own
+        copies, and is on the safe side since one warp streams them: on this side of it the launch wins but for narrow models with 16 sequences and long
+        contexts, beyond it it wins as well at many sizes.  us, fused / operators, 512 cached tokens (8000 in brackets).  This side: 768 x 12 blocks, 1 sequence
+        212 / 453 (264 / 506), 8: 196 / 449 (543 / 781); 1024 x 24 blocks, 8: 499 / 1191 (1339 / 2125); 512 x 4 heads x 8 blocks, 16: 234 / 445 (525 / 726);
+        384 x 6 blocks, 16: 165 / 197 (407 / 387); 256 x 4 blocks, 16: 109 / 121 (246 / 223).  Beyond, where the launch wins: 768 x 12 blocks, 16: 287 / 460
+        (1135 / 1172); 1024 x 24 blocks, 16: 790 / 1220 (2850 / 3084); 1280 x 8 blocks, 8: 435 / 650 (1038 / 1091); 512 x 8 blocks, 1: 136 / 238 (182 / 290);
+        1536 x 24 blocks, 1: 920 / 1067 (1087 / 1135).  Where it may lose: 640 x 8 blocks, 16: 300 / 344 (914 / 755); 1536 x 24 blocks, 8: 1235 / 1039
+        (3072 / 2537); 2048 x 8 blocks, 4: 509 / 480 (857 / 786); 256 x 4 blocks, 1: 103 / 99 (125 / 117)."""
         return (8 if B <= 8 else 16) * d_model <= 8192 and (B > 1 or (d_model >= 768 and d_ffn % 2 == 0))
 
     def stands(self, model) -> bool:

@@ -12,7 +12,7 @@
 //                S^T = K Q^T, dP^T = V dO^T -> P^T = F inv, dS^T (TMEM) -> dV += P^T dO, dK += dS^T Q
 // In both main kernels the element-wise work is split in two phases so that the tensor core
 // never waits for it: phase A needs only the scores (sigma, F, g), phase B only dP'.
-// Eight element-wise warps share a tile: warpgroup w owns score columns [64w, 64w+64).
+// Eight element-wise warps share a tile: warpgroup w owns score columns [64w, 64w+64) (sixteen in the fused kernel of heads of 64: [32w, 32w+32)).
 #include <type_traits>
 
 #include "attn_tc_common.cuh"
@@ -824,7 +824,7 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
   }
 
   if (warp >= F::kTma) {
-    reg_share_dec<F::kRegsAux>();                             // warps 12..15 (15 only takes part in this)
+    reg_share_dec<F::kRegsAux>();                             // the last four warps (one of them only takes part in this)
     if (warp == F::kTma) {
       // ---------------------------------------------------------------- TMA producer
       if (elect_one()) {
@@ -926,7 +926,7 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
     reg_share_dec<F::kRegsDrain>();
     const int dl = tid - F::kDrainWarp * 32;                   // head-dimension index == TMEM lane
     const uint32_t lane_base = uint32_t(warp & 3) * 32;
-    float* stage0 = sm.dq_stage;                              // two staging tiles of [32 query rows][D] float32
+    float* stage0 = sm.dq_stage;                              // D = 128: two staging tiles of [32 query rows][D] float32 (D = 64: four)
     float* stage1 = sm.dq_stage + 32 * D;
     bool ok = true;
     // One quarter (32 query rows) of dQ^T: registers -> staging tile -> reduce-add.  One bulk group may still be reading
@@ -976,41 +976,41 @@ attn_bwd_fused_tc_kernel(const __grid_constant__ FusedMaps maps, const AttnParam
         }
       }
     } else {
-    for (int i = 0; i < n; ++i) {
-      const int row0 = (q0 + i) * BLK;
-      if (!(ok = g.wait(&sm.dq_full, i & 1, 160))) break;
-      tc_fence_after();
-      uint32_t a[32], c[32];
-      tmem_ld32(tmem_addr(tP, lane_base, 0), a);
-      tmem_ld32(tmem_addr(tP, lane_base, 32), c);
-      tmem_wait_ld_regs(a);
-      tmem_wait_ld_regs(c);
-      if (dl == 0) tma_store_wait_read();                     // both staging tiles are free (the previous step's reduces were issued long ago)
-      named_barrier(3, 128);
-      if (dl < D) {                                           // lanes beyond the head dimension hold nothing (D = 64)
+      for (int i = 0; i < n; ++i) {
+        const int row0 = (q0 + i) * BLK;
+        if (!(ok = g.wait(&sm.dq_full, i & 1, 160))) break;
+        tc_fence_after();
+        uint32_t a[32], c[32];
+        tmem_ld32(tmem_addr(tP, lane_base, 0), a);
+        tmem_ld32(tmem_addr(tP, lane_base, 32), c);
+        tmem_wait_ld_regs(a);
+        tmem_wait_ld_regs(c);
+        if (dl == 0) tma_store_wait_read();                     // both staging tiles are free (the previous step's reduces were issued long ago)
+        named_barrier(3, 128);
+        if (dl < D) {                                           // lanes beyond the head dimension hold nothing
 #pragma unroll
-        for (int qi = 0; qi < 32; ++qi) {
-          stage0[qi * D + dl] = __uint_as_float(a[qi]);
-          stage1[qi * D + dl] = __uint_as_float(c[qi]);
+          for (int qi = 0; qi < 32; ++qi) {
+            stage0[qi * D + dl] = __uint_as_float(a[qi]);
+            stage1[qi * D + dl] = __uint_as_float(c[qi]);
+          }
         }
+        tmem_ld32(tmem_addr(tP, lane_base, 64), a);            // second half into the same registers: dQ^T leaves TMEM early
+        tmem_ld32(tmem_addr(tP, lane_base, 96), c);
+        tmem_wait_ld_regs(a);
+        tmem_wait_ld_regs(c);
+        tc_fence_before();
+        mbar_arrive(&sm.dq_free);                               // the next dP^T may be issued
+        fence_async_smem();
+        named_barrier(3, 128);
+        if (dl == 0) {
+          tma_reduce_add_4d(&maps.dq_acc, stage0, 0, row0, h, b);
+          tma_store_commit();
+          if (row0 + 32 < p.T) { tma_reduce_add_4d(&maps.dq_acc, stage1, 0, row0 + 32, h, b); }
+          tma_store_commit();
+        }
+        flush(a, stage0, row0 + 64, true);                      // waits until only the stage1 group is still reading
+        flush(c, stage1, row0 + 96, true);
       }
-      tmem_ld32(tmem_addr(tP, lane_base, 64), a);            // second half into the same registers: dQ^T leaves TMEM early
-      tmem_ld32(tmem_addr(tP, lane_base, 96), c);
-      tmem_wait_ld_regs(a);
-      tmem_wait_ld_regs(c);
-      tc_fence_before();
-      mbar_arrive(&sm.dq_free);                               // the next dP^T may be issued
-      fence_async_smem();
-      named_barrier(3, 128);
-      if (dl == 0) {
-        tma_reduce_add_4d(&maps.dq_acc, stage0, 0, row0, h, b);
-        tma_store_commit();
-        if (row0 + 32 < p.T) { tma_reduce_add_4d(&maps.dq_acc, stage1, 0, row0 + 32, h, b); }
-        tma_store_commit();
-      }
-      flush(a, stage0, row0 + 64, true);                      // waits until only the stage1 group is still reading
-      flush(c, stage1, row0 + 96, true);
-    }
     }
     if (dl == 0) tma_store_wait_all();
   } else {

@@ -484,12 +484,13 @@ attn_fwd_tc_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p, int
 // How many of the longest query blocks per (batch, head) two CTAs should share (0: none, no clusters).  A CTA costs about
 // 5.5 us (6 with the exchange) and 2.05 us per key tile of its 256 queries; the first num_sms() CTAs start at once and the
 // rest, the shortest ones, behind the first to finish.  Sharing every block is not the best where that makes a second wave.
-// us for none / the rule's choice / all shared (bfloat16, causal): 16 x 2000 x 128: 43.5 / 35.0 / 37.0; 8 x 4096 x 128:
-// 76.9 / 51.7 / 51.9; 2 x 8192 x 128: 143.7 / 78.3 / 78.4; 24 x 1024 x 64: 22.6 / 16.6 / 20.7; 24 x 1500 x 128: 35.0 / 30.9 / 35.0;
-// 4 x 1024 x 128: 24.7 / 18.5 / 18.5; 48 x 777 x 64 (192 CTAs): 26.7 / none shared / 32.9.
-// The constants are those of D = 128, causal; heads of 64 and calls that are not causal gain by the same rule, or nothing is shared (us
-// for none / the rule's choice): D = 64: 16 x 2000: 36.5 / 28.0; 8 x 4096: 68.8 / 50.0; 2 x 8192: 132.4 / 67.4; 12 x 1024: 20.3 / 14.6; 2 x 512: 12.3 / 10.5;
-// 24 x 1500: 28.9 / 28.3; not causal, D = 64: 4 x 1024: 21.3 / 15.1; 16 x 1024: 21.8 / 16.0; 12 x 2000: 38.8 / 38.8; D = 128: 16 x 1500: 33.0 / 33.0.
+// us for none (in the work order of attn_tc_common.cuh) / the rule's choice, bfloat16, causal, medians of launches under the profiler: 16 x 2000 x 128: 42.5 / 36.6;
+// 8 x 4096 x 128: 76.0 / 62.2; 2 x 8192 x 128: 141.9 / 79.3; 24 x 1024 x 64: 22.0 / 16.5; 4 x 1024 x 128: 24.1 / 19.3; 12 x 3000 x 128: 59.1 / 57.2; 48 x 777 x 64 (192 CTAs):
+// 23.3, none shared; with all blocks shared 16 x 2000 x 128 took 6 % longer than by the rule, 24 x 1024 x 64 25 %.  The work order has made none shared the faster
+// way where the rule's gain was small: 24 x 1500 x 128: 34.6 / 38.5; 20 x 2000 x 64: 38.7 / 40.3.
+// The constants are those of D = 128, causal; heads of 64 and calls that are not causal gain by the same rule, or nothing is shared: D = 64: 16 x 2000: 38.4 / 30.6;
+// 8 x 4096: 70.7 / 53.2; 2 x 8192: 133.7 / 69.0; 12 x 1024: 21.6 / 15.6; 2 x 512: 12.9 / 11.2; 24 x 1500: 30.6 / 30.6; not causal, D = 64: 4 x 1024: 22.4 / 15.9;
+// 16 x 1024: 23.3 / 17.4; 12 x 2000: 41.1 / 41.1; D = 128: 16 x 1500: 36.5 / 36.6.
 int shared_blocks(const AttnParams& p) {
   const int n_qb = (p.T + 2 * BLK - 1) / (2 * BLK), n_kv = (p.T + BLK - 1) / BLK, sms = num_sms();
   const int64_t n_bh = int64_t(p.B) * p.H;

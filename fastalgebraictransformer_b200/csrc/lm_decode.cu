@@ -4,7 +4,7 @@
 // A step of generate() (algebraic_model.py:239-265) with a key/value cache moves every weight once through the GPU for 1-16
 // tokens: for the small model (110 M parameters, 8 sequences, 530 cached tokens) 219 MB of weights and 160 MB of cache,
 // 58 us at the copy bandwidth.  Issued operator by operator it is about 110 launches of 2-9 us that each wait for the one
-// before: 444 us on the GPU and 2.6 ms on the host (this kernel: 203 us).  What bounds it is latency, so this kernel keeps one CTA per SM
+// before: 449 us on the GPU and 2.6 ms on the host (this kernel: 197 us).  What bounds it is latency, so this kernel keeps one CTA per SM
 // resident for the whole step and the CTAs hand their results on through L2, five times per block of the model:
 //   P1  h += pending, y = norm(h) (every CTA for itself), qkv = y Wqkv^T
 //   P2  attention of the new token over the cache, one (batch, head) pair - or a share of its keys - per CTA; appends the row
@@ -17,13 +17,13 @@
 // them).  Buffers alternate between even and odd layers: a word of layer l is overwritten in layer l + 2 only after a chain of all-to-all
 // phases that contains every reader of layer l (each CTA owns a P1 unit, the grid is cut to that), so no tag is lost.
 // Weights and old cache rows do not depend on the phase before: one warp streams them through a ring of chunks in shared memory with
-// bulk copies, up to five chunks (160 KB) ahead of their use, across phases and layers, and the computing warps take their first
+// bulk copies, up to five chunks (165 KB) ahead of their use, across phases and layers, and the computing warps take their first
 // pieces into registers before they wait for the words.  When every thread asked for its own pieces (cp.async) and worked out their
 // addresses between the products and the hand-over, a step took 373 us: a warp issues an instruction every ten cycles here, so what
 // counts is how few of them stand between the words and the results.  That is also why the usual widths are compiled in, why
 // h, o, pending and qkv travel as the 16-bit pairs that they are rounded to anyway, and why scores come from the tensor cores.
-// us per step, 12 blocks of 768, 512 cached tokens, before / after: 1 sequence 380 / 202, 8 sequences 373 / 201, 16 sequences 566 / 321;
-// 64 cached tokens, 8 sequences: 171; 1800: 350.
+// us per step, 12 blocks of 768, 512 cached tokens, before / after: 1 sequence 415 / 212, 8 sequences 379 / 197, 16 sequences 571 / 287;
+// 8 sequences, 64 cached tokens 341 / 170, 1800 tokens 480 / 261.
 // Taken back: fetching the next block's weights and rows into L2 ahead of the ring (8 sequences 212 -> 272, one sequence a little
 // faster); keys of the next rows loaded behind the sums of these (registers spill); a copy of the tries on a barrier by one lane
 // instead of 32 (slower to wake up).
@@ -34,9 +34,9 @@
 // Roundings: h, qkv, o, gate, value and pending are rounded to 16 bits where the operator-by-operator path rounds them (operands,
 // cached rows and logits are 16-bit anyway), in every block, so that a step may run either way.  The two differ in the order of
 // float32 sums; now and then that tips a rounding, which moves every later one: two such evaluations drift apart while both keep
-// their distance from the exact result.  bfloat16 logits of 16-32 steps, 2-norm, this kernel / operators against 64 bits, and
-// against each other: 2 blocks of width 768 0.0095 / 0.0095, 0.0062; 5 blocks 0.0142 / 0.0143, 0.0112; 12 blocks 0.0205 / 0.0205,
-// 0.0187; 8 blocks of 1024 0.0220 / 0.0224, 0.0180.
+// their distance from the exact result.  bfloat16 logits of 16 steps, mean of four seeds, 2-norm, this kernel / the one whose scores were summed by
+// float32 FMAs / operators against 64 bits, and this kernel against the operators: 2 blocks of width 768 0.00959 / 0.00958 / 0.00960, 0.0061; 5 blocks
+// (heads of 128) 0.01444 / 0.01442 / 0.01443, 0.0114; 12 blocks 0.02062 / 0.02066 / 0.02059, 0.0184; 8 blocks of 1024 0.02154 / 0.02141 / 0.02181, 0.0183.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -75,8 +75,8 @@ struct LmArgs {
   const int64_t* ids; const void* embed; const void* norm; const void* head; void* logits; int* n_cached; int* status;
   unsigned* ctl;                                // [0] launches so far, [1] CTAs that have left this one, [2] one of them gave up waiting (both 0 between launches),
                                                 // [3] some step since the workspace was zeroed gave up
-  // tagged words, two copies each (even / odd layers): float32 values qkv [B][3C], o [B][C], pend [B][C], part [B*H][n_split]
-  // [D + 2] (n_split > 1); pairs of 16-bit values att [B][C/2], act [B][act_words]
+  // tagged words, two copies each (even / odd layers): pairs of 16-bit values qkv [B][3C/2], o [B][C/2], pend [B][C/2], att [B][C/2],
+  // act [B][act_words]; float32 values part [B*H][n_split][D + 2] (n_split > 1)
   uint2 *qkv, *o, *pend, *att, *act, *part;
   int64_t ids_stride, cs_b, cs_h, cs_t;
   int L, B, C, H, F, V, capacity, act_words, n_split, slopes_f32, a_stride;
@@ -955,6 +955,9 @@ bool plan_step(int B, int C, int H, int D, int F, int V, int L, int capacity, Pl
   return true;
 }
 
+// The usual widths are compiled in.  The instance for any other width keeps its loops and spills 420-610 bytes a thread; run at the usual widths, us per
+// step, 12 blocks, 512 cached tokens, compiled in / general: 512 wide, 8 sequences 218 / 314; 768 wide, 1 sequence 225 / 298, 8 198 / 308, 16 288 / 481;
+// 1024 wide, 8 sequences 263 / 401.
 template <typename T, int D, int MR>
 int launch_step(LmArgs& a, const Plan& pl, cudaStream_t st) {
   void (*kern)(const LmArgs, int) = a.C == 512 ? lm_decode_kernel<T, D, MR, 2> : a.C == 768 ? lm_decode_kernel<T, D, MR, 3>

@@ -251,7 +251,7 @@ def _both_ways(model, ids, prompt):
 
 
 # more blocks than there are word buffers (two, used in turn).  The keys of a (batch, head) pair whole and shared out; heads of 128
-# for up to eight sequences; 16 sequences at width 1024, which leave room for one chunk in flight
+# for up to eight sequences; 16 sequences at width 1024, which leave room for a ring of two chunks
 @pytest.mark.parametrize("dtype,d_model,n_head,n_layers,vocab,B,prompt", [
     (torch.bfloat16, 768, 12, 5, 1000, 8, 150), (torch.bfloat16, 512, 8, 12, 509, 1, 300), (torch.float16, 768, 6, 3, 500, 4, 90),
     (torch.bfloat16, 1024, 16, 3, 300, 16, 40), (torch.float16, 512, 4, 4, 200, 3, 33),

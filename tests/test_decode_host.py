@@ -171,7 +171,7 @@ def test_decode_step_operator_declares_what_it_writes_and_its_shape():
     (9, 768, 2048, False), (16, 1024, 2730, False), (1, 512, 1365, False), (1, 896, 2389, False), (4, 1280, 3413, False), (1, 1536, 4096, False),
 ])
 def test_which_way_a_captured_step_goes(B, d_model, d_ffn, fused):
-    """On both sides of the line: at these sizes the launch was measured faster, or slower, than the operators' replay."""
+    """Both sides of the line (which is on the safe side: beyond it the launch is the faster way at some of these sizes too)."""
     from fastalgebraictransformer_b200.algebraic_model import _DecodeStep
     assert _DecodeStep.beats_replayed_operators(B, d_ffn, d_model) == fused
 
